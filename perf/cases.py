@@ -10,8 +10,8 @@ differentiable boxes; 32,768 bodies with cooked hulls) or lie between them.
 
 The stepping cases run worlds that have landed and keep moving in place
 (sleeping off, or velocities written back each frame, which wakes every
-body), so that every pass does the same kind of work; `asleep` is the
-default world after it has come to rest.  The rollouts rewind to the same
+body), so that every pass does the same kind of work; `resting` is the
+default world after most of it has fallen asleep.  The rollouts rewind to the same
 start each pass, so they cover the fall and the landing.
 """
 from __future__ import annotations
@@ -52,9 +52,10 @@ def listed():
         # The same pile in a host loop: each frame steps once, reads every
         # body to pinned host memory and writes every velocity back.
         {"name": "pile_131072_loop", "kind": "pile", "n": 131072, "scenes": 1, "steps": 1, "loop": True},
-        # A level that has come to rest, sleeping on (the default): most
-        # islands asleep, eight substeps, bodies read back.
-        {"name": "asleep_40000", "kind": "asleep", "n": 40000, "steps": 8},
+        # A level of scattered props that has come to rest, sleeping on (the
+        # default): three bodies in four asleep, eight substeps, bodies read
+        # back.
+        {"name": "resting_40000", "kind": "resting", "n": 40000, "steps": 8},
         # Batched forward: 4,096 independent scenes of 16 to 512 bodies
         # (piles and stacks of unit cubes), as a trainer steps them.
         {"name": "batch_4096", "kind": "batch", "n": 4096, "high": 512, "steps": 4},
@@ -76,7 +77,7 @@ def draw(rng):
     def log(a, b):
         return int(round(math.exp(rng.uniform(math.log(a), math.log(b)))))
 
-    kind = rng.choice(["platform", "boxes", "mechanisms", "pile", "pile", "pile_loop", "asleep", "batch", "hulls",
+    kind = rng.choice(["platform", "boxes", "mechanisms", "pile", "pile", "pile_loop", "resting", "batch", "hulls",
                        "rollout", "rollout_mixed", "sap"])
     if kind == "platform":
         return {"kind": kind, "n": log(8, 200)}
@@ -89,7 +90,7 @@ def draw(rng):
                 "loop": False}
     if kind == "pile_loop":
         return {"kind": "pile", "n": log(500, 131072), "scenes": 1, "steps": 1, "loop": True}
-    if kind == "asleep":
+    if kind == "resting":
         return {"kind": kind, "n": log(1000, 40000), "steps": rng.randint(1, 8)}
     if kind == "batch":
         return {"kind": kind, "n": log(16, 4000), "high": rng.randint(64, 512), "steps": rng.randint(1, 4)}
@@ -260,8 +261,8 @@ def prepare(case, seed):
     elif kind == "pile":
         w = _world([_pile(n // case["scenes"], seed + k) for k in range(case["scenes"])], 240)
         s["loop"] = case["loop"]
-    elif kind == "asleep":
-        w = _world([_pile(n, seed)], 900, sleeping=True)
+    elif kind == "resting":
+        w = _world([_mixed(n, seed, math.sqrt(n / 0.6), 3.0)], 900, sleeping=True)
     elif kind == "batch":
         w = _world(_batch(n, case["high"], 100_000 * (seed % 10_000)), 200)
     elif kind == "hulls":
@@ -335,7 +336,7 @@ def run(s):
         w.read_bodies(s["states"])
         w.write_states(s["states"])
         return s["states"]
-    if kind in ("mechanisms", "asleep"):
+    if kind in ("mechanisms", "resting"):
         return w.read_bodies(s["states"])
     return _resident(w)
 
@@ -396,6 +397,6 @@ def work(case):
     ops = pairs * _PAIR_OPS
     if kind in ("rollout", "rollout_mixed"):   # the forward, its recompute and the adjoint of each step
         unit, ops = 3 * unit, 4 * ops
-    host = 56 * bodies * (2 if case.get("loop") else 1) if kind in ("platform", "boxes", "mechanisms", "asleep") or \
+    host = 56 * bodies * (2 if case.get("loop") else 1) if kind in ("platform", "boxes", "mechanisms", "resting") or \
         case.get("loop") else 0
     return {"bytes": bodies * steps * unit + host, "flops": bodies * steps * ops}
