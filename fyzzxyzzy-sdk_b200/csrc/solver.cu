@@ -440,27 +440,35 @@ __global__ void __launch_bounds__(kScanThreads) k_island_compact(DevState s) {
         [&](uint32_t total) {
             *s.n_isl = total;
             s.isl_begin[total] = n;
-            for (int c = 0; c < 4; ++c) s.counters[kCntList + c] = 0u;
-            for (int c = 0; c < 5; ++c) s.counters[kCntList4 + c] = 0u;   // lists 4-5, work-queue tickets
+            for (int c = 0; c < DevState::kIslLists; ++c) s.counters[list_counter(c)] = 0u;
+            s.counters[kCntQueue] = 0u;   // the packed solver's work-queue ticket
         });
 }
 
 // Size classes of the islands (lists consumed by the partition and PGS
-// kernels of each class).
+// kernels of each class).  Pushes to one list are aggregated over the warp:
+// most islands of a world fall into the first few classes, and one atomic
+// an island on their counters would queue up.
+__device__ __forceinline__ void push_island(const DevState& s, int c, uint32_t isl) {
+    if (c < 0) return;
+    const uint32_t peers = __match_any_sync(__activemask(), c), lane = threadIdx.x & 31u;
+    const int leader = __ffs(peers) - 1;
+    uint32_t at = 0;
+    if (int(lane) == leader) at = atomicAdd(&s.counters[list_counter(c)], uint32_t(__popc(peers)));
+    at = __shfl_sync(peers, at, leader);
+    s.isl_list[c][at + __popc(peers & ((1u << lane) - 1u))] = isl;
+}
 __global__ void k_island_classes(DevState s) {
     const uint32_t ni = *s.n_isl;
     const uint32_t stride = gridDim.x * blockDim.x;
     for (uint32_t isl = blockIdx.x * blockDim.x + threadIdx.x; isl < ni; isl += stride) {
         const uint32_t n = s.isl_begin[isl + 1] - s.isl_begin[isl];
-        auto push = [&](int c) { s.isl_list[c][atomicAdd(&s.counters[list_counter(c)], 1u)] = isl; };
         // partitions
-        if (n > kSerialIsland && n <= kMidIsland) push(0);
-        else if (n > kMidIsland && n <= kBigIsland) push(2);
-        else if (n > kBigIsland) push(3);
+        push_island(s, n <= kSerialIsland ? -1 : n <= kMidIsland ? 0 : n <= kBigIsland ? 2 : 3, isl);
+        // reverse sweep of a rollout
+        push_island(s, n > s.isl_warp && n <= s.isl_mid ? 1 : -1, isl);
         // PGS
-        if (n > s.isl_thread && n <= s.isl_warp) push(5);
-        else if (n > s.isl_warp && n <= s.isl_mid) push(1);
-        else if (n > s.isl_mid && n <= kBigIsland) push(4);
+        push_island(s, pgs_list(n), isl);
     }
 }
 
@@ -1322,11 +1330,10 @@ __global__ void k_prep_contacts(DevState s) {
 }
 
 // ---------------- PGS ----------------
-// Velocity deltas of the solver bodies, addressed either by global body
-// (islands too large for shared memory) or by island-local slot in shared
-// memory.  Handle -1 is the static world (zero delta, never written).
+// Velocity deltas of the solver bodies in global memory, addressed by body
+// (islands beyond kBigIsland descriptors).  Handle -1 is the static world
+// (zero delta, never written).
 struct GlobalDeltas {
-    static constexpr bool kLocal = false;
     const DevState& s;
     __device__ __forceinline__ void load(int32_t b, v3& dv, v3& dw) const {
         if (b < 0) { dv = dw = {0, 0, 0}; return; }
@@ -1339,23 +1346,6 @@ struct GlobalDeltas {
         s.sb_dw[b] = st4(dw, 0.0f);
     }
 };
-struct LocalDeltas {
-    static constexpr bool kLocal = true;
-    float4* dv_;
-    float4* dw_;
-    __device__ __forceinline__ void load(int32_t l, v3& dv, v3& dw) const {
-        if (l < 0) { dv = dw = {0, 0, 0}; return; }
-        dv = ld3(dv_[l]);
-        dw = ld3(dw_[l]);
-    }
-    __device__ __forceinline__ void store(int32_t l, v3 dv, v3 dw) const {
-        if (l < 0) return;
-        dv_[l] = st4(dv, 0.0f);
-        dw_[l] = st4(dw, 0.0f);
-    }
-};
-__device__ __forceinline__ int32_t unpack_local(uint32_t v) { return v == 0xffffu ? -1 : int32_t(v); }
-
 // 32 bytes per thread in one load (sm_100's 256-bit global loads): a solver
 // row is two loads instead of four 128-bit ones.  Scattered rows (one
 // manager per thread) cost one L1 wavefront per thread and load instruction,
@@ -1372,9 +1362,8 @@ __device__ __forceinline__ void ldg256(const void* p, float4& a, float4& b) {
 
 // A joint's rows in order (scene.cpp:8905-8945) between bodies b0 / b1
 // (-1: the static world).
-template <class D>
 __device__ __forceinline__ void solve_joint(const DevState& s, uint32_t d, int32_t b0, int32_t b1, int it, int pos,
-                                            const D& D_) {
+                                            const GlobalDeltas& D_) {
     v3 av, aw, bv, bw;
     D_.load(b0, av, aw);
     D_.load(b1, bv, bw);
@@ -1400,22 +1389,11 @@ __device__ __forceinline__ void solve_joint(const DevState& s, uint32_t d, int32
 }
 
 // One descriptor's rows for pass `it` (scene.cpp:8853-9148), read from the
-// per-manager arrays prep writes.  lid carries the island-local bodies when
-// D addresses shared memory.
-// kEagerFriction issues the friction-row loads together with the normal
-// rows (lowest latency); otherwise they are issued after the normal rows
-// are solved (fewer registers).
-template <class D, bool kEagerFriction = true>
-__device__ void solve_desc(const DevState& s, uint32_t d, uint32_t lid, int it, int pos, int vel, const D& D_) {
+// per-manager arrays prep writes (islands beyond kBigIsland descriptors).
+__device__ void solve_desc(const DevState& s, uint32_t d, int it, int pos, int vel, const GlobalDeltas& D_) {
     if (d < s.n_joints) {
-        int32_t b0, b1;
-        if constexpr (D::kLocal) {
-            b0 = unpack_local(lid & 0xffffu);
-            b1 = unpack_local(lid >> 16);
-        } else {
-            b0 = is_dyn(s, s.j_a[d]) ? int32_t(s.j_a[d]) : -1;
-            b1 = is_dyn(s, s.j_b[d]) ? int32_t(s.j_b[d]) : -1;
-        }
+        const int32_t b0 = is_dyn(s, s.j_a[d]) ? int32_t(s.j_a[d]) : -1;
+        const int32_t b1 = is_dyn(s, s.j_b[d]) ? int32_t(s.j_b[d]) : -1;
         solve_joint(s, d, b0, b1, it, pos, D_);
         return;
     }
@@ -1439,38 +1417,22 @@ __device__ void solve_desc(const DevState& s, uint32_t d, uint32_t lid, int it, 
     const float4* fq = reinterpret_cast<const float4*>(s.frow + 4 * size_t(m));
     float4 n0[4], n1[4], n2[4], n3[4], f0[4], f1[4], f2[4];
     float fa[4];
-    if constexpr (kEagerFriction) {
-        // All four row slots of the manager are read without waiting for
-        // the header (unused slots are never consumed), so the row loads and
-        // the header load are in flight together.
-        const bool friction_pass = it >= pos || pos - it <= 3;
+    // All four row slots of the manager are read without waiting for the
+    // header (unused slots are never consumed), so the row loads and the
+    // header load are in flight together.
+    const bool friction_pass = it >= pos || pos - it <= 3;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            ldg256(nr + 4 * j, n0[j], n1[j]);
-            ldg256(nr + 4 * j + 2, n2[j], n3[j]);
-            if (friction_pass) {
-                float4 f3;
-                ldg256(fq + 4 * j, f0[j], f1[j]);
-                ldg256(fq + 4 * j + 2, f2[j], f3);
-                fa[j] = f3.x;
-            }
+    for (int j = 0; j < 4; ++j) {
+        ldg256(nr + 4 * j, n0[j], n1[j]);
+        ldg256(nr + 4 * j + 2, n2[j], n3[j]);
+        if (friction_pass) {
+            float4 f3;
+            ldg256(fq + 4 * j, f0[j], f1[j]);
+            ldg256(fq + 4 * j + 2, f2[j], f3);
+            fa[j] = f3.x;
         }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-            if (uint32_t(j) < hd.count) {
-                ldg256(nr + 4 * j, n0[j], n1[j]);
-                ldg256(nr + 4 * j + 2, n2[j], n3[j]);
-            }
     }
-    int32_t h0, h1;
-    if constexpr (D::kLocal) {
-        h0 = unpack_local(lid & 0xffffu);
-        h1 = unpack_local(lid >> 16);
-    } else {
-        h0 = hd.b0;
-        h1 = hd.b1;
-    }
+    const int32_t h0 = hd.b0, h1 = hd.b1;
     v3 av, aw, bv, bw;
     D_.load(h0, av, aw);
     D_.load(h1, bv, bw);
@@ -1498,16 +1460,6 @@ __device__ void solve_desc(const DevState& s, uint32_t d, uint32_t lid, int it, 
         nsum += ni;
     }
     if (friction) {
-        if constexpr (!kEagerFriction) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-                if (uint32_t(j) < 2 * hd.anchors) {
-                    float4 f3;
-                    ldg256(fq + 4 * j, f0[j], f1[j]);
-                    ldg256(fq + 4 * j + 2, f2[j], f3);
-                    fa[j] = f3.x;
-                }
-        }
         const float coeff = hd.anchors == 2 ? 0.5f : 1.0f;
         const float ms = hd.sf * coeff * nsum;
         const float md = hd.df * coeff * nsum;
@@ -1543,206 +1495,6 @@ __device__ void solve_desc(const DevState& s, uint32_t d, uint32_t lid, int it, 
     D_.store(h1, bv, bw);
 }
 
-// ---- placed-order planes (DevState::slot_rows) ----
-// The island solvers copy each manager's rows once per step into planes
-// indexed by placed slot, keeping only what the passes read.  Slots come in
-// blocks of 32; a block holds kSlotVecPlanes float4 planes of 32 records --
-// 0: {sf, df, ima, imb}; normal row j at 1 + 3j: {n.xyz, ra.x} {ra.yz,
-// rb.xy} {rb.z, vel_mult, imp_mult, max_impulse}; friction row k at
-// 13 + 3k: {t.xyz, ra.x} {ra.yz, rb.xy} {rb.z, vel_mult, bias, target} --
-// and, after all blocks' vector planes, kSlotScalarPlanes float planes of
-// 32 records -- biased j (0 + j), unbiased j (4 + j), normal applied j
-// (8 + j), friction applied k (12 + k).  Lanes solving consecutive slots
-// read consecutive records, a plane is a constant offset from the slot's
-// first record, and only the rows a manager has are read (its point and
-// anchor counts travel with its island-local bodies).
-struct SlotPtr {
-    float4* v;   // plane 0 record of the slot; plane p at v + 32 p
-    float* f;    // scalar plane 0 record; plane p at f + 32 p
-    __device__ __forceinline__ SlotPtr(const DevState& s, uint32_t slot) {
-        const size_t blk = slot >> 5, lane = slot & 31u;
-        v = s.slot_rows + blk * (32u * kSlotVecPlanes) + lane;
-        const size_t nblk = (size_t(s.desc_cap) + 31u) >> 5;
-        f = reinterpret_cast<float*>(s.slot_rows + nblk * (32u * kSlotVecPlanes)) + blk * (32u * kSlotScalarPlanes) +
-            lane;
-    }
-    __device__ __forceinline__ float4& vec(uint32_t p) const { return v[32 * p]; }
-    __device__ __forceinline__ float& sca(uint32_t p) const { return f[32 * p]; }
-};
-// Island-local bodies in 13 bits each (0x1fff: the static world), the
-// manager's point count in bits 13-15 and anchor count in bits 29-31.
-__device__ __forceinline__ uint32_t pack_slot_meta(uint32_t lid, uint32_t count, uint32_t anchors) {
-    const uint32_t lo = lid & 0xffffu, hi = lid >> 16;
-    const uint32_t lo13 = lo == 0xffffu ? 0x1fffu : lo, hi13 = hi == 0xffffu ? 0x1fffu : hi;
-    return lo13 | (count << 13) | (hi13 << 16) | (anchors << 29);
-}
-__device__ __forceinline__ int32_t unpack_local13(uint32_t v) {
-    v &= 0x1fffu;
-    return v == 0x1fffu ? -1 : int32_t(v);
-}
-// Copies manager m's rows to slot `slot` and returns its island-local
-// bodies with the counts (pack_slot_meta).
-__device__ __forceinline__ uint32_t stage_slot_rows(const DevState& s, uint32_t m, uint32_t slot, uint32_t lid) {
-    const float4* nr = reinterpret_cast<const float4*>(s.nrow + 4 * size_t(m));
-    const float4* fq = reinterpret_cast<const float4*>(s.frow + 4 * size_t(m));
-    const SlotPtr P(s, slot);
-    float4 h0, h1, q[2][4];
-    // rows 0-1 travel with the header; the rest once the counts are known
-    ldg256(s.mh + m, h0, h1);
-    ldg256(nr, q[0][0], q[0][1]);
-    ldg256(nr + 2, q[0][2], q[0][3]);
-    ldg256(nr + 4, q[1][0], q[1][1]);
-    ldg256(nr + 6, q[1][2], q[1][3]);
-    const uint32_t count = min(__float_as_uint(h0.z), 4u), anchors = min(__float_as_uint(h0.w), 2u);
-    P.vec(0) = h1;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if (uint32_t(j) >= count) break;
-        if (j == 2) {
-            ldg256(nr + 8, q[0][0], q[0][1]);
-            ldg256(nr + 10, q[0][2], q[0][3]);
-            if (count > 3) {
-                ldg256(nr + 12, q[1][0], q[1][1]);
-                ldg256(nr + 14, q[1][2], q[1][3]);
-            }
-        }
-        const float4* r = q[j & 1];
-        P.vec(1 + 3 * j) = r[0];
-        P.vec(2 + 3 * j) = r[1];
-        P.vec(3 + 3 * j) = make_float4(r[2].x, r[2].y, r[2].z, r[3].z);
-        P.sca(0 + j) = r[2].w;
-        P.sca(4 + j) = r[3].x;
-        P.sca(8 + j) = r[3].y;
-    }
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (uint32_t(k) >= 2 * anchors) break;
-        float4 f0, f1, f2, f3;
-        ldg256(fq + 4 * k, f0, f1);
-        ldg256(fq + 4 * k + 2, f2, f3);
-        P.vec(13 + 3 * k) = f0;
-        P.vec(14 + 3 * k) = f1;
-        P.vec(15 + 3 * k) = f2;
-        P.sca(12 + k) = f3.x;
-    }
-    return pack_slot_meta(lid, count, anchors);
-}
-
-// solve_desc on the placed-order planes: descriptor d in slot `slot`, its
-// island-local bodies and counts in meta (pack_slot_meta).  The same
-// arithmetic in the same order; the impulses of the last pass also go back
-// to the per-manager rows, where the events, the force thresholds and the
-// rollouts read them.
-template <class D, bool kEagerFriction = true>
-__device__ void solve_slot(const DevState& s, uint32_t d, uint32_t meta, int it, int pos, int vel, const D& D_,
-                           uint32_t slot) {
-    const int32_t h0 = unpack_local13(meta), h1 = unpack_local13(meta >> 16);
-    if (d < s.n_joints) {
-        solve_joint(s, d, h0, h1, it, pos, D_);
-        return;
-    }
-    const uint32_t m = d - s.n_joints;
-    const uint32_t count = (meta >> 13) & 7u, anchors = meta >> 29;
-    const bool last = it + 1 == pos + vel;
-    const bool friction = (it >= pos || pos - it <= 3) && anchors;
-    const SlotPtr P(s, slot);
-    const float4 hd = P.vec(0);   // {sf, df, ima, imb}
-    const float ima = hd.z, imb = hd.w;        // 0 for the static world
-    float4 n0[4], n1[4], n2[4], f0[4], f1[4], f2[4];
-    float ne[4], na[4], fa[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j)
-        if (uint32_t(j) < count) {
-            n0[j] = P.vec(1 + 3 * j);
-            n1[j] = P.vec(2 + 3 * j);
-            n2[j] = P.vec(3 + 3 * j);
-            ne[j] = P.sca((it < pos ? 0 : 4) + j);
-            na[j] = P.sca(8 + j);
-        }
-    if constexpr (kEagerFriction) {
-        if (friction) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (uint32_t(k) < 2 * anchors) {
-                    f0[k] = P.vec(13 + 3 * k);
-                    f1[k] = P.vec(14 + 3 * k);
-                    f2[k] = P.vec(15 + 3 * k);
-                    fa[k] = P.sca(12 + k);
-                }
-        }
-    }
-    v3 av, aw, bv, bw;
-    D_.load(h0, av, aw);
-    D_.load(h1, bv, bw);
-    float nsum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        if (uint32_t(j) >= count) break;
-        const v3 n = {n0[j].x, n0[j].y, n0[j].z};
-        const v3 ra = {n0[j].w, n1[j].x, n1[j].y};
-        const v3 rb = {n1[j].z, n1[j].w, n2[j].x};
-        const float vel_mult = n2[j].y, imp_mult = n2[j].z, max_impulse = n2[j].w;
-        const float applied = na[j];
-        const float nvel = vdot(n, av) - vdot(n, bv) + vdot(aw, ra) - vdot(bw, rb);
-        const float dc = smax(-nvel * vel_mult + ne[j], -applied);
-        const float ni = smin(max_impulse, imp_mult * applied + dc);
-        const float dl = ni - applied;
-        const float da = dl * ima, db = dl * imb;
-        av = {av.x + n.x * da, av.y + n.y * da, av.z + n.z * da};
-        bv = {bv.x - n.x * db, bv.y - n.y * db, bv.z - n.z * db};
-        aw = {aw.x + ra.x * dl, aw.y + ra.y * dl, aw.z + ra.z * dl};
-        bw = {bw.x - rb.x * dl, bw.y - rb.y * dl, bw.z - rb.z * dl};
-        P.sca(8 + j) = ni;
-        if (last) s.nrow[4 * size_t(m) + j].applied = ni;
-        if (s.tape_n) s.tape_n[(size_t(it) * s.pair_cap + m) * 4 + j] = ni;
-        nsum += ni;
-    }
-    if (friction) {
-        if constexpr (!kEagerFriction) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-                if (uint32_t(k) < 2 * anchors) {
-                    f0[k] = P.vec(13 + 3 * k);
-                    f1[k] = P.vec(14 + 3 * k);
-                    f2[k] = P.vec(15 + 3 * k);
-                    fa[k] = P.sca(12 + k);
-                }
-        }
-        const float coeff = anchors == 2 ? 0.5f : 1.0f;
-        const float ms = hd.x * coeff * nsum;
-        const float md = hd.y * coeff * nsum;
-        bool broken = false;
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            if (uint32_t(k) >= 2 * anchors) break;
-            const v3 n = {f0[k].x, f0[k].y, f0[k].z};
-            const v3 ra = {f0[k].w, f1[k].x, f1[k].y};
-            const v3 rb = {f1[k].z, f1[k].w, f2[k].x};
-            const float vel_mult = f2[k].y, target = f2[k].w, applied = fa[k];
-            const float td = vdot(n, av) - vdot(n, bv) + vdot(aw, ra) - vdot(bw, rb);
-            const float bias = it < pos ? f2[k].z : 0.0f;
-            const float cand = applied + (target - bias - td) * vel_mult;
-            const bool clamped = fabsf(cand) > ms;
-            const float nx = clamped ? smin(md, smax(-md, cand)) : cand;
-            const float dl = nx - applied;
-            const float da = dl * ima, db = dl * imb;
-            av = {av.x + n.x * da, av.y + n.y * da, av.z + n.z * da};
-            bv = {bv.x - n.x * db, bv.y - n.y * db, bv.z - n.z * db};
-            aw = {aw.x + ra.x * dl, aw.y + ra.y * dl, aw.z + ra.z * dl};
-            bw = {bw.x - rb.x * dl, bw.y - rb.y * dl, bw.z - rb.z * dl};
-            P.sca(12 + k) = nx;
-            if (last) s.frow[4 * size_t(m) + k].applied = nx;
-            if (s.tape_f) s.tape_f[(size_t(it) * s.pair_cap + m) * 4 + k] = nx;
-            broken |= clamped;
-        }
-        if (last) {
-            FrictionHist& h = s.cur.fric[s.man_list[m]];
-            h.meta = (h.meta & ~256u) | (broken ? 256u : 0u);
-        }
-    }
-    D_.store(h0, av, aw);
-    D_.store(h1, bv, bw);
-}
 __device__ __forceinline__ void save_motion(const DevState& s, uint32_t d) {
     int32_t b0, b1;
     if (d < s.n_joints) {
@@ -1756,178 +1508,515 @@ __device__ __forceinline__ void save_motion(const DevState& s, uint32_t d) {
     if (b1 >= 0) { s.sb_mdv[b1] = s.sb_dv[b1]; s.sb_mdw[b1] = s.sb_dw[b1]; }
 }
 
-// Copies of an island's shared-memory deltas to the solver bodies.
-__device__ __forceinline__ void island_deltas_out(float4* dst_v, float4* dst_w, const int32_t* ib, uint32_t nb,
-                                                  const float4* sdv, const float4* sdw, uint32_t t0,
-                                                  uint32_t nt) {
-    for (uint32_t l = t0; l < nb; l += nt) {
-        const int32_t g = ib[l];
-        dst_v[g] = sdv[l];
-        dst_w[g] = sdw[l];
-    }
+// ---- islands of at most kBigIsland descriptors ----
+// Gauss-Seidel over an island is a chain of passes x levels dependent row
+// solves.  With the rows in global memory a link of that chain took 1.2 us
+// in a small island and 2.7 us in one of 1,900 descriptors, most of it the
+// round trips of up to 464 bytes a descriptor and the instruction stream
+// around them; the eight rows' arithmetic itself is 885 cycles as scalar
+// code.  A unit of work (one island, or a group of small islands whose
+// levels are stepped together to fill the lanes) therefore reads its rows
+// into shared memory once, laid out so that the two bodies' components are
+// register pairs: sm_100's packed f32x2 multiplies and adds (each half
+// rounded like the scalar operation) then do both bodies at once, 685 cycles
+// for eight rows.  The row loop is unrolled (rolled: 2,160 cycles) and does
+// nothing but the rows; impulses leave through separate loops.  Four lanes a
+// descriptor, one per velocity vector, were slower (1,043 cycles: four
+// 26-cycle shuffles a row), and one thread a descriptor with its rows in
+// registers leaves all lanes but a level's idle.
+//
+// A descriptor's record (slot i of CAP; planes of float4, then of float):
+//   contact  0 {normal, max_impulse}, 1 {inverse masses, friction
+//            coefficients}, 2 {tangent 0, tangent 1.x}, 3 + 2j {ra.x, rb.x,
+//            ra.y, rb.y} 4 + 2j {ra.z, rb.z, vel_mult, error} of normal row
+//            j, 11 + 2k / 12 + 2k the same of friction row k (its error is
+//            target - bias); scalars 0 + j and 4 + k applied, 8 + j
+//            imp_mult, 12 / 13 tangent 1.y / z, 14 broken (set by the
+//            friction rows), and what the velocity passes read instead: 15 + j
+//            unbiased error, 19 + k target.  A manager's normal rows share
+//            the normal and its friction rows the two tangents
+//            (k_prep_contacts).
+//   joint    3q {ang_a.x, ang_b.x, ang_a.y, ang_b.y} 3q + 1 {ang_a.z,
+//            ang_b.z, vel_mult, constant} 3q + 2 {axis, -} of row q, 18
+//            {inverse masses, -, -}; scalars 0 + q applied, 15 + q unbiased.
+constexpr uint32_t kRowVec = 19, kRowScalar = 23;
+__device__ __forceinline__ uint64_t pair2(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpair(uint64_t v, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+// Packed arithmetic rounded like the scalar operations.  The product is an
+// fma with a zero the compiler cannot see through (DevState::neg_zero2: -0,
+// which leaves every product as it is, signed zeros included): written as
+// mul.rn.f32x2 followed by add.rn.f32x2, ptxas 12.9 contracts the two into
+// one fma, whose single rounding differs (13 % of random operands).
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b, uint64_t nz) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(nz));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+// Both bodies' deltas, component by component ({a, b} pairs).
+struct Pairs { uint64_t x, y, z; };
+__device__ __forceinline__ Pairs pairs(v3 a, v3 b) { return {pair2(a.x, b.x), pair2(a.y, b.y), pair2(a.z, b.z)}; }
+__device__ __forceinline__ uint64_t dot2(const Pairs& j, const Pairs& v, uint64_t nz) {   // vdot of each half
+    return add2(add2(mul2(j.x, v.x, nz), mul2(j.y, v.y, nz)), mul2(j.z, v.z, nz));
+}
+__device__ __forceinline__ Pairs axpy2(const Pairs& v, const Pairs& j, uint64_t k, uint64_t nz) {
+    return {add2(v.x, mul2(j.x, k, nz)), add2(v.y, mul2(j.y, k, nz)), add2(v.z, mul2(j.z, k, nz))};
+}
+// Slot word: local bodies in bits 0-12 and 13-25 (0x1fff: the static
+// world), contact points or joint rows in bits 26-28, anchors in bits
+// 29-30, bit 31 a joint.
+constexpr uint32_t kNoBody = 0x1fffu;
+__device__ __forceinline__ uint32_t slot_word(uint32_t la, uint32_t lb, uint32_t count, uint32_t anchors, bool joint) {
+    return (la & kNoBody) | ((lb & kNoBody) << 13) | (count << 26) | (anchors << 29) | (joint ? 1u << 31 : 0u);
 }
 
-// One thread per tiny island (<= kTinyIsland descriptors): the island's
-// placed descriptors are solved in order (level by level, the order the
-// wider kernels use, since a level's descriptors share no body) with the
-// deltas in the thread's slice of shared memory.  Tiny islands (a body
-// resting alone, a short chain) are most islands of a spread-out scene; a
-// warp each would leave 31 lanes idle for all five passes.
-constexpr uint32_t kTinyIsland = 8;
-constexpr uint32_t kPgsThreadBlock = 128;
-__global__ void __launch_bounds__(kPgsThreadBlock) k_pgs_thread(DevState s) {
-    __shared__ float4 sh[kPgsThreadBlock][2][kTinyIsland + 1];
-    const uint32_t ni = *s.n_isl;
-    const int pos = s.pos_iters, vel = s.vel_iters < 1 ? 1 : s.vel_iters;
-    float4* sdv = sh[threadIdx.x][0];
-    float4* sdw = sh[threadIdx.x][1];
-    const LocalDeltas D{sdv, sdw};
-    const float4 zero = make_float4(0, 0, 0, 0);
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t isl = blockIdx.x * blockDim.x + threadIdx.x; isl < ni; isl += stride) {
-        const uint32_t begin = s.isl_begin[isl], end = s.isl_begin[isl + 1];
-        if (end - begin > s.isl_thread) continue;
-        const uint32_t nb = s.isl_nbod[isl];
-        const int32_t* ib = s.isl_bod + begin + isl;
-        for (uint32_t l = 0; l < nb; ++l) { sdv[l] = zero; sdw[l] = zero; }
-        for (int it = 0; it < pos + vel; ++it) {
-            for (uint32_t i = begin; i < end; ++i)
-                solve_desc<LocalDeltas>(s, s.d_val2[i], s.d_lbod[i], it, pos, vel, D);
-            if (it + 1 == pos) island_deltas_out(s.sb_mdv, s.sb_mdw, ib, nb, sdv, sdw, 0u, 1u);
-        }
-        island_deltas_out(s.sb_dv, s.sb_dw, ib, nb, sdv, sdw, 0u, 1u);
+// Shared memory of a unit of at most CAP descriptors and NBOD bodies a CTA
+// on a cluster of CL CTAs (slot i on CTA i % CL, body l on CTA l % CL).
+template <uint32_t CAP, uint32_t NBOD, uint32_t NT, uint32_t CL> struct Unit {
+    static constexpr uint32_t kBounds = kMaxLevels + 1;
+    static constexpr size_t kBytes = size_t(CAP) * (16 * kRowVec + 4 * kRowScalar + 8) + size_t(NBOD) * 32 + kBounds * 4;
+    static_assert(CAP % 4 == 0 && NBOD * CL <= kNoBody, "slot planes and body words");
+    float4* vec;         // kRowVec planes of CAP
+    float4* bd;          // body deltas: NBOD linear, NBOD angular
+    float* sca;          // kRowScalar planes of CAP
+    uint32_t *word, *desc;
+    uint32_t* bound;     // level starts (this CTA's slots)
+    __device__ __forceinline__ explicit Unit(float4* sm) {
+        vec = sm;
+        bd = vec + kRowVec * CAP;
+        sca = reinterpret_cast<float*>(bd + 2 * NBOD);
+        word = reinterpret_cast<uint32_t*>(sca + kRowScalar * CAP);
+        desc = word + CAP;
+        bound = desc + CAP;
     }
-}
+    __device__ __forceinline__ float4& v(uint32_t p, uint32_t i) const { return vec[p * CAP + i]; }
+    __device__ __forceinline__ float& f(uint32_t p, uint32_t i) const { return sca[p * CAP + i]; }
+    static __device__ __forceinline__ void barrier() {
+        if constexpr (CL > 1) {
+            __syncwarp();
+            asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    }
+    // Deltas of local body l (kNoBody: the static world, zero and never
+    // written), in the shared memory of CTA l % CL.
+    __device__ __forceinline__ uint32_t remote(uint32_t l) const {
+        uint32_t r;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;"
+            : "=r"(r) : "r"(uint32_t(__cvta_generic_to_shared(bd)) + (l / CL) * 16u), "r"(l % CL));
+        return r;
+    }
+    static __device__ __forceinline__ v3 remote_ld(uint32_t a) {
+        v3 x;
+        float w;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(x.x), "=f"(x.y), "=f"(x.z), "=f"(w) : "r"(a) : "memory");
+        return x;
+    }
+    static __device__ __forceinline__ void remote_st(uint32_t a, v3 x) {
+        asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(x.x), "f"(x.y), "f"(x.z), "f"(0.0f)
+                     : "memory");
+    }
+    __device__ __forceinline__ void load_body(uint32_t l, v3& dv, v3& dw) const {
+        if (l == kNoBody) { dv = dw = {0, 0, 0}; return; }
+        if constexpr (CL == 1) {
+            dv = ld3(bd[l]);
+            dw = ld3(bd[NBOD + l]);
+        } else {
+            const uint32_t a = remote(l);
+            dv = remote_ld(a);
+            dw = remote_ld(a + NBOD * 16u);
+        }
+    }
+    __device__ __forceinline__ void store_body(uint32_t l, v3 dv, v3 dw) const {
+        if (l == kNoBody) return;
+        if constexpr (CL == 1) {
+            bd[l] = st4(dv, 0.0f);
+            bd[NBOD + l] = st4(dw, 0.0f);
+        } else {
+            const uint32_t a = remote(l);
+            remote_st(a, dv);
+            remote_st(a + NBOD * 16u, dw);
+        }
+    }
 
-// One warp per small island (kTinyIsland < descriptors <= kSmallIsland, so
-// <= 97 bodies): the island's deltas live in this warp's slice of shared
-// memory.
-constexpr uint32_t kWarpBodies = kSmallIsland + 1;
-constexpr uint32_t kPgsWarpsPerBlock = 4;
-__global__ void __launch_bounds__(kPgsWarpsPerBlock * 32, 3) k_pgs_warp(DevState s, const uint32_t* lvl_bound) {
-    __shared__ float4 sh[kPgsWarpsPerBlock][2][kWarpBodies];
-    __shared__ uint32_t sdesc[kPgsWarpsPerBlock][2][kSmallIsland];   // descriptor, local bodies per slot
-    __shared__ uint32_t sbound[kPgsWarpsPerBlock][kSmallIsland + 1];
-    const uint32_t n_list = s.counters[list_counter(5)];
-    const uint32_t* list = s.isl_list[5];
-    const uint32_t lane = threadIdx.x & 31;
-    const uint32_t wib = threadIdx.x >> 5;
-    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    const int pos = s.pos_iters, vel = s.vel_iters < 1 ? 1 : s.vel_iters;
-    float4* sdv = sh[wib][0];
-    float4* sdw = sh[wib][1];
-    const LocalDeltas D{sdv, sdw};
-    const float4 zero = make_float4(0, 0, 0, 0);
-    for (uint32_t k = warp;;) {
-        if (s.work_queue) {
-            uint32_t t = 0;
-            if (lane == 0) t = atomicAdd(&s.counters[kCntQueue], 1u);
-            k = __shfl_sync(0xffffffffu, t, 0);
-        }
-        if (k >= n_list) break;
-        const uint32_t isl = list[k];
-        if (!s.work_queue) k += nwarps;
-        const uint32_t begin = s.isl_begin[isl], end = s.isl_begin[isl + 1];
-        const uint32_t nlev = s.isl_end[isl];
-        const uint32_t nb = s.isl_nbod[isl];
-        const int32_t* ib = s.isl_bod + begin + isl;
-        const uint32_t* bound = lvl_bound + begin + isl;
-        uint32_t* sd = sdesc[wib][0];
-        uint32_t* sl = sdesc[wib][1];
-        uint32_t* sb = sbound[wib];
-        for (uint32_t l = lane; l < nb; l += 32) { sdv[l] = zero; sdw[l] = zero; }
-        for (uint32_t i = lane; i < end - begin; i += 32) {
-            const uint32_t d = s.d_val2[begin + i], lid = s.d_lbod[begin + i];
-            sd[i] = d;
-            sl[i] = d >= s.n_joints ? stage_slot_rows(s, d - s.n_joints, begin + i, lid) : pack_slot_meta(lid, 0u, 0u);
-        }
-        for (uint32_t l = lane; l <= nlev; l += 32) sb[l] = bound[l] - begin;
-        __syncwarp();
-        for (int it = 0; it < pos + vel; ++it) {
-            for (uint32_t l = 0; l < nlev; ++l) {
-                const uint32_t lb = sb[l], le = sb[l + 1];
-                for (uint32_t i = lb + lane; i < le; i += 32)
-                    solve_slot<LocalDeltas>(s, sd[i], sl[i], it, pos, vel, D, begin + i);
-                __syncwarp();
+    // Descriptor d with local bodies la / lb into slot i.
+    __device__ __forceinline__ void load_slot(const DevState& s, uint32_t i, uint32_t d, uint32_t la, uint32_t lb) const {
+        desc[i] = d;
+        if (d < s.n_joints) {
+            const float4* jr = reinterpret_cast<const float4*>(s.jrow + s.j_row[d]);
+            const uint32_t nr = joint_row_count(s.j_kind[d]);
+            word[i] = slot_word(la, lb, nr, 0u, true);
+            for (uint32_t q = 0; q < nr; ++q) {
+                float4 a, b, c, e;   // {axis, ang_a.x} {ang_a.yz, ang_b.xy} {ang_b.z, ima, imb, constant} {unbiased, vel_mult, applied}
+                ldg256(jr + 4 * q, a, b);
+                ldg256(jr + 4 * q + 2, c, e);
+                v(3 * q, i) = make_float4(a.w, b.z, b.x, b.w);
+                v(3 * q + 1, i) = make_float4(b.y, c.x, e.y, c.w);
+                v(3 * q + 2, i) = make_float4(a.x, a.y, a.z, 0.0f);
+                f(q, i) = e.z;
+                f(15 + q, i) = e.x;
+                if (q == 0) v(18, i) = make_float4(c.y, c.z, 0.0f, 0.0f);
             }
+            return;
+        }
+        const uint32_t m = d - s.n_joints;
+        const float4* nr = reinterpret_cast<const float4*>(s.nrow + 4 * size_t(m));
+        const float4* fq = reinterpret_cast<const float4*>(s.frow + 4 * size_t(m));
+        // row 0 travels with the header; the rest once the counts are known
+        float4 h0, h1, r[4][4];
+        ldg256(s.mh + m, h0, h1);
+        ldg256(nr, r[0][0], r[0][1]);
+        ldg256(nr + 2, r[0][2], r[0][3]);
+        const uint32_t count = min(__float_as_uint(h0.z), 4u), anchors = min(__float_as_uint(h0.w), 2u);
+        word[i] = slot_word(la, lb, count, anchors, false);
+        const float coeff = anchors == 2 ? 0.5f : 1.0f;
+#pragma unroll
+        for (int j = 1; j < 4; ++j)
+            if (uint32_t(j) < count) {
+                ldg256(nr + 4 * j, r[j][0], r[j][1]);
+                ldg256(nr + 4 * j + 2, r[j][2], r[j][3]);
+            }
+        v(0, i) = make_float4(r[0][0].x, r[0][0].y, r[0][0].z, r[0][3].z);
+        v(1, i) = make_float4(h1.z, h1.w, h1.x * coeff, h1.y * coeff);
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (uint32_t(j) < count) {   // {n, ra.x} {ra.yz, rb.xy} {rb.z, vel_mult, imp_mult, biased} {unbiased, applied, max_impulse}
+                const float4* q = r[j];
+                v(3 + 2 * j, i) = make_float4(q[0].w, q[1].z, q[1].x, q[1].w);
+                v(4 + 2 * j, i) = make_float4(q[1].y, q[2].x, q[2].y, q[2].w);
+                f(j, i) = q[3].y;
+                f(8 + j, i) = q[2].z;
+                f(15 + j, i) = q[3].x;
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (uint32_t(k) < 2 * anchors) {
+                ldg256(fq + 4 * k, r[k][0], r[k][1]);
+                ldg256(fq + 4 * k + 2, r[k][2], r[k][3]);
+            }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (uint32_t(k) < 2 * anchors) {   // {t, ra.x} {ra.yz, rb.xy} {rb.z, vel_mult, bias, target} {applied}
+                const float4* q = r[k];
+                if (k == 1) {
+                    v(2, i) = make_float4(r[0][0].x, r[0][0].y, r[0][0].z, q[0].x);
+                    f(12, i) = q[0].y;
+                    f(13, i) = q[0].z;
+                }
+                v(11 + 2 * k, i) = make_float4(q[0].w, q[1].z, q[1].x, q[1].w);
+                v(12 + 2 * k, i) = make_float4(q[1].y, q[2].x, q[2].y, q[2].w - q[2].z);
+                f(4 + k, i) = q[3].x;
+                f(19 + k, i) = q[2].w;
+            }
+    }
+    // Slot i's errors and targets of the velocity passes.
+    __device__ __forceinline__ void enter_velocity(uint32_t i) const {
+        const uint32_t w = word[i], count = (w >> 26) & 7u, rows = w >> 31 ? 0u : 2u * ((w >> 29) & 3u);
+        if (w >> 31) {
+            for (uint32_t q = 0; q < count; ++q) v(3 * q + 1, i).w = f(15 + q, i);
+            return;
+        }
+        for (uint32_t j = 0; j < count; ++j) v(4 + 2 * j, i).w = f(15 + j, i);
+        for (uint32_t k = 0; k < rows; ++k) v(12 + 2 * k, i).w = f(19 + k, i);
+    }
+
+    // Slot i's rows in one pass (friction: with its friction rows): the
+    // arithmetic and order of solve_desc, both bodies at once.
+    __device__ __forceinline__ void solve(uint32_t i, bool friction, uint64_t nz) const {
+        const uint32_t w = word[i], la = w & kNoBody, lb = (w >> 13) & kNoBody, count = (w >> 26) & 7u;
+        v3 av, aw, bv, bw;
+        load_body(la, av, aw);
+        load_body(lb, bv, bw);
+        Pairs A = pairs(aw, bw);
+        if (w >> 31) {
+            const float4 im = v(18, i);
+#pragma unroll
+            for (uint32_t q = 0; q < 6; ++q) {
+                if (q >= count) break;
+                const float4 a = v(3 * q, i), b = v(3 * q + 1, i), c = v(3 * q + 2, i);
+                const float applied = f(q, i);
+                const Pairs J = {pair2(a.x, a.y), pair2(a.z, a.w), pair2(b.x, b.y)};
+                float ga, gb;
+                unpair(dot2(J, A, nz), ga, gb);
+                const float nd = c.x * (av.x - bv.x) + c.y * (av.y - bv.y) + c.z * (av.z - bv.z) + ga - gb;
+                const float nx = sclamp(applied + nd * b.z + b.w, -FLT_MAX, FLT_MAX);
+                const float imp = nx - applied;
+                const float ia = imp * im.x, ib = imp * im.y;
+                av = {av.x + ia * c.x, av.y + ia * c.y, av.z + ia * c.z};
+                bv = {bv.x - ib * c.x, bv.y - ib * c.y, bv.z - ib * c.z};
+                A = axpy2(A, J, pair2(imp, -imp), nz);
+                f(q, i) = nx;
+            }
+        } else {
+            Pairs V = pairs(av, bv);
+            const float4 h0 = v(0, i), h1 = v(1, i);   // inverse masses: 0 for the static world
+            const Pairs N = {pair2(h0.x, h0.x), pair2(h0.y, h0.y), pair2(h0.z, h0.z)};
+            float nsum = 0.0f;
+#pragma unroll
+            for (uint32_t j = 0; j < 4; ++j) {
+                if (j >= count) break;
+                const float4 a = v(3 + 2 * j, i), b = v(4 + 2 * j, i);
+                const float applied = f(j, i), im = f(8 + j, i);
+                const Pairs J = {pair2(a.x, a.y), pair2(a.z, a.w), pair2(b.x, b.y)};
+                float na, nb, ga, gb;
+                unpair(dot2(N, V, nz), na, nb);
+                unpair(dot2(A, J, nz), ga, gb);
+                const float nvel = na - nb + ga - gb;
+                const float dc = smax(-nvel * b.z + b.w, -applied);
+                const float ni = smin(h0.w, im * applied + dc);
+                const float dl = ni - applied;
+                V = axpy2(V, N, pair2(dl * h1.x, -(dl * h1.y)), nz);
+                A = axpy2(A, J, pair2(dl, -dl), nz);
+                f(j, i) = ni;
+                nsum += ni;
+            }
+            const uint32_t rows = friction ? 2u * ((w >> 29) & 3u) : 0u;
+            if (rows) {
+                const float ms = h1.z * nsum, md = h1.w * nsum;
+                const float4 tt = v(2, i);
+                const float ty = f(12, i), tz = f(13, i);
+                const Pairs T[2] = {{pair2(tt.x, tt.x), pair2(tt.y, tt.y), pair2(tt.z, tt.z)},
+                                    {pair2(tt.w, tt.w), pair2(ty, ty), pair2(tz, tz)}};
+                bool broken = false;
+#pragma unroll
+                for (uint32_t k = 0; k < 4; ++k) {
+                    if (k >= rows) break;
+                    const float4 a = v(11 + 2 * k, i), b = v(12 + 2 * k, i);
+                    const float applied = f(4 + k, i);
+                    const Pairs J = {pair2(a.x, a.y), pair2(a.z, a.w), pair2(b.x, b.y)};
+                    float na, nb, ga, gb;
+                    unpair(dot2(T[k & 1], V, nz), na, nb);
+                    unpair(dot2(A, J, nz), ga, gb);
+                    const float td = na - nb + ga - gb;
+                    const float cand = applied + (b.w - td) * b.z;
+                    const bool clamped = fabsf(cand) > ms;
+                    const float nx = clamped ? smin(md, smax(-md, cand)) : cand;
+                    const float dl = nx - applied;
+                    V = axpy2(V, T[k & 1], pair2(dl * h1.x, -(dl * h1.y)), nz);
+                    A = axpy2(A, J, pair2(dl, -dl), nz);
+                    f(4 + k, i) = nx;
+                    broken |= clamped;
+                }
+                f(14, i) = broken ? 1.0f : 0.0f;
+            }
+            unpair(V.x, av.x, bv.x);
+            unpair(V.y, av.y, bv.y);
+            unpair(V.z, av.z, bv.z);
+        }
+        unpair(A.x, aw.x, bw.x);
+        unpair(A.y, aw.y, bw.y);
+        unpair(A.z, aw.z, bw.z);
+        store_body(la, av, aw);
+        store_body(lb, bv, bw);
+    }
+    // Slot i's impulses: to the rollout's tape after every pass, to the
+    // per-manager rows after the last (events, force thresholds and rollouts
+    // read them there).
+    __device__ __forceinline__ void tape_slot(const DevState& s, uint32_t i, int it, bool friction) const {
+        const uint32_t w = word[i], count = (w >> 26) & 7u, d = desc[i];
+        if (w >> 31) {
+            for (uint32_t q = 0; q < count; ++q) s.tape_j[size_t(it) * s.n_jrows + s.j_row[d] + q] = f(q, i);
+            return;
+        }
+        const size_t at = (size_t(it) * s.pair_cap + (d - s.n_joints)) * 4;
+        for (uint32_t j = 0; j < count; ++j) s.tape_n[at + j] = f(j, i);
+        if (friction)
+            for (uint32_t k = 0; k < 2u * ((w >> 29) & 3u); ++k) s.tape_f[at + k] = f(4 + k, i);
+    }
+    __device__ __forceinline__ void publish_slot(const DevState& s, uint32_t i, bool friction) const {
+        const uint32_t w = word[i], count = (w >> 26) & 7u, anchors = (w >> 29) & 3u, d = desc[i];
+        if (w >> 31) {
+            for (uint32_t q = 0; q < count; ++q) s.jrow[s.j_row[d] + q].applied = f(q, i);
+            return;
+        }
+        const uint32_t m = d - s.n_joints;
+        for (uint32_t j = 0; j < count; ++j) s.nrow[4 * size_t(m) + j].applied = f(j, i);
+        if (!friction || !anchors) return;
+        for (uint32_t k = 0; k < 2u * anchors; ++k) s.frow[4 * size_t(m) + k].applied = f(4 + k, i);
+        FrictionHist& h = s.cur.fric[s.man_list[m]];
+        h.meta = (h.meta & ~256u) | (f(14, i) != 0.0f ? 256u : 0u);
+    }
+
+    // All passes over the loaded unit; body(l): the global body of this
+    // CTA's local body l in [0, nb) (~0: none).
+    template <class Body>
+    __device__ __forceinline__ void run(const DevState& s, uint32_t levels, uint32_t nb, Body body) const {
+        const int pos = s.pos_iters, vel = s.vel_iters < 1 ? 1 : s.vel_iters;
+        const uint32_t slots = bound[levels];
+        for (int it = 0; it < pos + vel; ++it) {
+            const bool friction = it >= pos || pos - it <= 3;
+            if (it == pos) {
+                for (uint32_t i = threadIdx.x; i < slots; i += NT) enter_velocity(i);
+                __syncthreads();
+            }
+            for (uint32_t l = 0; l < levels; ++l) {
+                const uint32_t end = bound[l + 1];
+                for (uint32_t i = bound[l] + threadIdx.x; i < end; i += NT) solve(i, friction, s.neg_zero2);
+                barrier();
+            }
+            if (s.tape_n)
+                for (uint32_t i = threadIdx.x; i < slots; i += NT) tape_slot(s, i, it, friction);
             if (it + 1 == pos) {
-                island_deltas_out(s.sb_mdv, s.sb_mdw, ib, nb, sdv, sdw, lane, 32);
-                __syncwarp();
+                for (uint32_t l = threadIdx.x; l < nb; l += NT) {
+                    const uint32_t g = body(l);
+                    if (g == ~0u) continue;
+                    s.sb_mdv[g] = bd[l];
+                    s.sb_mdw[g] = bd[NBOD + l];
+                }
+                barrier();
             }
         }
-        island_deltas_out(s.sb_dv, s.sb_dw, ib, nb, sdv, sdw, lane, 32);
-        __syncwarp();
+        for (uint32_t i = threadIdx.x; i < slots; i += NT) publish_slot(s, i, true);
+        for (uint32_t l = threadIdx.x; l < nb; l += NT) {
+            const uint32_t g = body(l);
+            if (g == ~0u) continue;
+            s.sb_dv[g] = bd[l];
+            s.sb_dw[g] = bd[NBOD + l];
+        }
+        barrier();
     }
-}
-
-// One CTA of NT threads per island of a size class (at most MAXN
-// descriptors), with the island's deltas in shared memory
-// (2 x (MAXN + 1) float4).
-// Shared memory of k_pgs_block_smem<MAXN>: deltas, then the island's
-// placed descriptors and local bodies, then its partition bounds.
-template <uint32_t MAXN> struct PgsSmem {
-    static constexpr size_t kBytes = 2 * size_t(MAXN + 1) * sizeof(float4) + 2 * size_t(MAXN) * 4 +
-                                     size_t(kMaxLevels + 1) * 4;
 };
-// Threads of the CTA that solves an island of (kMidIsland, kBigIsland]
-// descriptors: 12 warps, the most the register budget of the solver (about
-// 160 registers a thread) allows on one SM; a level of such an island holds
-// a few hundred descriptors, so more threads mean fewer rounds per level.
-constexpr uint32_t kBigPgsThreads = 384;
-template <uint32_t MAXN, uint32_t NT>
-__global__ void __launch_bounds__(NT) k_pgs_block_smem(DevState s, const uint32_t* lvl_bound, int list_class) {
+
+// One island of a size class of at most CAP x CL descriptors (n descriptors
+// have n + 1 bodies at most) on a CTA, or on a cluster of CL CTAs sharing
+// the deltas through distributed shared memory.
+template <uint32_t CAP, uint32_t NT, uint32_t CL>
+__global__ void __launch_bounds__(NT) k_pgs_island(DevState s, int list_class) {
     extern __shared__ float4 shb[];
-    float4* sdv = shb;
-    float4* sdw = shb + (MAXN + 1);
-    uint32_t* sd = reinterpret_cast<uint32_t*>(shb + 2 * (MAXN + 1));   // descriptor per placed slot
-    uint32_t* sl = sd + MAXN;                                             // local bodies per placed slot
-    uint32_t* sb = sl + MAXN;                                             // partition bounds (island-relative)
-    const LocalDeltas D{sdv, sdw};
+    const Unit<CAP, CAP + 1, NT, CL> U(shb);
     const uint32_t n_list = s.counters[list_counter(list_class)];
     const uint32_t* list = s.isl_list[list_class];
-    const int pos = s.pos_iters, vel = s.vel_iters < 1 ? 1 : s.vel_iters;
-    const float4 zero = make_float4(0, 0, 0, 0);
-    uint32_t* ticket = s.counters + kCntQueue + (list_class == 1 ? 1 : 2);
-    __shared__ uint32_t s_next;
-    for (uint32_t k = blockIdx.x;;) {
-        if (s.work_queue) {
-            if (threadIdx.x == 0) s_next = atomicAdd(ticket, 1u);
-            __syncthreads();
-            k = s_next;
-        }
-        if (k >= n_list) break;
+    const uint32_t rank = CL == 1 ? 0u : blockIdx.x % CL;
+    for (uint32_t k = blockIdx.x / CL; k < n_list; k += gridDim.x / CL) {
         const uint32_t isl = list[k];
-        if (!s.work_queue) k += gridDim.x;
-        const uint32_t begin = s.isl_begin[isl];
-        const uint32_t nlev = s.isl_end[isl];
-        const uint32_t nb = s.isl_nbod[isl];
+        const uint32_t begin = s.isl_begin[isl], n = s.isl_begin[isl + 1] - begin;
+        const uint32_t nlev = s.isl_end[isl], nb = s.isl_nbod[isl];
         const int32_t* ib = s.isl_bod + begin + isl;
-        const uint32_t* bound = lvl_bound + begin + isl;
-        const uint32_t n = s.isl_begin[isl + 1] - begin;
-        for (uint32_t l = threadIdx.x; l < nb; l += blockDim.x) { sdv[l] = zero; sdw[l] = zero; }
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint32_t d = s.d_val2[begin + i], lid = s.d_lbod[begin + i];
-            sd[i] = d;
-            sl[i] = d >= s.n_joints ? stage_slot_rows(s, d - s.n_joints, begin + i, lid) : pack_slot_meta(lid, 0u, 0u);
+        const uint32_t* lvl = s.lvl_bound + begin + isl;
+        for (uint32_t i = threadIdx.x; i * CL + rank < n; i += NT) {
+            const uint32_t at = begin + i * CL + rank, lid = s.d_lbod[at];
+            U.load_slot(s, i, s.d_val2[at], lid & 0xffffu, lid >> 16);
         }
-        for (uint32_t l = threadIdx.x; l <= nlev; l += blockDim.x) sb[l] = bound[l] - begin;
-        __syncthreads();
-        for (int it = 0; it < pos + vel; ++it) {
-            for (uint32_t l = 0; l < nlev; ++l) {
-                const uint32_t lb = sb[l], le = sb[l + 1];
-                for (uint32_t i = lb + threadIdx.x; i < le; i += blockDim.x)
-                    solve_slot<LocalDeltas>(s, sd[i], sl[i], it, pos, vel, D, begin + i);
-                __syncthreads();
-            }
-            if (it + 1 == pos) {
-                island_deltas_out(s.sb_mdv, s.sb_mdw, ib, nb, sdv, sdw, threadIdx.x, blockDim.x);
-                __syncthreads();
-            }
+        const uint32_t my_bodies = nb > rank ? (nb - rank + CL - 1) / CL : 0u;
+        for (uint32_t l = threadIdx.x; l < my_bodies; l += NT)
+            U.bd[l] = U.bd[CAP + 1 + l] = make_float4(0, 0, 0, 0);
+        for (uint32_t l = threadIdx.x; l <= nlev; l += NT) {
+            const uint32_t b = lvl[l] - begin;   // slots of this CTA below the level's start
+            U.bound[l] = b > rank ? (b - rank + CL - 1) / CL : 0u;
         }
-        island_deltas_out(s.sb_dv, s.sb_dw, ib, nb, sdv, sdw, threadIdx.x, blockDim.x);
-        __syncthreads();
+        U.barrier();
+        U.run(s, nlev, my_bodies, [&](uint32_t l) { return uint32_t(ib[l * CL + rank]); });
     }
+}
+
+// Islands of at most kSmallUnit descriptors, in groups of one size class c
+// ((2^(c-1), 2^c] descriptors): kGroupCap / 2^c islands share a unit, whose
+// slots are their descriptors sorted by level.  The longest class first:
+// its chains are the longest.
+constexpr uint32_t kSmallUnit = 32, kGroupCap = 96, kGroupThreads = 96;
+static_assert(kGroupCap % kSmallUnit == 0 && kGroupCap <= kGroupThreads, "a thread a descriptor when a group loads");
+using GroupUnit = Unit<kGroupCap, 2 * kGroupCap, kGroupThreads, 1>;
+__global__ void __launch_bounds__(kGroupThreads, 4) k_pgs_group(DevState s) {
+    extern __shared__ float4 shb[];
+    const GroupUnit U(shb);
+    __shared__ uint32_t gbody[2 * kGroupCap], cursor[kSmallUnit + 1], s_unit, s_levels;
+    uint32_t units[DevState::kSmallClasses], total = 0;
+#pragma unroll
+    for (int c = 0; c < DevState::kSmallClasses; ++c) {
+        const uint32_t per = kGroupCap >> c;
+        units[c] = (s.counters[list_counter(DevState::kSmallList + c)] + per - 1u) / per;
+        total += units[c];
+    }
+    const uint32_t t = threadIdx.x;
+    for (uint32_t u = blockIdx.x;;) {
+        if (s.work_queue) {
+            if (t == 0) s_unit = atomicAdd(&s.counters[kCntQueue], 1u);
+            __syncthreads();
+            u = s_unit;
+        }
+        if (u >= total) break;
+        uint32_t at = u, c = 0;
+#pragma unroll
+        for (int k = DevState::kSmallClasses - 1; k >= 0; --k) {
+            c = uint32_t(k);
+            if (at < units[k]) break;
+            at -= units[k];
+        }
+        if (!s.work_queue) u += gridDim.x;
+        // one thread a descriptor: island t >> c of the group, its t % 2^c-th
+        const uint32_t per = kGroupCap >> c, e = at * per + (t >> c), i = t & ((1u << c) - 1u);
+        const bool live = t < kGroupCap && e < s.counters[list_counter(DevState::kSmallList + int(c))];
+        uint32_t d = kInvalid, la = kNoBody, lb = kNoBody, level = 0, nlev = 0;
+        int2 b = make_int2(-1, -1);
+        if (live) {
+            const uint32_t isl = s.isl_list[DevState::kSmallList + c][e];
+            const uint32_t begin = s.isl_begin[isl], n = s.isl_begin[isl + 1] - begin;
+            nlev = s.isl_end[isl];
+            if (i < n) {
+                d = s.d_val2[begin + i];
+                const uint32_t lid = s.d_lbod[begin + i], b0 = (t >> c) * ((1u << c) + 1u);
+                if ((lid & 0xffffu) != 0xffffu) la = b0 + (lid & 0xffffu);
+                if ((lid >> 16) != 0xffffu) lb = b0 + (lid >> 16);
+                level = min(s.d_level[d], nlev - 1u);
+                b = s.d_bod[d];
+            }
+        }
+        if (t < kSmallUnit + 1u) U.bound[t] = 0u;
+        if (t == 0) s_levels = 0u;
+        for (uint32_t l = t; l < 2 * kGroupCap; l += kGroupThreads) {
+            gbody[l] = ~0u;
+            U.bd[l] = U.bd[2 * kGroupCap + l] = make_float4(0, 0, 0, 0);
+        }
+        __syncthreads();
+        const bool mine = d != kInvalid && level < kSmallUnit;
+        if (mine) {
+            atomicAdd(&U.bound[level + 1u], 1u);
+            if (la != kNoBody) gbody[la] = uint32_t(b.x);
+            if (lb != kNoBody) gbody[lb] = uint32_t(b.y);
+        }
+        if (live && i == 0) atomicMax(&s_levels, nlev);
+        __syncthreads();
+        if (t < 32) {   // counts -> starts
+            uint32_t x = U.bound[t + 1u];
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (int(t) >= o) x += y;
+            }
+            __syncwarp();
+            U.bound[t + 1u] = x;
+            cursor[t + 1u] = x;
+            if (t == 0) cursor[0] = 0u;
+        }
+        __syncthreads();
+        if (mine) U.load_slot(s, atomicAdd(&cursor[level], 1u), d, la, lb);
+        __syncthreads();
+        U.run(s, s_levels, per * ((1u << c) + 1u), [&](uint32_t l) { return gbody[l]; });
+    }
+}
+
+// The solver kernels of the size classes above kSmallUnit descriptors,
+// largest first: f(kernel, threads, CTAs a cluster, shared memory, island
+// list).  An island has about ten levels, so a class's threads cover the
+// descriptors of a level; its records fill shared memory.
+template <class F> void for_island_solvers(F f) {
+    f(k_pgs_island<512, 128, 8>, 128u, 8u, Unit<512, 513, 128, 8>::kBytes, 9);
+    f(k_pgs_island<256, 64, 8>, 64u, 8u, Unit<256, 257, 64, 8>::kBytes, 8);
+    f(k_pgs_island<128, 32, 8>, 32u, 8u, Unit<128, 129, 32, 8>::kBytes, 7);
+    f(k_pgs_island<512, 128, 1>, 128u, 1u, Unit<512, 513, 128, 1>::kBytes, 6);
+    f(k_pgs_island<256, 64, 1>, 64u, 1u, Unit<256, 257, 64, 1>::kBytes, 5);
+    f(k_pgs_island<112, 64, 1>, 64u, 1u, Unit<112, 113, 64, 1>::kBytes, 4);
 }
 
 // One CTA per island beyond kBigIsland descriptors: deltas in global memory.
@@ -1944,7 +2033,7 @@ __global__ void __launch_bounds__(256) k_pgs_block(DevState s, const uint32_t* l
             for (uint32_t l = 0; l < nlev; ++l) {
                 const uint32_t lb = bound[l], le = bound[l + 1];
                 for (uint32_t i = lb + threadIdx.x; i < le; i += blockDim.x)
-                    solve_desc(s, s.d_val2[i], 0u, it, pos, vel, D);
+                    solve_desc(s, s.d_val2[i], it, pos, vel, D);
                 __syncthreads();
             }
             if (it + 1 == pos) {
@@ -2062,28 +2151,30 @@ inline uint32_t grid_for(uint32_t n, uint32_t t, uint32_t cap) {
 // the concurrent branches (graphs are instantiated with node priorities).
 static int g_high_priority = 0;
 template <class... KArgs, class... Args>
-static void launch_high(void (*kernel)(KArgs...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st,
-                        Args... args) {
+static void launch(void (*kernel)(KArgs...), uint32_t grid, uint32_t block, size_t smem, uint32_t cluster,
+                   int priority, cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributePriority;
-    attr[0].val.priority = g_high_priority;
+    attr[0].val.priority = priority;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
     cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// Fork n side branches off st (or run everything on st without branches).
-static void fork_branches(const Branches* br, cudaStream_t st, int n) {
+void fork_branches(const Branches* br, cudaStream_t st, int n) {
     if (!br) return;
     cudaEventRecord(br->fork, st);
     for (int i = 0; i < n; ++i) cudaStreamWaitEvent(br->st[i], br->fork, 0);
 }
-static void join_branches(const Branches* br, cudaStream_t st, int n) {
+void join_branches(const Branches* br, cudaStream_t st, int n) {
     if (!br) return;
     for (int i = 0; i < n; ++i) {
         cudaEventRecord(br->join[i], br->st[i]);
@@ -2181,8 +2272,10 @@ void init_solver_kernels() {
     if (cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess) g_high_priority = greatest;
     cudaFuncSetAttribute(k_partition_smem<kBigIsland>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          int(PartSmem<kBigIsland>::kBytes));
-    cudaFuncSetAttribute(k_pgs_block_smem<kBigIsland, kBigPgsThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(PgsSmem<kBigIsland>::kBytes));
+    for_island_solvers([](auto kernel, uint32_t, uint32_t, size_t smem, int) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    });
+    cudaFuncSetAttribute(k_pgs_group, cudaFuncAttributeMaxDynamicSharedMemorySize, int(GroupUnit::kBytes));
 }
 
 void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, const Branches* br) {
@@ -2231,9 +2324,9 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     // partitions by island size class, and row preparation: independent
     hook(kStPrep, st);
     fork_branches(br, st, 3);
-    launch_high(k_partition_smem<kBigIsland>, grid_for(s.desc_cap, kMidIsland + 1, 148u * 2u), 256u,
-                PartSmem<kBigIsland>::kBytes, side(1), s, lvl_bound, 2);
-    launch_high(k_partition_large, grid_for(s.desc_cap, kBigIsland + 1, 148u), 256u, size_t(0), side(1), s,
+    launch(k_partition_smem<kBigIsland>, grid_for(s.desc_cap, kMidIsland + 1, 148u * 2u), 256u,
+                PartSmem<kBigIsland>::kBytes, 1u, g_high_priority, side(1), s, lvl_bound, 2);
+    launch(k_partition_large, grid_for(s.desc_cap, kBigIsland + 1, 148u), 256u, size_t(0), 1u, g_high_priority, side(1), s,
                 lvl_bound);
     k_partition<<<grid_for(s.desc_cap, kPartWarps, 148u * 16u), kPartWarps * 32, 0, st>>>(s, lvl_bound);
     k_partition_smem<kMidIsland><<<grid_for(s.desc_cap, kSerialIsland + 1, 148u * 8u), 256,
@@ -2241,18 +2334,21 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     if (s.n_joints) k_prep_joints<<<grid_for(s.n_joints, 128, 1u << 30), 128, 0, side(2)>>>(s);   // ~150 registers
     k_prep_contacts<<<grid_for(s.desc_cap, 128, cap_blocks), 128, 0, side(2)>>>(s);
     join_branches(br, st, 3);
-    // PGS: islands by size class, independent
+    // PGS: islands by size class, independent.  The clusters' eight CTAs
+    // need room in one part of the chip at once: they go first and with
+    // priority, or they wait until the other classes have drained (127 us of
+    // a 320 us stage on the 131,072-body pile).
     hook(kStPgs, st);
-    fork_branches(br, st, 3);
-    launch_high(k_pgs_block_smem<kBigIsland, kBigPgsThreads>, grid_for(s.desc_cap, s.isl_mid + 1, 148u),
-                kBigPgsThreads, PgsSmem<kBigIsland>::kBytes, side(1), s, lvl_bound, 4);
-    launch_high(k_pgs_block, grid_for(s.desc_cap, kBigIsland + 1, 148u), 256u, size_t(0), side(1), s, lvl_bound);
-    k_pgs_warp<<<grid_for(s.desc_cap * 32u, kPgsWarpsPerBlock * 32u, 148u * 3u), kPgsWarpsPerBlock * 32u, 0, st>>>(
-        s, lvl_bound);
-    k_pgs_block_smem<kMidIsland, 128><<<grid_for(s.desc_cap, s.isl_warp + 1, 148u * 3u), 128,
-                                        PgsSmem<kMidIsland>::kBytes, side(0)>>>(s, lvl_bound, 1);
-    k_pgs_thread<<<grid_for(s.desc_cap, kPgsThreadBlock, 148u * 8u), kPgsThreadBlock, 0, side(2)>>>(s);
-    join_branches(br, st, 3);
+    fork_branches(br, st, Branches::kN);
+    int branch = 0;
+    for_island_solvers([&](auto kernel, uint32_t nt, uint32_t cl, size_t smem, int list) {
+        const uint32_t islands = grid_for(s.desc_cap, kListMinDesc[list] + 1, 148u * uint32_t(232448u / smem) / cl);
+        launch(kernel, islands * cl, nt, smem, cl, cl > 1 ? g_high_priority : 0, side(branch++), s, list);
+    });
+    launch(k_pgs_block, grid_for(s.desc_cap, kBigIsland + 1, 148u), 256u, size_t(0), 1u, g_high_priority, side(0), s,
+           lvl_bound);
+    k_pgs_group<<<grid_for(s.desc_cap, kGroupCap / kSmallUnit, 148u * 4u), kGroupThreads, GroupUnit::kBytes, st>>>(s);
+    join_branches(br, st, Branches::kN);
     hook(kStIntegrate, st);
     k_integrate<<<grid_for(s.n_bodies, T, 1u << 30), T, 0, st>>>(s);
     if (s.n_kinematic) k_kinematic_publish<<<grid_for(s.n_bodies, T, 1u << 30), T, 0, st>>>(s);

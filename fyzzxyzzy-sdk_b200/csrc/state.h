@@ -55,6 +55,7 @@ struct DevState {
     // takes the next entry from a per-step device counter).
     bool work_queue = false;
     int pos_iters = 4, vel_iters = 1;
+    uint64_t neg_zero2 = 0x8000000080000000ull;   // {-0, -0}, opaque to the kernels' compiler
     float dt = 1.0f / 120.0f;
     uint32_t frame = 0;
 
@@ -134,10 +135,6 @@ struct DevState {
     ManagerHeader* mh = nullptr;       // per touching manager
     NormalRow* nrow = nullptr;         // 4 per touching manager
     FrictionRow* frow = nullptr;       // 4 per touching manager
-    // The island solvers' copy of the rows in placed-descriptor order (slot
-    // i = position in d_val2): kSlotVecPlanes float4 planes then
-    // kSlotScalarPlanes float planes of desc_cap records.
-    float4* slot_rows = nullptr;
 
     // joints (static, sorted by scene then constraint slot descending)
     uint32_t *j_a = nullptr, *j_b = nullptr;  // descriptor bodies (distance: ordered pair; others: authored)
@@ -172,10 +169,11 @@ struct DevState {
     uint32_t* isl_nbod = nullptr;      // per island
     // Islands by size class (descriptors), listed each step by
     // k_island_classes: 0 (32, 512] shared-memory partition, 1 (isl_warp,
-    // isl_mid] 128-thread CTA solver, 2 (512, 4096] shared-memory partition,
-    // 3 beyond 4096 global-memory paths, 4 (isl_mid, 4096] 384-thread CTA
-    // solver, 5 (isl_thread, isl_warp] warp solver.
-    static constexpr int kIslLists = 6;
+    // isl_mid] the rollout's 128-thread reverse sweep, 2 (512, 4096]
+    // shared-memory partition, 3 beyond 4096 global-memory paths, 4-9 the
+    // CTA and cluster solvers, kSmallList + c the small islands of
+    // (2^(c-1), 2^c] descriptors (pgs_list).
+    static constexpr int kSmallList = 10, kSmallClasses = 6, kIslLists = kSmallList + kSmallClasses;
     uint32_t* isl_list[kIslLists] = {};
 
     // step scratch
@@ -290,11 +288,16 @@ struct StageHook {
 // back into the main stream through events, so inside a stream capture they
 // become parallel branches of the step's graph.
 struct Branches {
-    static constexpr int kN = 3;
+    static constexpr int kN = 6;
     cudaStream_t st[kN] = {};
     cudaEvent_t fork = nullptr;
     cudaEvent_t join[kN] = {};
 };
+
+// Fork n side branches off st / join them (or run everything on st without
+// branches).
+void fork_branches(const Branches* br, cudaStream_t st, int n);
+void join_branches(const Branches* br, cudaStream_t st, int n);
 
 // Reverse-mode state of a differentiated rollout (adjoint.cu).  Per body,
 // the adjoint of the mass-frame state (centre c, orientation Q) and the
@@ -354,9 +357,6 @@ void init_solver_kernels();
 constexpr uint32_t kSmallIsland = 96;     // one warp
 constexpr uint32_t kMidIsland = 512;      // one CTA, shared-memory deltas
 constexpr uint32_t kBigIsland = 4096;     // one CTA, shared-memory deltas (1 CTA / SM)
-// Planes of DevState::slot_rows, desc_cap records each: 25 of float4, then
-// 16 of float (the layout is described where the solver stages them).
-constexpr uint32_t kSlotVecPlanes = 25, kSlotScalarPlanes = 16;
 // counters[] slots
 enum : int { kCntMan = 0, kCntDesc = 1, kCntIsl = 2, kCntFrame = 3, kCntLevels = 4, kCntGjk = 5,
              kCntAwake = 6 /* descriptors of awake islands */, kCntSleeping = 7 /* asleep at step start */,
@@ -371,13 +371,25 @@ enum : int { kCntMan = 0, kCntDesc = 1, kCntIsl = 2, kCntFrame = 3, kCntLevels =
              kCntThRows = 21 /* managers with a reportable impulse */,
              kCntThChanges = 22 /* force-threshold changes of the step */,
              kCntThCommon = 23 /* pairs exceeding in this step and the previous one */,
-             kCntList4 = 24 /* length of island list 4 */, kCntList5 = 25 /* length of island list 5 */,
-             kCntQueue = 26 /* 3 work-queue tickets: warp, mid CTA, big CTA solvers */, kCntSlots = 29 };
+             kCntList4 = 24 /* lengths of island lists 4 .. kIslLists - 1 */,
+             kCntQueue = kCntList4 + DevState::kIslLists - 4 /* work-queue ticket of the small islands' solver */,
+             kCntSlots = kCntQueue + 1 };
 // Counter slot of island list c.
 __host__ __device__ constexpr int list_counter(int c) { return c < 4 ? kCntList + c : kCntList4 + (c - 4); }
 // Each list holds islands of more than this many descriptors (its capacity
 // is descriptors / (bound + 1) + 2).
-constexpr uint32_t kListMinDesc[6] = {32, 32, 512, 4096, 128, 0};
+constexpr uint32_t kListMinDesc[DevState::kIslLists] = {32,  32,   512,  4096, 32, 112, 256, 512,
+                                                            1024, 2048, 0,    1,    2,  4,   8,   16};
+// The solver list of an island of n descriptors (-1: beyond kBigIsland,
+// list 3 holds it).
+__host__ __device__ constexpr int pgs_list(uint32_t n) {
+    if (n > kBigIsland) return -1;
+    if (n > 512u) return n <= 1024u ? 7 : n <= 2048u ? 8 : 9;
+    if (n > 32u) return n <= 112u ? 4 : n <= 256u ? 5 : 6;
+    int c = 0;
+    while ((1u << c) < n) ++c;
+    return DevState::kSmallList + c;
+}
 
 // Contact event records in device memory; the layouts of
 // fyzz_b200_contact_event_t and fyzz_b200_contact_event_point_t.
