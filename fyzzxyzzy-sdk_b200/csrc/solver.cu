@@ -62,6 +62,7 @@ __global__ void k_bodies_begin(DevState s) {
     s.sb_mask[b] = 0u;
     s.sb_maxdyn[b] = 0u;
     s.sb_static[b] = 0u;
+    s.sb_earliest[b] = kInvalid;
     const float4 z = make_float4(0, 0, 0, 0);
     s.sb_dv[b] = z; s.sb_dw[b] = z; s.sb_mdv[b] = z; s.sb_mdw[b] = z;
     if (s.sleep) {
@@ -72,11 +73,16 @@ __global__ void k_bodies_begin(DevState s) {
     }
 }
 
+__device__ uint32_t uf_find(uint32_t* parent, uint32_t x);
 // Unconstrained velocity + solver-body data for every awake dynamic body
 // (scene.cpp:10383 prepare_unconstrained_velocities skips sleeping actors).
 __global__ void k_bodies_velocity(DevState s) {
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b >= s.n_bodies || !is_dyn(s, b)) return;
+    // the smallest body of each touch-graph island names it (k_desc_keys);
+    // blocks start in body order, so most bodies find a smaller one there
+    uint32_t* name = s.sb_earliest + uf_find(s.uf_parent, b);
+    if (*reinterpret_cast<volatile uint32_t*>(name) > b) atomicMin(name, b);
     if (is_asleep(s, b)) {
         const float4 z = make_float4(0, 0, 0, 0);
         s.sb_v[b] = z;
@@ -151,20 +157,27 @@ __global__ void __launch_bounds__(kScanThreads) k_touch_compact(DevState s) {
 
 // Lock-free union-find after ECL-CC (Jaiganesh and Burtscher, "A
 // high-performance connected components implementation for GPUs", HPDC
-// 2018): a root is hooked under the smaller root, so every parent index is
-// at most its child's and the root of a set is its smallest member; finds
-// shorten the path they walk (intermediate pointer jumping, plain stores:
-// a node that is not a root only ever gets an ancestor written); a failed
-// hook continues from the value it found instead of finding both roots
-// again.  Loads go through L1: a stale parent is still an ancestor (sets
-// only merge), a stale root fails its hook and the hook continues from the
-// value the atomic returns, and the root of a large set is then read from
-// each SM's L1 instead of by every thread from one L2 line.
+// 2018): a root is hooked under another root, finds shorten the path they
+// walk (intermediate pointer jumping, plain stores: a node that is not a
+// root only ever gets an ancestor written); a failed hook continues from
+// the value it found instead of finding both roots again.  Loads go through
+// L1: a stale parent is still an ancestor (sets only merge), a stale root
+// fails its hook and the hook continues from the value the atomic returns,
+// and the root of a large set is then read from each SM's L1 instead of by
+// every thread from one L2 line.
+//
+// Which root goes under which follows a fixed scramble of the body index
+// (linking in random order: Goel et al., "Disjoint set union with randomized
+// linking", SODA 2014): trees then stay some log n deep.  Linking by the
+// index itself made chains of neighbours, about a hundred hops deep in a
+// 1,900-descriptor island, and the find that walked one set the length of the
+// key pass (32 us; 36 us on the 131,072-body pile).
+__device__ __forceinline__ uint32_t uf_rank(uint32_t x) { return x * 0x9E3779B1u; }   // odd factor: no two alike
 __device__ uint32_t uf_find(uint32_t* parent, uint32_t x) {
     uint32_t cur = parent[x];
     if (cur == x) return x;
     uint32_t prev = x, next;
-    for (int it = 0; it < (1 << 24) && cur > (next = parent[cur]); ++it) {
+    for (int it = 0; it < (1 << 24) && cur != (next = parent[cur]); ++it) {
         parent[prev] = next;
         prev = cur;
         cur = next;
@@ -173,10 +186,10 @@ __device__ uint32_t uf_find(uint32_t* parent, uint32_t x) {
 }
 __device__ void uf_union(const DevState& s, uint32_t* parent, uint32_t a, uint32_t b) {
     uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
-    // every failed hook moves one root strictly down, so this ends
+    // every failed hook moves one root strictly down in rank, so this ends
     for (int it = 0; it < (1 << 24); ++it) {
         if (ra == rb) return;
-        if (ra < rb) {
+        if (uf_rank(ra) < uf_rank(rb)) {
             const uint32_t r = atomicCAS(&parent[rb], rb, ra);
             if (r == rb) return;
             rb = r;
@@ -227,25 +240,31 @@ __global__ void k_union(DevState s) {
         if (b0 >= 0 && b1 >= 0) uf_union(s, s.uf_parent, uint32_t(b0), uint32_t(b1));
     }
 }
-// Island key of every descriptor: the union-find root of its bodies.  The
+// Island key of every descriptor: the smallest body of its island.  The
 // descriptors of sleeping islands (every island is either awake or asleep
 // once the step's sleep decisions are made) take the key n_bodies, which
 // sorts them after every awake island; kCntAwake counts the others.
 __global__ void k_desc_keys(DevState s) {
     const uint32_t n = s.counters[kCntDesc];
     const uint32_t stride = gridDim.x * blockDim.x;
+    uint32_t awake = 0;
     for (uint32_t d = blockIdx.x * blockDim.x + threadIdx.x; d < n; d += stride) {
         int32_t b0, b1;
         desc_bodies(s, d, b0, b1);
         const uint32_t body = b0 >= 0 ? uint32_t(b0) : uint32_t(b1);
         const bool asleep = is_asleep(s, body);
-        s.d_key[d] = asleep ? s.n_bodies : uf_find(s.uf_parent, body);
+        s.d_key[d] = asleep ? s.n_bodies : s.sb_earliest[uf_find(s.uf_parent, body)];
         s.d_val[d] = d;
         s.d_level[d] = kInvalid;
-        const uint32_t am = __activemask();
-        const uint32_t votes = __ballot_sync(am, !asleep);
-        if ((threadIdx.x & 31u) == uint32_t(__ffs(am) - 1)) atomicAdd(&s.counters[kCntAwake], __popc(votes));
+        awake += asleep ? 0u : 1u;
     }
+    __shared__ uint32_t total;
+    if (threadIdx.x == 0) total = 0u;
+    __syncthreads();
+    awake = __reduce_add_sync(0xffffffffu, awake);
+    if ((threadIdx.x & 31u) == 0 && awake) atomicAdd(&total, awake);
+    __syncthreads();
+    if (threadIdx.x == 0 && total) atomicAdd(&s.counters[kCntAwake], total);
 }
 
 // Replayed order (one step): descriptors are first sorted by their rank in
