@@ -7,10 +7,9 @@
 // the point where they need a pair set: a frame loop that shares the GPU with
 // other work and must not take the device-wide synchronisation that
 // cudaMalloc / cudaFree imply, or a process that runs under a fixed device
-// memory budget reserved up front.  This entry point serves them: the same
-// sort + sweep + canonical owner-bucket emission as the world's broadphase,
-// in one CTA, with its working set in a fixed file-scope device array
-// instead of allocated buffers.
+// memory budget reserved up front.  This entry point serves them: the pair
+// set and canonical order of the world's broadphase, with its working set in
+// a fixed file-scope device array instead of allocated buffers.
 //
 // Pair semantics follow the reference's full sweep (src/native/scene.cpp,
 // Scene::update_pairs 2635-2704): two finite shapes pair when their encoded
@@ -26,7 +25,7 @@
 //    one stream;
 //  * the first call on a device resolves the scratch array's address with
 //    cudaGetSymbolAddress (which loads this module on that device) and
-//    raises the kernel's dynamic shared-memory limit; make that first call
+//    raises a kernel's dynamic shared-memory limit; make that first call
 //    before any stream capture on the device.  The resolved address is kept
 //    per CUDA context, so a context made after cudaDeviceReset resolves it
 //    again on its first call;
@@ -46,157 +45,185 @@ namespace {
 
 constexpr uint32_t kStaticSapMaxShapes = FYZZ_B200_STATIC_SAP_MAX_SHAPES;
 static_assert(kStaticSapMaxShapes == 8192u, "the rejection message states the limit");
-constexpr int kThreads = 1024;
-// Sorted (min x << 32 | shape) keys live in shared memory: 8 bytes a shape.
-constexpr size_t kMaxSortSmem = size_t(kStaticSapMaxShapes) * sizeof(unsigned long long);
-static_assert(kMaxSortSmem <= 227u * 1024u, "sort keys must fit one CTA's shared memory");
-
 // Scratch layout, 32 bytes a shape (256 KiB at the maximum):
-//   rec  uint4  sorted-order (min y, max y, min z, max z)
-//   meta uint2  sorted-order (max x, body | dynamic << 31)
-//   cnt  u32    pairs owned by each shape      -- must start at zero; the
-//                                                 kernel clears it first
-//   off  u32    bucket offsets (written by the kernel's scan before use)
-constexpr size_t kRecOff = 0;
-constexpr size_t kMetaOff = kRecOff + size_t(kStaticSapMaxShapes) * 16;
-constexpr size_t kCntOff = kMetaOff + size_t(kStaticSapMaxShapes) * 8;
-constexpr size_t kOffOff = kCntOff + size_t(kStaticSapMaxShapes) * 4;
-constexpr size_t kScratchBytes = kOffOff + size_t(kStaticSapMaxShapes) * 4;
+//   cnt      u32            pairs owned by each shape (the lower shape id)
+//   partner  u16 x kKept    its first partners, ascending
+constexpr uint32_t kKept = 14;
+constexpr size_t kPartnerOff = size_t(kStaticSapMaxShapes) * 4;
+constexpr size_t kScratchBytes = kPartnerOff + size_t(kStaticSapMaxShapes) * kKept * 2;
+static_assert(kScratchBytes == 256u * 1024u && kStaticSapMaxShapes <= 65536u, "documented size; partners fit 16 bits");
 
 static __device__ __align__(256) unsigned char g_sap_scratch[kScratchBytes];
 
-// Block-wide exclusive scan of cnt[0, n) into off[0, n); returns the total.
+// The whole device tests every shape against all shapes of larger id:
+// lanes hold 32 consecutive candidates, so an owner's pairs come out in
+// partner order by ballots and nothing is sorted.  At 8,192 shapes that is
+// 1.05 million 32-wide tests in x and z of about eight instructions; a
+// candidate's y and body are read only where some lane passes them.  Every
+// block holds all shapes in shared memory (28 bytes each, 224 KiB at the
+// maximum): with only x there, two thirds of the x tests went on to a round
+// trip to L2 (317 us).  The sort + sweep in one CTA that it replaces waited
+// for one SM's barriers and scattered L2 reads: 1,453 us on 8,192 shapes
+// with 23,200 pairs.
+struct Owner {
+    uint32_t id, mnx, mxx, mny, mxy, mnz, mxz, body;
+};
+__device__ __forceinline__ Owner load_owner(const uint32_t* __restrict__ bounds, const uint32_t* __restrict__ body,
+                                            uint32_t i) {
+    const uint32_t* b = bounds + 6 * size_t(i);
+    return {i, b[0], b[3], b[1], b[4], b[2], b[5], body[i]};
+}
+// In x the shape that starts first (lower id on ties) must reach the other's
+// start, as in a sweep over the sorted minima.
+__device__ __forceinline__ bool overlap_x(const Owner& a, uint32_t mn, uint32_t mx) {
+    return mn >= a.mnx ? mn <= a.mxx : a.mnx <= mx;
+}
+__device__ __forceinline__ bool overlap_z(const Owner& a, uint32_t mn, uint32_t mx) {
+    return !(a.mnz > mx || mn > a.mxz);
+}
+// The rest of the test: y, different bodies, one of them dynamic.
+__device__ __forceinline__ bool overlap_rest(const Owner& a, uint32_t mn, uint32_t mx, uint32_t body) {
+    return (body & 0x7fffffffu) != (a.body & 0x7fffffffu) && ((body | a.body) >> 31) && !(a.mny > mx || mn > a.mxy);
+}
+
+// Four owners a warp, two from either end of the shapes, so that every warp
+// tests the same number of candidates.  Counts each owner's pairs and keeps
+// its first kKept partners.
+constexpr int kCountThreads = 512;
+constexpr size_t kShapeSmem = sizeof(uint4) + sizeof(uint2) + sizeof(uint32_t);
+constexpr size_t kMaxCountSmem = size_t(kStaticSapMaxShapes) * kShapeSmem;
+static_assert(kMaxCountSmem <= 227u * 1024u, "every shape fits one block's shared memory");
+__global__ void __launch_bounds__(kCountThreads) k_sap_count(const uint32_t* __restrict__ bounds,
+                                                             const uint32_t* __restrict__ body, uint32_t n,
+                                                             unsigned char* scratch) {
+    extern __shared__ uint4 xz[];   // every shape: min x, max x, min z, max z; then min y, max y; then body
+    uint2* ys = reinterpret_cast<uint2*>(xz + n);
+    uint32_t* bs = reinterpret_cast<uint32_t*>(ys + n);
+    uint32_t* cnt = reinterpret_cast<uint32_t*>(scratch);
+    uint16_t* kept = reinterpret_cast<uint16_t*>(scratch + kPartnerOff);
+    for (uint32_t i = threadIdx.x; i < n; i += kCountThreads) {
+        const uint32_t* b = bounds + 6 * size_t(i);
+        xz[i] = make_uint4(b[0], b[3], b[2], b[5]);
+        ys[i] = make_uint2(b[1], b[4]);
+        bs[i] = body[i];
+    }
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u, w = (blockIdx.x * kCountThreads + threadIdx.x) >> 5;
+    const uint32_t half = (n + 1) / 2;   // owners below half from the front, the others from the back
+    if (2 * w >= half) return;
+    Owner o[4];
+    uint32_t found[4] = {0, 0, 0, 0};
+    bool on[4];
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k) {
+        const uint32_t at = 2 * w + (k & 1u);
+        on[k] = k < 2 ? at < half : at < n - half;
+        o[k] = load_owner(bounds, body, !on[k] ? 0u : k < 2 ? at : n - 1u - at);
+        if (!on[k]) o[k].id = n;
+    }
+    const uint32_t lt = (1u << lane) - 1u;
+    for (uint32_t base = (2 * w + 1) & ~31u; base < n; base += 32) {
+        const uint32_t j = base + lane;
+        const uint4 x = j < n ? xz[j] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            bool hit = j < n && j > o[k].id && overlap_x(o[k], x.x, x.y) && overlap_z(o[k], x.z, x.w);
+            if (!__any_sync(0xffffffffu, hit)) continue;
+            if (hit) {
+                const uint2 y = ys[j];
+                hit = overlap_rest(o[k], y.x, y.y, bs[j]);
+            }
+            const uint32_t bits = __ballot_sync(0xffffffffu, hit);
+            const uint32_t at = found[k] + __popc(bits & lt);
+            if (hit && at < kKept) kept[o[k].id * kKept + at] = uint16_t(j);
+            found[k] += __popc(bits);
+        }
+    }
+#pragma unroll
+    for (uint32_t k = 0; k < 4; ++k)
+        if (on[k] && lane == 0) cnt[o[k].id] = found[k];
+}
+
+// Block-wide exclusive scan of cnt[0, n) into off; returns the total.
+constexpr int kFillThreads = 1024;
 __device__ uint32_t block_scan(const uint32_t* cnt, uint32_t* off, uint32_t n) {
-    __shared__ uint32_t warp_sum[kThreads / 32];
-    __shared__ uint32_t total;
-    const uint32_t chunk = (n + kThreads - 1) / kThreads;
+    __shared__ uint32_t warp_sum[kFillThreads / 32];
+    constexpr uint32_t chunk = kStaticSapMaxShapes / kFillThreads;
     const uint32_t b = threadIdx.x * chunk;
-    const uint32_t e = b + chunk < n ? b + chunk : n;
-    uint32_t local = 0;
-    for (uint32_t i = b; i < e; ++i) local += __ldcg(cnt + i);
+    uint32_t v[chunk], local = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < chunk; ++i) {
+        v[i] = b + i < n ? __ldcg(cnt + b + i) : 0u;
+        local += v[i];
+    }
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t incl = local;
     for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t v = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= uint32_t(d)) incl += v;
+        const uint32_t x = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= uint32_t(d)) incl += x;
     }
     if (lane == 31) warp_sum[warp] = incl;
     __syncthreads();
     if (warp == 0) {
-        uint32_t w = warp_sum[lane];
+        uint32_t x = warp_sum[lane];
         for (int d = 1; d < 32; d <<= 1) {
-            const uint32_t v = __shfl_up_sync(0xffffffffu, w, d);
-            if (lane >= uint32_t(d)) w += v;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+            if (lane >= uint32_t(d)) x += y;
         }
-        warp_sum[lane] = w;                  // inclusive over warps
-        if (lane == 31) total = w;
+        warp_sum[lane] = x;                  // inclusive over warps
     }
     __syncthreads();
     uint32_t run = (warp ? warp_sum[warp - 1] : 0u) + incl - local;
-    for (uint32_t i = b; i < e; ++i) {
-        off[i] = run;
-        run += __ldcg(cnt + i);
+#pragma unroll
+    for (uint32_t i = 0; i < chunk; ++i) {
+        if (b + i < n) off[b + i] = run;
+        run += v[i];
     }
     __syncthreads();
-    return total;
+    return warp_sum[kFillThreads / 32 - 1];
 }
 
-// One CTA: sort min-x endpoints, gather the sweep records, count pairs per
-// owner (the lower shape id), scan, fill the owner buckets, sort each bucket
-// by partner.  bounds: n x 6 encoded values (min x, y, z, max x, y, z), the
-// layout fyzz_b200_read_encoded_bounds produces.
-__global__ void __launch_bounds__(kThreads) k_sap_static(const uint32_t* __restrict__ bounds,
-                                                         const uint32_t* __restrict__ body,
-                                                         uint32_t n, uint32_t* __restrict__ pairs,
-                                                         uint32_t cap, uint32_t* __restrict__ count,
-                                                         unsigned char* scratch) {
-    extern __shared__ unsigned long long sk[];
-    __shared__ uint32_t s_total;
-    uint4* rec = reinterpret_cast<uint4*>(scratch + kRecOff);
-    uint2* meta = reinterpret_cast<uint2*>(scratch + kMetaOff);
-    uint32_t* cnt = reinterpret_cast<uint32_t*>(scratch + kCntOff);
-    uint32_t* off = reinterpret_cast<uint32_t*>(scratch + kOffOff);
-    uint32_t m = 1;
-    while (m < n) m <<= 1;
-    for (uint32_t i = threadIdx.x; i < n; i += kThreads) cnt[i] = 0u;
-    for (uint32_t i = threadIdx.x; i < m; i += kThreads)
-        sk[i] = i < n ? (static_cast<unsigned long long>(bounds[6 * size_t(i)]) << 32) | i : ~0ull;
-    __syncthreads();
-    // bitonic sort by (min x, shape id), the reference's endpoint order
-    for (uint32_t k = 2; k <= m; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < m; i += kThreads) {
-                const uint32_t ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = sk[i], c = sk[ixj];
-                    const bool up = (i & k) == 0;
-                    if ((a > c) == up) { sk[i] = c; sk[ixj] = a; }
-                }
+// Every block scans all counts for itself (cheaper than a launch of its
+// own), then its warps write their owners' buckets: the kept partners, or,
+// for an owner with more, the candidates tested again.  A bucket is written
+// only when all of it fits, so a truncated list is a canonical prefix.
+constexpr uint32_t kFillOwners = 128;   // owners a block
+__global__ void __launch_bounds__(kFillThreads) k_sap_fill(const uint32_t* __restrict__ bounds,
+                                                           const uint32_t* __restrict__ body, uint32_t n,
+                                                           uint32_t* __restrict__ pairs, uint32_t cap,
+                                                           uint32_t* __restrict__ count, const unsigned char* scratch) {
+    __shared__ uint32_t off[kStaticSapMaxShapes];
+    const uint32_t* cnt = reinterpret_cast<const uint32_t*>(scratch);
+    const uint16_t* kept = reinterpret_cast<const uint16_t*>(scratch + kPartnerOff);
+    const uint32_t total = block_scan(cnt, off, n);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *count = total;
+    const uint32_t lane = threadIdx.x & 31u, lt = (1u << lane) - 1u;
+    const uint32_t stop = min(n, (blockIdx.x + 1) * kFillOwners);
+    for (uint32_t i = blockIdx.x * kFillOwners + (threadIdx.x >> 5); i < stop; i += kFillThreads / 32) {
+        const uint32_t begin = off[i], end = i + 1 < n ? off[i + 1] : total;
+        if (begin == end || end > cap) continue;
+        uint32_t* p = pairs + 2 * size_t(begin);
+        if (end - begin <= kKept) {
+            if (lane < end - begin) {
+                p[2 * lane] = i;
+                p[2 * lane + 1] = kept[i * kKept + lane];
             }
-            __syncthreads();
+            continue;
         }
-    for (uint32_t i = threadIdx.x; i < n; i += kThreads) {
-        const uint32_t id = uint32_t(sk[i]);
-        const uint32_t* bd = bounds + 6 * size_t(id);
-        rec[i] = make_uint4(bd[1], bd[4], bd[2], bd[5]);
-        meta[i] = make_uint2(bd[3], body[id]);
-    }
-    __syncthreads();
-    for (int fill = 0; fill < 2; ++fill) {
-        for (uint32_t i = threadIdx.x; i < n; i += kThreads) {
-            const uint32_t id = uint32_t(sk[i]);
-            const uint4 a = rec[i];
-            const uint2 am = meta[i];
-            const uint32_t abody = am.y & 0x7fffffffu;
-            const bool adyn = (am.y >> 31) != 0u;
-            for (uint32_t j = i + 1; j < n; ++j) {
-                const unsigned long long kj = sk[j];
-                if (uint32_t(kj >> 32) > am.x) break;
-                const uint2 bm = meta[j];
-                if ((bm.y & 0x7fffffffu) == abody) continue;
-                if (!adyn && (bm.y >> 31) == 0u) continue;
-                const uint4 c = rec[j];
-                if (a.x > c.y || c.x > a.y || a.z > c.w || c.z > a.w) continue;
-                const uint32_t other = uint32_t(kj);
-                const uint32_t owner = id < other ? id : other;
-                const uint32_t partner = id < other ? other : id;
-                if (!fill) {
-                    atomicAdd(cnt + owner, 1u);
-                } else {
-                    // bucket [off[owner], off[owner + 1]): written only when
-                    // all of it fits, so a truncated list is a canonical prefix
-                    const uint32_t end = owner + 1 < n ? __ldcg(off + owner + 1) : s_total;
-                    if (end <= cap) {
-                        const uint32_t pos = __ldcg(off + owner) + atomicSub(cnt + owner, 1u) - 1u;
-                        pairs[2 * size_t(pos)] = owner;
-                        pairs[2 * size_t(pos) + 1] = partner;
-                    }
-                }
+        const Owner o = load_owner(bounds, body, i);
+        uint32_t found = 0;
+        for (uint32_t base = (i + 1) & ~31u; base < n && found < end - begin; base += 32) {
+            const uint32_t j = base + lane;
+            const uint32_t* b = bounds + 6 * size_t(j < n ? j : i);
+            const bool hit = j < n && j > i && overlap_x(o, b[0], b[3]) && overlap_z(o, b[2], b[5]) &&
+                             overlap_rest(o, b[1], b[4], body[j]);
+            const uint32_t bits = __ballot_sync(0xffffffffu, hit);
+            const size_t at = found + __popc(bits & lt);
+            if (hit) {
+                p[2 * at] = i;
+                p[2 * at + 1] = j;
             }
-        }
-        __syncthreads();
-        if (!fill) {
-            const uint32_t total = block_scan(cnt, off, n);
-            if (threadIdx.x == 0) {
-                *count = total;
-                s_total = total;
-            }
-            __syncthreads();
-        }
-    }
-    // each written owner bucket [off[o], off[o + 1]) sorted by partner
-    // (insertion sort; buckets are short)
-    for (uint32_t o = threadIdx.x; o < n; o += kThreads) {
-        const uint32_t begin = __ldcg(off + o);
-        const uint32_t end = o + 1 < n ? __ldcg(off + o + 1) : s_total;
-        const uint32_t c = end - begin;
-        if (c < 2 || end > cap) continue;
-        uint32_t* p = pairs + 2 * size_t(begin) + 1;
-        for (uint32_t i = 1; i < c; ++i) {
-            const uint32_t v = p[2 * size_t(i)];
-            uint32_t j = i;
-            while (j > 0 && p[2 * size_t(j - 1)] > v) { p[2 * size_t(j)] = p[2 * size_t(j - 1)]; --j; }
-            p[2 * size_t(j)] = v;
+            found += __popc(bits);
         }
     }
 }
@@ -219,8 +246,8 @@ void put_message(char* out, size_t len, const char* a, const char* b = "") {
 
 // Once per device (per CUDA context of the device: a context made after
 // cudaDeviceReset loads this module again), with that device current:
-// resolve the scratch array's address and allow the kernel the shared
-// memory its largest sort needs.
+// resolve the scratch array's address and allow the counting kernel the
+// shared memory its largest input needs.
 int setup_device(int dev, unsigned char** out, char* msg, size_t msg_len) {
     std::lock_guard<std::mutex> lock(g_setup_mutex);
     if (!g_ctx_get) {
@@ -245,8 +272,8 @@ int setup_device(int dev, unsigned char** out, char* msg, size_t msg_len) {
             put_message(msg, msg_len, "cudaGetSymbolAddress failed: ", cudaGetErrorString(e));
             return FYZZ_B200_RUNTIME_ERROR;
         }
-        e = cudaFuncSetAttribute(k_sap_static, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(kMaxSortSmem));
+        e = cudaFuncSetAttribute(k_sap_count, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(kMaxCountSmem));
         if (e != cudaSuccess) {
             put_message(msg, msg_len, "cudaFuncSetAttribute failed: ", cudaGetErrorString(e));
             return FYZZ_B200_RUNTIME_ERROR;
@@ -285,11 +312,15 @@ extern "C" int fyzz_b200_sap_pairs_static_scratch(const uint32_t* bounds_dev, co
     }
     unsigned char* scratch = nullptr;
     if (const int rc = setup_device(dev, &scratch, message, message_len)) return rc;
-    uint32_t m = 1;
-    while (m < n_shapes) m <<= 1;
-    k_sap_static<<<1, kThreads, size_t(m) * sizeof(unsigned long long),
-                   static_cast<cudaStream_t>(stream)>>>(bounds_dev, body_dev, n_shapes, pairs_dev,
-                                                        pair_cap, count_dev, scratch);
+    const auto st = static_cast<cudaStream_t>(stream);
+    const uint32_t warps = ((n_shapes + 1) / 2 + 1) / 2;
+    if (n_shapes > 1)
+        k_sap_count<<<(warps * 32 + kCountThreads - 1) / kCountThreads, kCountThreads, n_shapes * kShapeSmem, st>>>(
+            bounds_dev, body_dev, n_shapes, scratch);
+    // a single shape has no pairs: its bucket is not counted
+    const uint32_t owners = n_shapes > 1 ? n_shapes : 0u;
+    k_sap_fill<<<owners ? (owners + kFillOwners - 1) / kFillOwners : 1u, kFillThreads, 0, st>>>(
+        bounds_dev, body_dev, owners, pairs_dev, pair_cap, count_dev, scratch);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         put_message(message, message_len, "launch failed: ", cudaGetErrorString(e));
