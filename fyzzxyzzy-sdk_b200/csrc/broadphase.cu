@@ -82,35 +82,56 @@ __global__ void k_shape_bounds(DevState s) {
 }
 
 // One CTA sorts one scene's min-x endpoints by (value, shape id): bitonic
-// sort of 64-bit keys in shared memory.
-constexpr int kSmallSortThreads = 1024;
-__global__ void __launch_bounds__(kSmallSortThreads) k_sort_small(DevState s) {
-    extern __shared__ unsigned long long sk[];
+// sort of 64-bit keys, two consecutive ones a thread.  Strides up to 32 stay
+// inside a warp (shuffles), wider ones exchange through shared memory, one
+// barrier each (two buffers in turn): 15 barriers for 2,048 keys where every
+// one of the 66 stages had its own.  Threads beyond the scene's keys leave
+// at once.  The stages are a serial chain and bound the kernel: 1,201 shapes
+// 21.8 us before.
+struct EndKey { uint32_t hi, lo; };   // value, shape id
+__device__ __forceinline__ bool key_less(EndKey a, EndKey b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
+__device__ __forceinline__ EndKey key_pick(EndKey mine, EndKey other, bool want_min) {
+    return key_less(other, mine) == want_min ? other : mine;
+}
+__global__ void __launch_bounds__(1024) k_sort_small(DevState s) {
+    extern __shared__ uint4 xchg[];   // 2 x blockDim.x
     const uint32_t scene = s.small_scenes[blockIdx.x];
-    const uint32_t begin = s.sc_fbegin[scene], end = s.sc_fbegin[scene + 1];
-    const uint32_t n = end - begin;
-    uint32_t m = 1;
+    const uint32_t begin = s.sc_fbegin[scene], n = s.sc_fbegin[scene + 1] - begin;
+    uint32_t m = 64;
     while (m < n) m <<= 1;
-    for (uint32_t i = threadIdx.x; i < m; i += blockDim.x)
-        sk[i] = i < n ? ((unsigned long long)s.srt_key[begin + i] << 32) | s.srt_id[begin + i]
-                      : ~0ull;
-    __syncthreads();
-    for (uint32_t k = 2; k <= m; k <<= 1)
-        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-                const uint32_t ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = sk[i], b = sk[ixj];
-                    const bool up = (i & k) == 0;
-                    if ((a > b) == up) { sk[i] = b; sk[ixj] = a; }
-                }
-            }
+    const uint32_t t = threadIdx.x, i = 2 * t;
+    if (t >= m / 2) return;           // whole warps
+    EndKey e0 = {~0u, ~0u}, e1 = {~0u, ~0u};
+    if (i < n) e0 = {s.srt_key[begin + i], s.srt_id[begin + i]};
+    if (i + 1 < n) e1 = {s.srt_key[begin + i + 1], s.srt_id[begin + i + 1]};
+    uint32_t buf = 0;
+    for (uint32_t k = 2; k <= m; k <<= 1) {
+        const bool up = (i & k) == 0;
+        for (uint32_t j = k >> 1; j >= 64; j >>= 1) {
+            xchg[buf + t] = make_uint4(e0.hi, e0.lo, e1.hi, e1.lo);
             __syncthreads();
+            const uint4 o = xchg[buf + (t ^ (j >> 1))];
+            const bool want_min = ((i & j) == 0) == up;
+            e0 = key_pick(e0, {o.x, o.y}, want_min);
+            e1 = key_pick(e1, {o.z, o.w}, want_min);
+            buf ^= blockDim.x;
         }
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        s.srt_key[begin + i] = uint32_t(sk[i] >> 32);
-        s.srt_id[begin + i] = uint32_t(sk[i]);
+        for (uint32_t j = min(k >> 1, 32u); j >= 2; j >>= 1) {
+            const int d = int(j >> 1);
+            const EndKey o0 = {__shfl_xor_sync(0xffffffffu, e0.hi, d), __shfl_xor_sync(0xffffffffu, e0.lo, d)};
+            const EndKey o1 = {__shfl_xor_sync(0xffffffffu, e1.hi, d), __shfl_xor_sync(0xffffffffu, e1.lo, d)};
+            const bool want_min = ((i & j) == 0) == up;
+            e0 = key_pick(e0, o0, want_min);
+            e1 = key_pick(e1, o1, want_min);
+        }
+        if (key_less(e1, e0) == up) {
+            const EndKey x = e0;
+            e0 = e1;
+            e1 = x;
+        }
     }
+    if (i < n) { s.srt_key[begin + i] = e0.hi; s.srt_id[begin + i] = e0.lo; }
+    if (i + 1 < n) { s.srt_key[begin + i + 1] = e1.hi; s.srt_id[begin + i + 1] = e1.lo; }
 }
 
 // ---- z bands of large scenes ----
@@ -470,9 +491,9 @@ void enqueue_broadphase(const DevState& s, cudaStream_t st, const StageHook& hoo
     k_shape_bounds<<<(s.n_shapes + T - 1) / T, T, 0, st>>>(s);
     hook(kStSort, st);
     if (s.n_small) {
-        uint32_t m = 1;
-        while (m < s.max_small_scene) m <<= 1;
-        k_sort_small<<<s.n_small, kSmallSortThreads, m * sizeof(unsigned long long), st>>>(s);
+        uint32_t m = 64;
+        while (m < s.largest_small_scene) m <<= 1;
+        k_sort_small<<<s.n_small, m / 2, size_t(m) * sizeof(uint4), st>>>(s);
     }
     for (uint32_t i = 0; i < s.n_large; ++i)
         radix_sort_pairs(s.srt_key + s.large_begin[i], s.srt_id + s.large_begin[i],

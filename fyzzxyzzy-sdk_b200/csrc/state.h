@@ -63,7 +63,7 @@ struct DevState {
     uint32_t* sc_fbegin = nullptr;     // S+1, finite-shape ranges (finite-rank space)
     int32_t* sc_plane = nullptr;       // plane shape of each scene or -1
     uint32_t* small_scenes = nullptr;  // scenes sorted inside one CTA
-    uint32_t n_small = 0;
+    uint32_t n_small = 0, largest_small_scene = 0;   // its finite shapes
 
     // bodies
     float4 *b_p = nullptr, *b_q = nullptr, *b_v = nullptr, *b_w = nullptr;

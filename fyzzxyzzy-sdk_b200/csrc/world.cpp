@@ -2054,7 +2054,10 @@ private:
         for (uint32_t sc = 0; sc < nsc; ++sc) {
             const uint32_t n = fbegin[sc + 1] - fbegin[sc];
             if (n == 0) continue;
-            if (n <= d.max_small_scene) small.push_back(sc);
+            if (n <= d.max_small_scene) {
+                small.push_back(sc);
+                d.largest_small_scene = std::max(d.largest_small_scene, n);
+            }
             else {
                 if (d.n_large >= DevState::kMaxLarge) throw std::logic_error("Too many scenes above the per-CTA sort size");
                 sc_large[sc] = int32_t(d.n_large);
