@@ -397,20 +397,45 @@ __global__ void __launch_bounds__(kSweepWarps * 32) k_sweep(DevState s, const ui
 }
 
 // Sort each owner's bucket by partner id.  Plane owners are filled in
-// ascending order already.
+// ascending order already.  Buckets of up to kBucketSerial keys (nearly all)
+// are sorted by one thread; a longer one (a platform under many bodies) by
+// its warp, each key placed at the number of smaller ones, with the partners
+// staged in found_flag (written by k_pair_match afterwards).  One thread's
+// insertion sort of a 60-key bucket in global memory took 43 us.
+constexpr uint32_t kBucketSerial = 8;
 __global__ void k_owner_sort(DevState s) {
     const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-    if (o >= s.n_shapes || s.s_type[o] == kPlane) return;
-    const uint32_t n = s.s_static_pairs[o] + s.own_cur[o];
-    if (n < 2) return;
-    const uint32_t b = s.own_off[o];
-    if (b + n > s.pair_cap) return;
+    uint32_t n = 0, b = 0;
+    if (o < s.n_shapes && s.s_type[o] != kPlane) {
+        n = s.s_static_pairs[o] + s.own_cur[o];
+        b = s.own_off[o];
+        if (b + n > s.pair_cap) n = 0;
+    }
     uint64_t* k = s.cur.key + b;
-    for (uint32_t i = 1; i < n; ++i) {
-        const uint64_t v = k[i];
-        uint32_t j = i;
-        while (j > 0 && k[j - 1] > v) { k[j] = k[j - 1]; --j; }
-        k[j] = v;
+    if (n <= kBucketSerial)
+        for (uint32_t i = 1; i < n; ++i) {
+            const uint64_t v = k[i];
+            uint32_t j = i;
+            while (j > 0 && k[j - 1] > v) { k[j] = k[j - 1]; --j; }
+            k[j] = v;
+        }
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t m = __ballot_sync(0xffffffffu, n > kBucketSerial); m; m &= m - 1) {
+        const int src = __ffs(m) - 1;
+        const uint32_t cn = __shfl_sync(0xffffffffu, n, src), cb = __shfl_sync(0xffffffffu, b, src);
+        uint64_t* key = s.cur.key + cb;
+        uint32_t* partner = s.found_flag + cb;
+        for (uint32_t i = lane; i < cn; i += 32) partner[i] = uint32_t(key[i]);
+        __syncwarp();
+        const uint64_t owner = key[0] & 0xffffffff00000000ull;
+        __syncwarp();
+        for (uint32_t i = lane; i < cn; i += 32) {
+            const uint32_t mine = partner[i];
+            uint32_t rank = 0;
+            for (uint32_t j = 0; j < cn; ++j) rank += partner[j] < mine ? 1u : 0u;
+            key[rank] = owner | mine;
+        }
+        __syncwarp();
     }
 }
 
