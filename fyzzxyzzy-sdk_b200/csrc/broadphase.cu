@@ -439,16 +439,6 @@ __global__ void k_owner_sort(DevState s) {
     }
 }
 
-__global__ void k_pair_total(DevState s) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        const uint32_t total = *s.cur.n;
-        if (total > s.pair_cap) {
-            atomicOr(s.err, kErrPairCapacity);
-            *s.cur.n = s.pair_cap;
-        }
-    }
-}
-
 __device__ __forceinline__ int32_t find_key(const uint64_t* keys, uint32_t lo, uint32_t hi, uint64_t key) {
     const uint32_t end = hi;
     while (lo < hi) {
@@ -459,9 +449,15 @@ __device__ __forceinline__ int32_t find_key(const uint64_t* keys, uint32_t lo, u
 }
 
 // Per shape, before the sweep: its bucket count starts at its plane pairs,
-// its fill cursor at zero, and its previous-generation bucket empty.
+// its fill cursor at zero, and its previous-generation bucket empty.  The
+// first thread also clears the narrowphase's list counters: a memset node of
+// its own costs the step's chain 2 to 4 us each.
 __global__ void k_owner_init(DevState s) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == 0) {
+        for (int c : {int(kCntGjk), int(kCntConvex), int(kCntConvexGjk), int(kCntConvexClip), int(kCntConvexEpa)})
+            s.counters[c] = 0u;
+    }
     if (i >= s.n_shapes) return;
     s.own_cnt[i] = s.s_static_pairs[i];
     s.own_cur[i] = 0u;
@@ -540,13 +536,14 @@ void enqueue_broadphase(const DevState& s, cudaStream_t st, const StageHook& hoo
                          s.sort_hist_words, s.scan_tmp, s.scan_tmp_words, st, s.err, 8, s.sort_os, s.sort_os_words);
         k_band_gather<<<(s.bx_cap + T - 1) / T, T, 0, st>>>(s, rec, meta);
     }
-    if (s.n_shapes) k_owner_init<<<(s.n_shapes + T - 1) / T, T, 0, st>>>(s);
+    k_owner_init<<<(s.n_shapes + T) / T, T, 0, st>>>(s);   // at least one block
     const uint32_t sweep_threads = kSweepWarps * 32;
     const uint32_t n_sweep = s.n_finite + s.bx_cap;
     const uint32_t sweep_blocks = s.n_finite ? (n_sweep + sweep_threads - 1) / sweep_threads : 0;
     if (sweep_blocks) k_sweep<<<sweep_blocks, sweep_threads, 0, st>>>(s, rec, meta, 0);
-    scan_exclusive(s.own_cnt, s.own_off, s.n_shapes, nullptr, s.cur.n, s.scan_tmp, s.scan_tmp_words, st, s.err);
-    k_pair_total<<<1, 32, 0, st>>>(s);
+    // more pairs than the budget: an error, and the count stops at the budget
+    scan_exclusive(s.own_cnt, s.own_off, s.n_shapes, nullptr, s.cur.n, s.scan_tmp, s.scan_tmp_words, st, s.err,
+                   s.pair_cap);
     if (sweep_blocks) k_sweep<<<sweep_blocks, sweep_threads, 0, st>>>(s, rec, meta, 1);
     k_owner_sort<<<(s.n_shapes + T - 1) / T, T, 0, st>>>(s);
     const uint32_t mb = (s.pair_cap + T - 1) / T;

@@ -2041,14 +2041,11 @@ __global__ void __launch_bounds__(kCvxWarps * 32) k_narrowphase_convex_clip(DevS
 void enqueue_narrowphase(const DevState& s, cudaStream_t st, const StageHook& hook) {
     const int T = 128;
     hook(kStNarrow, st);
-    cudaMemsetAsync(s.counters + kCntGjk, 0, 4, st);
-    cudaMemsetAsync(s.counters + kCntConvex, 0, 8, st);
     const uint32_t blocks = (s.pair_cap + T - 1) / T;
     k_narrowphase<<<blocks < 148u * 16u ? blocks : 148u * 16u, T, 0, st>>>(s);
     const uint32_t gb = (s.pair_cap + kGjkWarps - 1) / kGjkWarps;
     k_narrowphase_gjk<<<gb < 148u * 8u ? gb : 148u * 8u, kGjkWarps * 32, 0, st>>>(s);
     if (s.n_meshes) {
-        cudaMemsetAsync(s.counters + kCntConvexClip, 0, 8, st);   // clip and EPA lists
         k_narrowphase_convex<<<blocks < 148u * 16u ? blocks : 148u * 16u, T, 0, st>>>(s);
         const uint32_t cb = (s.pair_cap + kCvxWarps - 1) / kCvxWarps;
         k_narrowphase_convex_gjk<<<cb < 148u * 8u ? cb : 148u * 8u, kCvxWarps * 32, 0, st>>>(s);

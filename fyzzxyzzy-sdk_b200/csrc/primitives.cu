@@ -38,7 +38,7 @@ __device__ __forceinline__ void os_state_store(unsigned long long* p, unsigned l
 }
 __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const uint32_t* in, uint32_t* out, uint32_t n,
                                                                const uint32_t* n_dev, uint32_t* total,
-                                                               uint32_t* tmp, uint32_t* err) {
+                                                               uint32_t* tmp, uint32_t* err, uint32_t total_cap) {
     __shared__ uint32_t sm[kScanThreads / 32 + 1];
     __shared__ uint32_t s_tile, s_prefix;
     unsigned long long* state = reinterpret_cast<unsigned long long*>(tmp + kScanHeader);
@@ -96,7 +96,11 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_lookback(const uint32_t* 
             if (lane == 0) {
                 if (tile != 0) scan_state_store(&state[tile], tag | (2ull << 32) | (prefix + agg));
                 s_prefix = prefix;
-                if (total && uint64_t(tile + 1) * kScanTile >= lim) *total = prefix + agg;
+                if (total && uint64_t(tile + 1) * kScanTile >= lim) {
+                    const uint32_t sum = prefix + agg;
+                    if (sum > total_cap && err) atomicOr(err, kErrPairCapacity);
+                    *total = min(sum, total_cap);
+                }
             }
         }
         __syncthreads();
@@ -213,7 +217,7 @@ constexpr int kOsMaxPasses = 4, kOsMaxDigits = 512;
 constexpr uint32_t kOsHeader = 4, kOsHist = kOsMaxPasses * kOsMaxDigits;
 constexpr int kOsLook = 8;   // predecessors read together in the look-back
 
-// Digit totals of every pass (ghist must be zero).
+// Digit totals of every pass (ghist is zero between sorts).
 template <int B>
 __global__ void __launch_bounds__(kSortThreads) k_os_hist(const uint32_t* __restrict__ keys, uint32_t n,
                                                          const uint32_t* n_dev, int begin_bit, int passes,
@@ -242,7 +246,8 @@ __global__ void __launch_bounds__(kSortThreads) k_os_scatter(const uint32_t* __r
                                                             uint32_t* __restrict__ vout, uint32_t n,
                                                             const uint32_t* n_dev, int shift,
                                                             const uint32_t* __restrict__ ghist, uint32_t* ctl,
-                                                            unsigned long long* state, uint32_t* err) {
+                                                            unsigned long long* state, uint32_t* err,
+                                                            uint32_t* clear, uint32_t clear_n) {
     constexpr uint32_t R = 1u << B, DPT = R / kSortThreads;   // digits a thread looks after
     __shared__ uint32_t wcount[kSortWarps][R + 1];
     __shared__ uint32_t wofs[kSortWarps][R + 1];
@@ -351,16 +356,23 @@ __global__ void __launch_bounds__(kSortThreads) k_os_scatter(const uint32_t* __r
             }
         }
     }
-    // the last live block to finish opens the next epoch and resets the ticket
+    // the last live block to finish opens the next epoch, resets the ticket
+    // and, in the sort's last pass, clears the digit totals for the next sort
+    // (a memset before every sort cost its chain about 6 us)
+    __shared__ bool last;
     if (threadIdx.x == 0) {
         __threadfence();
-        if (atomicAdd(&ctl[2], 1u) == live - 1) {
+        last = atomicAdd(&ctl[2], 1u) == live - 1;
+        if (last) {
             ctl[0] = (epoch + 1u) & 0x3fffffffu;
             ctl[1] = 0u;
             ctl[2] = 0u;
             __threadfence();
         }
     }
+    __syncthreads();
+    if (last)
+        for (uint32_t i = threadIdx.x; i < clear_n; i += kSortThreads) clear[i] = 0u;
 }
 
 // The live entries of a sort that ended in the alternate buffers, copied
@@ -380,13 +392,13 @@ void onesweep_sort(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t*
                    cudaStream_t st, uint32_t* err) {
     uint32_t* ghist = os_scratch + kOsHeader;
     auto* state = reinterpret_cast<unsigned long long*>(os_scratch + kOsHeader + kOsHist);
-    cudaMemsetAsync(ghist, 0, size_t(passes) * (1u << B) * 4, st);
     k_os_hist<B><<<ntiles < 296u ? ntiles : 296u, kSortThreads, 0, st>>>(keys, n_cap, n_dev, begin_bit, passes,
                                                                          ghist);
     uint32_t *ki = keys, *vi = vals, *ko = keys_alt, *vo = vals_alt;
     for (int p = 0; p < passes; ++p) {
         k_os_scatter<B><<<ntiles, kSortThreads, 0, st>>>(ki, vi, ko, vo, n_cap, n_dev, begin_bit + B * p,
-                                                          ghist + (1u << B) * p, os_scratch, state, err);
+                                                          ghist + (1u << B) * p, os_scratch, state, err, ghist,
+                                                          p + 1 == passes ? uint32_t(passes) << B : 0u);
         uint32_t* t = ki; ki = ko; ko = t;
         t = vi; vi = vo; vo = t;
     }
@@ -414,7 +426,8 @@ size_t scan_tmp_words_for(uint32_t n_cap) {
 
 // The scratch must be zero when first used (world allocation clears it).
 void scan_exclusive(const uint32_t* in, uint32_t* out, uint32_t n, const uint32_t* n_dev,
-                    uint32_t* total, uint32_t* tmp, size_t tmp_words, cudaStream_t st, uint32_t* err) {
+                    uint32_t* total, uint32_t* tmp, size_t tmp_words, cudaStream_t st, uint32_t* err,
+                    uint32_t total_cap) {
     const uint32_t nb = (n + kScanTile - 1) / kScanTile;
     if (nb == 0) {
         if (total) cudaMemsetAsync(total, 0, 4, st);
@@ -425,7 +438,8 @@ void scan_exclusive(const uint32_t* in, uint32_t* out, uint32_t n, const uint32_
         return;
     }
     // two blocks per SM at most: the whole grid is resident
-    k_scan_lookback<<<nb < 296u ? nb : 296u, kScanThreads, 0, st>>>(in, out, n, n_dev, total, tmp, err);
+    k_scan_lookback<<<nb < 296u ? nb : 296u, kScanThreads, 0, st>>>(in, out, n, n_dev, total, tmp, err,
+                                                                total_cap);
 }
 
 size_t onesweep_words(uint32_t n_cap) {

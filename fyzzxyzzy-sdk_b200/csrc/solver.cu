@@ -36,7 +36,9 @@ constexpr int kMaxLevels = 256;
 constexpr uint32_t kSerialIsland = 32;   // partitioned by one thread
 
 __global__ void k_frame_begin(DevState s) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) s.counters[kCntFrame] += 1u;
+    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    s.counters[kCntFrame] += 1u;
+    for (int c : {int(kCntAwake), int(kCntSleeping), int(kCntReady), int(kCntActivating)}) s.counters[c] = 0u;
 }
 
 __device__ __forceinline__ bool is_asleep(const DevState& s, uint32_t b) {
@@ -2304,9 +2306,6 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     auto side = [&](int i) { return br ? br->st[i] : st; };
     hook(kStIslands, st);
     k_frame_begin<<<1, 32, 0, st>>>(s);
-    cudaMemsetAsync(s.counters + kCntAwake, 0, 2 * sizeof(uint32_t), st);
-    cudaMemsetAsync(s.counters + kCntReady, 0, sizeof(uint32_t), st);
-    cudaMemsetAsync(s.counters + kCntActivating, 0, sizeof(uint32_t), st);
     k_bodies_begin<<<grid_for(s.n_bodies, T, 1u << 30), T, 0, st>>>(s);
     // touching managers in canonical pair order
     k_touch_compact<<<lookback_grid(s.pair_cap), kScanThreads, 0, st>>>(s);
