@@ -251,20 +251,30 @@ __device__ __forceinline__ void rel_adj(v3 n, v3 ra, v3 rb, v3 av, v3 aw, v3 bv,
     g.rb = vsub(g.rb, vmul(bw, gb));
 }
 
-// Adds a row-gradient increment to its accumulator with 128-bit accesses
-// (the row records are 16-byte aligned; fields the increment leaves at 0
-// are unchanged).
+// Adds a row-gradient increment to its accumulator: reductions of 128 bits
+// without a reply.  One thread at a time owns a row (its descriptor's), so
+// the sum is that of a load, an add and a store, but no row waits for the
+// previous row's accumulator to come back.
 template <class T> __device__ __forceinline__ void add_row(T& dst, const T& inc) {
     static_assert(sizeof(T) % 16 == 0 && alignof(T) == 16, "16-byte row record");
     float4* d = reinterpret_cast<float4*>(&dst);
     const float4* a = reinterpret_cast<const float4*>(&inc);
 #pragma unroll
-    for (int k = 0; k < int(sizeof(T) / 16); ++k) {
-        float4 x = d[k];
-        const float4 y = a[k];
-        x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
-        d[k] = x;
-    }
+    for (int k = 0; k < int(sizeof(T) / 16); ++k)
+        asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d + k), "f"(a[k].x), "f"(a[k].y),
+                     "f"(a[k].z), "f"(a[k].w)
+                     : "memory");
+}
+// A row of the forward step (read-only here, so the loads of all a
+// manager's rows can be in flight before the first is used).
+template <class T> __device__ __forceinline__ T load_row(const T* row) {
+    static_assert(sizeof(T) == 64 && alignof(T) == 16, "64-byte row record");
+    T r;
+    const float4* s = reinterpret_cast<const float4*>(row);
+    float4* d = reinterpret_cast<float4*>(&r);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) d[k] = __ldg(s + k);
+    return r;
 }
 template <class R>
 __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, uint32_t lid, int it, int pos,
@@ -307,6 +317,18 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
     const uint32_t m = d - s.n_joints;
     const ManagerHeader hd = s.mh[m];
     const float ima = hd.ima, imb = hd.imb;
+    // Every load of the descriptor is issued here, before the first use: a
+    // row at a time, each waited for its own round trip, which made up nearly
+    // all of the 10 us a level took.
+    const bool friction = (it >= pos || pos - it <= 3) && hd.anchors;
+    FrictionRow frow[4];
+    NormalRow nrow[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (friction && k < int(2 * hd.anchors)) frow[k] = load_row(s.frow + 4 * size_t(m) + k);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        if (j < int(hd.count)) nrow[j] = load_row(s.nrow + 4 * size_t(m) + j);
     int32_t h0, h1;
     if constexpr (R::kLocal) {
         h0 = local_handle(lid & 0xffffu); h1 = local_handle(lid >> 16);
@@ -327,7 +349,7 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
     float yv[4] = {y4.x, y4.y, y4.z, y4.w};
     RowAdj hg = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, 0.0f, 0.0f};
     float nsumb = 0.0f, dfb = 0.0f;
-    const bool friction = (it >= pos || pos - it <= 3) && hd.anchors;
+    const float4 yo4 = it > 0 ? tn4[slot - cap] : zero4;
     if (friction) {
         const bool prev_friction = it > 0 && (it - 1 >= pos || pos - (it - 1) <= 3);
         const float4 x4 = tf4[slot], xo4 = prev_friction ? tf4[slot - cap] : zero4;
@@ -344,7 +366,7 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
 #pragma unroll
         for (int k = 3; k >= 0; --k) {
             if (k >= int(2 * hd.anchors)) continue;
-            const FrictionRow f = s.frow[4 * size_t(m) + k];
+            const FrictionRow& f = frow[k];
             const v3 t = lv(f.t), ra = lv(f.ra), rb = lv(f.rb);
             const float xn = xt[k];
             const float xo = xto[k];
@@ -380,12 +402,11 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
         dfb += coeff * nsum * mdb;
         nsumb += hd.df * coeff * mdb;
     }
-    const float4 yo4 = it > 0 ? tn4[slot - cap] : zero4;
     const float tno[4] = {yo4.x, yo4.y, yo4.z, yo4.w};
 #pragma unroll
     for (int j = 3; j >= 0; --j) {
         if (j >= int(hd.count)) continue;
-        const NormalRow r = s.nrow[4 * size_t(m) + j];
+        const NormalRow& r = nrow[j];
         const v3 n = lv(r.n), ra = lv(r.ra), rb = lv(r.rb);
         const float yn = tn[j];
         const float yo = tno[j];
@@ -411,9 +432,9 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
         yv[j] = yob;
     }
     reinterpret_cast<float4*>(A.yn)[m] = make_float4(yv[0], yv[1], yv[2], yv[3]);
-    float4 h = A.hd[m];
-    h.x += hg.ima; h.y += hg.imb; h.w += dfb;
-    A.hd[m] = h;
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(A.hd + m), "f"(hg.ima), "f"(hg.imb),
+                 "f"(0.0f), "f"(dfb)
+                 : "memory");
     D.store(h0, av, aw, avb, awb);
     D.store(h1, bv, bw, bvb, bwb);
 }
