@@ -300,6 +300,11 @@ struct Branches {
 void fork_branches(const Branches* br, cudaStream_t st, int n);
 void join_branches(const Branches* br, cudaStream_t st, int n);
 
+// Fork n side branches off st / join them (or run everything on st without
+// branches).
+void fork_branches(const Branches* br, cudaStream_t st, int n);
+void join_branches(const Branches* br, cudaStream_t st, int n);
+
 // Reverse-mode state of a differentiated rollout (adjoint.cu).  Per body,
 // the adjoint of the mass-frame state (centre c, orientation Q) and the
 // velocities: on entry to a step's reverse pass it refers to the end of
@@ -329,7 +334,7 @@ struct AdjState {
 void enqueue_copy_set(const ManagerSet& dst, const ManagerSet& src, uint32_t cap, cudaStream_t st);
 // adjoint.cu
 void enqueue_adjoint_save_start(const DevState& s, const AdjState& a, cudaStream_t st);
-void enqueue_adjoint_step(const DevState& s, const AdjState& a, cudaStream_t st);
+void enqueue_adjoint_step(const DevState& s, const AdjState& a, cudaStream_t st, const Branches* br = nullptr);
 
 // broadphase.cu / narrowphase.cu / solver.cu
 void enqueue_broadphase(const DevState& s, cudaStream_t st, const StageHook& hook = {});

@@ -1139,7 +1139,7 @@ public:
         s.counters = f.counters;
         AdjState a = adj_;
         a.x_c = f.x_c; a.x_q = f.x_q;
-        enqueue_adjoint_step(s, a, stream_);
+        enqueue_adjoint_step(s, a, stream_, &br_);
     }
     void rollout_backward(const float* gc, const float* gq, const float* gv, const float* gw,
                           float* gv0, float* gw0, float* gmass, float* gfs, float* gfd) {
