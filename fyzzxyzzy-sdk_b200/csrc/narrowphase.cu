@@ -370,27 +370,50 @@ template <bool G> __device__ Sup bp_support(const BPair& p, v3 dir) {
 }
 __device__ __forceinline__ v3 bp_local_a(const BPair& p, v3 pb) { return rotinv_gu(p.rel, vsub(pb, p.a_in_b)); }
 __device__ __forceinline__ float box_min_margin(v3 h) { return 0.05f * smin(smin(h.x, h.y), h.z); }
-__device__ bool solve_small(int n, float a[3][4], float r[3]) {
+// Gauss-Jordan elimination with partial pivoting of n <= 3 equations (a, right
+// side b; the solution in b).  Every index is static and the size a
+// predicate, so the system stays in registers: with indexed loops it lived
+// in local memory, whose round trips were most of a sub-simplex search.
+__device__ __forceinline__ bool solve_small(int n, float (&a)[3][3], float (&b)[3]) {
     float scale = 0.0f;
-    for (int i = 0; i < n; ++i) scale = smax(scale, fabsf(a[i][i]));
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (i < n) scale = smax(scale, fabsf(a[i][i]));
     if (!(scale > 0.0f) || !isfinite(scale)) return false;
     const float tol = FLT_EPSILON * scale;
-    for (int col = 0; col < n; ++col) {
+    bool ok = true;
+#pragma unroll
+    for (int col = 0; col < 3; ++col) {
+        if (col >= n) break;
+        float best = fabsf(a[col][col]);
         int piv = col;
-        for (int row = col + 1; row < n; ++row)
-            if (fabsf(a[row][col]) > fabsf(a[piv][col])) piv = row;
-        if (!(fabsf(a[piv][col]) > tol)) return false;
-        for (int j = col; j <= n; ++j) { const float t = a[col][j]; a[col][j] = a[piv][j]; a[piv][j] = t; }
+#pragma unroll
+        for (int row = col + 1; row < 3; ++row)
+            if (row < n && fabsf(a[row][col]) > best) { best = fabsf(a[row][col]); piv = row; }
+        if (!(best > tol)) { ok = false; break; }
+#pragma unroll
+        for (int row = col + 1; row < 3; ++row)
+            if (row == piv) {
+#pragma unroll
+                for (int j = col; j < 3; ++j) { const float t = a[col][j]; a[col][j] = a[row][j]; a[row][j] = t; }
+                const float t = b[col]; b[col] = b[row]; b[row] = t;
+            }
         const float div = a[col][col];
-        for (int j = col; j <= n; ++j) a[col][j] /= div;
-        for (int row = 0; row < n; ++row)
-            if (row != col) {
+#pragma unroll
+        for (int j = col; j < 3; ++j)
+            if (j < n) a[col][j] /= div;
+        b[col] /= div;
+#pragma unroll
+        for (int row = 0; row < 3; ++row)
+            if (row != col && row < n) {
                 const float f = a[row][col];
-                for (int j = col; j <= n; ++j) a[row][j] = fmaf(-f, a[col][j], a[row][j]);
+#pragma unroll
+                for (int j = col; j < 3; ++j)
+                    if (j < n) a[row][j] = fmaf(-f, a[col][j], a[row][j]);
+                b[row] = fmaf(-f, b[col], b[row]);
             }
     }
-    for (int i = 0; i < n; ++i) r[i] = a[i][n];
-    return true;
+    return ok;
 }
 struct Closest { v3 point, a, b; float w[4]; unsigned mask; float dist2; };
 // Closest point of the simplex to the origin (GuPCMGjkEpa.cpp's sub-simplex
@@ -402,7 +425,7 @@ struct Closest { v3 point, a, b; float w[4]; unsigned mask; float dist2; };
 // distance).  Each lane's arithmetic is that of one iteration of the
 // sequential search, so the winner is bit for bit the same.  Every lane of
 // the warp calls this with the same simplex and gets the same result.
-__device__ Closest closest_simplex_warp(const Sup* s, int count) {
+__device__ __forceinline__ Closest closest_simplex_warp(const Sup (&s)[4], int count) {
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned mask = lane + 1u;
     Closest mine;
@@ -410,38 +433,46 @@ __device__ Closest closest_simplex_warp(const Sup* s, int count) {
     mine.w[0] = mine.w[1] = mine.w[2] = mine.w[3] = 0.0f;
     bool ok = mask < (1u << count);
     if (ok) {
-        int ids[4] = {0, 0, 0, 0}, n = 0;
-        for (int i = 0; i < count; ++i)
-            if (mask & (1u << i)) ids[n++] = i;
-        float w[4] = {0, 0, 0, 0};
-        w[ids[0]] = 1.0f;
+        // the subset's vertices in order: base, then up to three others
+        const int n = __popc(mask);
+        const auto pick = [&](unsigned m) -> v3 {
+            return m & 1u ? s[0].q : m & 2u ? s[1].q : m & 4u ? s[2].q : s[3].q;
+        };
+        const unsigned m1 = mask & (mask - 1u), m2 = m1 & (m1 - 1u), m3 = m2 & (m2 - 1u);
+        const v3 base = pick(mask);
+        float coef[3] = {0, 0, 0};
         if (n > 1) {
-            const v3 base = s[ids[0]].q;
-            v3 dirs[3];
-            float m[3][4] = {{0, 0, 0, 0}, {0, 0, 0, 0}, {0, 0, 0, 0}};
-            for (int i = 1; i < n; ++i) dirs[i - 1] = vsub(s[ids[i]].q, base);
-            for (int i = 1; i < n; ++i) {
-                for (int j = 1; j < n; ++j) m[i - 1][j - 1] = vdot(dirs[i - 1], dirs[j - 1]);
-                m[i - 1][n - 1] = -vdot(dirs[i - 1], base);
+            const v3 dirs[3] = {vsub(pick(m1), base), vsub(pick(m2), base), vsub(pick(m3), base)};
+            float a[3][3];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+#pragma unroll
+                for (int j = 0; j < 3; ++j) a[i][j] = vdot(dirs[i], dirs[j]);
+                coef[i] = -vdot(dirs[i], base);
             }
-            float coef[3] = {0, 0, 0};
-            if (!solve_small(n - 1, m, coef)) ok = false;
-            for (int i = 1; i < n; ++i) {
-                w[ids[i]] = coef[i - 1];
-                w[ids[0]] -= coef[i - 1];
-            }
+            if (!solve_small(n - 1, a, coef)) ok = false;
         }
-        for (int i = 0; i < n; ++i)
-            if (w[ids[i]] < -1.0e-5f) ok = false;
+        float w0 = 1.0f;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            if (i + 1 < n) w0 -= coef[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int at = __popc(mask & ((1u << i) - 1u));   // place of vertex i in the subset
+            const float w = at == 0 ? w0 : at == 1 ? coef[0] : at == 2 ? coef[1] : coef[2];
+            mine.w[i] = (mask >> i) & 1u ? w : 0.0f;
+            if (((mask >> i) & 1u) && w < -1.0e-5f) ok = false;
+        }
         if (ok) {
             v3 q = {0, 0, 0}, pa = {0, 0, 0}, pb = {0, 0, 0};
-            for (int i = 0; i < count; ++i) {
-                q = vadd(q, vmul(s[i].q, w[i]));
-                pa = vadd(pa, vmul(s[i].a, w[i]));
-                pb = vadd(pb, vmul(s[i].b, w[i]));
-            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (i < count) {
+                    q = vadd(q, vmul(s[i].q, mine.w[i]));
+                    pa = vadd(pa, vmul(s[i].a, mine.w[i]));
+                    pb = vadd(pb, vmul(s[i].b, mine.w[i]));
+                }
             mine.point = q; mine.a = pa; mine.b = pb;
-            for (int i = 0; i < 4; ++i) mine.w[i] = w[i];
             mine.dist2 = vlen2(q);
             ok = mine.dist2 < FLT_MAX;
         }
@@ -471,10 +502,16 @@ __device__ Closest closest_simplex_warp(const Sup* s, int count) {
     best.dist2 = d;
     return best;
 }
-__device__ void compact_simplex(Sup* s, int& count, const Closest& c) {
+__device__ __forceinline__ void put_vertex(Sup (&s)[4], int at, const Sup& v) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        if (i == at) s[i] = v;
+}
+__device__ __forceinline__ void compact_simplex(Sup (&s)[4], int& count, const Closest& c) {
     int write = 0;
-    for (int read = 0; read < count; ++read)
-        if ((c.mask & (1u << read)) && c.w[read] > 1.0e-6f) s[write++] = s[read];
+#pragma unroll
+    for (int read = 0; read < 4; ++read)
+        if (read < count && (c.mask & (1u << read)) && c.w[read] > 1.0e-6f) put_vertex(s, write++, s[read]);
     if (write == 0 && count > 0) write = 1;
     count = write;
 }
@@ -567,13 +604,16 @@ template <bool G> __device__ bool contact_from_facet(const BPair& p, const Sup* 
 // returns the same mode, witness and simplex.
 // A sphere point core (G only) converges its separated distance before EPA
 // is admitted and falls back to EPA where the polyhedral search gives up.
-template <bool G> __device__ int gjk_phase(const BPair& p, float cd, Cand& out, Sup* simplex, int& count) {
+template <bool G> __device__ int gjk_phase(const BPair& p, float cd, Cand& out, Sup (&simplex)[4], int& count) {
     const float eps = 0.1f * smin(box_min_margin(p.ha), box_min_margin(p.hb));
     const float progress = 1.0f - 0.000225f;
     const bool pc = G && (p.ra > 0.f || p.rb > 0.f);
     count = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) simplex[i] = Sup{};
     v3 closest = vlen2(p.a_in_b) > 0.0f ? p.a_in_b : v3{1, 0, 0};
     float previous = FLT_MAX;
+#pragma unroll 1
     for (int it = 0; it < 32; ++it) {
         const float dist = sqrtf(vlen2(closest));
         if (count > 0 && dist <= eps && !pc) return 2;
@@ -582,21 +622,22 @@ template <bool G> __device__ int gjk_phase(const BPair& p, float cd, Cand& out, 
         const Sup s = bp_support<G>(p, vneg(closest));
         const float proj = vdot(normal, s.q);
         if (proj > cd) return 0;
-        if (count > 0 && proj > dist * progress) {
-            const Closest cur = closest_simplex_warp(simplex, count);
-            return cur.mask && contact_from_gjk(p, cur, out) ? 1 : 0;
-        }
-        for (int i = 0; i < count; ++i)
-            if (s.ai == simplex[i].ai && s.bi == simplex[i].bi) {
-                if (proj > 0.f) {
-                    const Closest cur = closest_simplex_warp(simplex, count);
-                    return cur.mask && contact_from_gjk(p, cur, out) && out.sep <= cd ? 1 : 0;
-                }
-                return pc ? 2 : 0;
+        // no more progress, or a support the simplex already holds: the
+        // witness is the simplex as it stands
+        const bool stalled = count > 0 && proj > dist * progress;
+        bool dup = false;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dup |= i < count && s.ai == simplex[i].ai && s.bi == simplex[i].bi;
+        if (!stalled) {
+            if (dup && !(proj > 0.f)) return pc ? 2 : 0;
+            if (!dup) {
+                if (count == 4) return 2;
+                put_vertex(simplex, count++, s);
             }
-        if (count == 4) return 2;
-        simplex[count++] = s;
+        }
         const Closest nx = closest_simplex_warp(simplex, count);
+        if (stalled || dup)
+            return nx.mask && contact_from_gjk(p, nx, out) && (stalled || out.sep <= cd) ? 1 : 0;
         if (!nx.mask) return 0;
         closest = nx.point;
         const float nd = sqrtf(nx.dist2);
@@ -623,7 +664,8 @@ struct EpaShared {
     int bc;
     int status;
 };
-template <bool G> __device__ bool run_epa_warp(const BPair& p, const Sup* simplex, int sc, Cand& out, EpaShared& E) {
+template <bool G>
+__device__ bool run_epa_warp(const BPair& p, const Sup (&simplex)[4], int sc, Cand& out, EpaShared& E) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t full = 0xffffffffu;
     if (G) {
@@ -632,7 +674,8 @@ template <bool G> __device__ bool run_epa_warp(const BPair& p, const Sup* simple
         Sup v0[4];
         Facet f0[4];
         int vc0 = sc, fc0 = 0;
-        for (int i = 0; i < sc; ++i) v0[i] = simplex[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v0[i] = simplex[i];
         const bool ok = init_epa<G>(p, v0, vc0, f0, fc0);
         if (lane == 0) {
             for (int i = 0; i < vc0; ++i) E.vtx[i] = v0[i];
@@ -642,7 +685,9 @@ template <bool G> __device__ bool run_epa_warp(const BPair& p, const Sup* simple
         }
     } else if (lane == 0) {
         int vc0 = sc;
-        for (int i = 0; i < sc; ++i) E.vtx[i] = simplex[i];
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (i < sc) E.vtx[i] = simplex[i];
         int fc0 = 0;
         E.status = init_epa<G>(p, E.vtx, vc0, E.facets, fc0) ? fc0 : -1;
         E.bc = vc0;
