@@ -300,11 +300,6 @@ struct Branches {
 void fork_branches(const Branches* br, cudaStream_t st, int n);
 void join_branches(const Branches* br, cudaStream_t st, int n);
 
-// Fork n side branches off st / join them (or run everything on st without
-// branches).
-void fork_branches(const Branches* br, cudaStream_t st, int n);
-void join_branches(const Branches* br, cudaStream_t st, int n);
-
 // Reverse-mode state of a differentiated rollout (adjoint.cu).  Per body,
 // the adjoint of the mass-frame state (centre c, orientation Q) and the
 // velocities: on entry to a step's reverse pass it refers to the end of
