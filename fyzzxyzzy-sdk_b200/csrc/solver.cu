@@ -823,6 +823,10 @@ __host__ __device__ constexpr uint32_t pow2_at_least(uint32_t x) {
 template <uint32_t MAXN> struct PartSmem {
     static constexpr uint32_t kTable = pow2_at_least(3 * (MAXN + 1) / 2 + 1);
     static constexpr size_t kBytes = (2 * size_t(kTable) + 2 * size_t(MAXN)) * 4;
+    // A round is a few dependent shared-memory accesses a descriptor: above
+    // 512 descriptors, 256 threads took eight turns at them (61 us for an
+    // island of 1,923, 35 rounds).
+    static constexpr uint32_t kThreads = MAXN > kMidIsland ? 1024u : 256u;
 };
 
 __device__ __forceinline__ uint32_t body_hash(int32_t b, uint32_t lg) {
@@ -847,7 +851,8 @@ __device__ __forceinline__ uint32_t find_local(const uint32_t* key, const uint32
 // descriptor offers its index to its bodies (atomicMin), then the ones that
 // won on both bodies are decided and clear their bodies' minimum.
 template <uint32_t MAXN>
-__global__ void __launch_bounds__(256) k_partition_smem(DevState s, uint32_t* lvl_bound, int list_class) {
+__global__ void __launch_bounds__(PartSmem<MAXN>::kThreads) k_partition_smem(DevState s, uint32_t* lvl_bound,
+                                                                            int list_class) {
     constexpr uint32_t TMAX = PartSmem<MAXN>::kTable;
     extern __shared__ uint32_t sm[];
     uint32_t* key = sm;              // [T] hashed body ids
@@ -2342,7 +2347,7 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     // partitions by island size class, and row preparation: independent
     hook(kStPrep, st);
     fork_branches(br, st, 3);
-    launch(k_partition_smem<kBigIsland>, grid_for(s.desc_cap, kMidIsland + 1, 148u * 2u), 256u,
+    launch(k_partition_smem<kBigIsland>, grid_for(s.desc_cap, kMidIsland + 1, 148u * 2u), PartSmem<kBigIsland>::kThreads,
                 PartSmem<kBigIsland>::kBytes, 1u, g_high_priority, side(1), s, lvl_bound, 2);
     launch(k_partition_large, grid_for(s.desc_cap, kBigIsland + 1, 148u), 256u, size_t(0), 1u, g_high_priority, side(1), s,
                 lvl_bound);
