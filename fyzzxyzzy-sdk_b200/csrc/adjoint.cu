@@ -459,47 +459,85 @@ __device__ __forceinline__ void inject_motion(const DevState& s, const AdjState&
     }
 }
 
-// Reverse PGS sweep over island-local slots in shared memory: one warp per
-// island of <= kSmallIsland descriptors (4 warps per block).
-// One thread per tiny island (<= kRevTiny descriptors): its descriptors in
-// reverse placed order (levels in reverse; a level's descriptors share no
-// body), with the deltas and their adjoints in the thread's slice of shared
-// memory.  Most islands of a loose pile are a box resting alone.
-constexpr uint32_t kRevTiny = 8;
-constexpr uint32_t kRevThreadBlock = 64;
-__global__ void __launch_bounds__(kRevThreadBlock) k_adj_pgs_thread(DevState s, AdjState A) {
-    __shared__ float4 sh[kRevThreadBlock][4 * (kRevTiny + 1)];
-    const uint32_t ni = *s.n_isl;
+// Reverse PGS sweeps over island-local slots in shared memory.
+constexpr uint32_t kRevWarps = 4;
+// Islands of at most kRevSmall descriptors, several to a warp: an island of
+// (2^(c-1), 2^c] descriptors (the forward's list kSmallList + c) takes 2^c
+// lanes, one descriptor each, and the warp steps through its islands' levels
+// together, in reverse.  One thread an island of up to 8 took 198 us a step
+// (its descriptors one after another, each a few round trips to memory), one
+// warp an island of up to 96 328 us (most lanes idle).
+constexpr uint32_t kRevSmall = 32;
+__global__ void __launch_bounds__(kRevWarps * 32) k_adj_pgs_packed(DevState s, AdjState A, const uint32_t* lvl_bound) {
+    __shared__ float4 sh[kRevWarps][4 * 2 * 32];
+    const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     const int pos = s.pos_iters, vel = s.vel_iters < 1 ? 1 : s.vel_iters;
-    float4* my = sh[threadIdx.x];
-    const RevLocal D{my};
-    const uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t isl = blockIdx.x * blockDim.x + threadIdx.x; isl < ni; isl += stride) {
-        const uint32_t begin = s.isl_begin[isl], end = s.isl_begin[isl + 1];
-        if (end - begin > kRevTiny) continue;
-        const uint32_t nb = s.isl_nbod[isl];
-        const int32_t* ib = s.isl_bod + begin + isl;
-        for (uint32_t l = 0; l < nb; ++l) {
-            const int32_t g = ib[l];
-            my[4 * l] = s.sb_dv[g]; my[4 * l + 1] = s.sb_dw[g];
-            my[4 * l + 2] = A.dv[g]; my[4 * l + 3] = A.dw[g];
+    const RevLocal D{sh[wib]};
+    uint32_t units[DevState::kSmallClasses], total = 0;   // warps' worth of islands per class
+#pragma unroll
+    for (int c = 0; c < DevState::kSmallClasses; ++c) {
+        units[c] = (s.counters[list_counter(DevState::kSmallList + c)] + (32u >> c) - 1u) >> (5 - c);
+        total += units[c];
+    }
+    for (uint32_t u = blockIdx.x * kRevWarps + wib; u < total; u += gridDim.x * kRevWarps) {
+        uint32_t at = u, c = 0;
+#pragma unroll
+        for (int k = DevState::kSmallClasses - 1; k >= 0; --k) {   // the longest chains first
+            c = uint32_t(k);
+            if (at < units[k]) break;
+            at -= units[k];
         }
+        const uint32_t g = 1u << c, sub = lane >> c, i = lane & (g - 1u), e = (at << (5 - c)) + sub;
+        uint32_t begin = 0, n = 0, nlev = 0, nb = 0, isl = 0;
+        if (e < s.counters[list_counter(DevState::kSmallList + int(c))]) {
+            isl = s.isl_list[DevState::kSmallList + c][e];
+            begin = s.isl_begin[isl];
+            n = s.isl_begin[isl + 1] - begin;
+            nlev = s.isl_end[isl];
+            nb = s.isl_nbod[isl];
+        }
+        const int32_t* ib = s.isl_bod + begin + isl;
+        float4* my = sh[wib] + 4 * (sub * 2u * g);   // g + 1 bodies at most
+        for (uint32_t l = i; l < nb; l += g) {
+            const int32_t b = ib[l];
+            my[4 * l] = s.sb_dv[b]; my[4 * l + 1] = s.sb_dw[b];
+            my[4 * l + 2] = A.dv[b]; my[4 * l + 3] = A.dw[b];
+        }
+        uint32_t d = 0, lid = 0;
+        int level = -1;
+        if (i < n) {
+            d = s.d_val2[begin + i];
+            const uint32_t w = s.d_lbod[begin + i], base = sub * 2u * g;
+            lid = ((w & 0xffffu) == 0xffffu ? 0xffffu : base + (w & 0xffffu)) |
+                  ((w >> 16) == 0xffffu ? 0xffff0000u : (base + (w >> 16)) << 16);
+            const uint32_t* bound = lvl_bound + begin + isl;
+            level = 0;
+            while (uint32_t(level) + 1u < nlev && bound[level + 1] <= begin + i) ++level;
+        }
+        const int levels = int(__reduce_max_sync(0xffffffffu, nlev));
+        __syncwarp();
         for (int it = pos + vel - 1; it >= 0; --it) {
-            if (it == pos - 1)
-                for (uint32_t l = 0; l < nb; ++l) {
-                    const int32_t g = ib[l];
+            if (it == pos - 1) {
+                for (uint32_t l = i; l < nb; l += g) {
+                    const int32_t b = ib[l];
                     float4 v = my[4 * l + 2], w = my[4 * l + 3];
-                    const float4 mv = A.dvm[g], mw = A.dwm[g];
+                    const float4 mv = A.dvm[b], mw = A.dwm[b];
                     v.x += mv.x; v.y += mv.y; v.z += mv.z;
                     w.x += mw.x; w.y += mw.y; w.z += mw.z;
                     my[4 * l + 2] = v; my[4 * l + 3] = w;
                 }
-            for (uint32_t i = end; i-- > begin;) reverse_desc(s, A, s.d_val2[i], s.d_lbod[i], it, pos, D);
+                __syncwarp();
+            }
+            for (int l = levels - 1; l >= 0; --l) {
+                if (level == l) reverse_desc(s, A, d, lid, it, pos, D);
+                __syncwarp();
+            }
         }
+        __syncwarp();
     }
 }
 
-constexpr uint32_t kRevWarps = 4;
+// One warp per island of (kRevSmall, isl_warp] descriptors.
 __global__ void __launch_bounds__(kRevWarps * 32) k_adj_pgs_warp_smem(DevState s, AdjState A,
                                                                      const uint32_t* lvl_bound) {
     __shared__ float4 sh[kRevWarps][4 * (kSmallIsland + 1)];
@@ -511,7 +549,7 @@ __global__ void __launch_bounds__(kRevWarps * 32) k_adj_pgs_warp_smem(DevState s
     const RevLocal D{sh[wib]};
     for (uint32_t isl = warp; isl < ni; isl += nwarps) {
         const uint32_t begin = s.isl_begin[isl], end = s.isl_begin[isl + 1];
-        if (end - begin > s.isl_warp || end - begin <= kRevTiny) continue;
+        if (end - begin > s.isl_warp || end - begin <= kRevSmall) continue;
         const uint32_t nlev = s.isl_end[isl];
         const uint32_t nb = s.isl_nbod[isl];
         const int32_t* ib = s.isl_bod + begin + isl;
@@ -1012,7 +1050,7 @@ void enqueue_adjoint_step(const DevState& s, const AdjState& a, cudaStream_t st,
     auto side = [&](int i) { return br ? br->st[i] : st; };
     k_adj_pgs_warp_smem<<<grid_n(s.desc_cap * 32u, kRevWarps * 32u, 148u * 8u), kRevWarps * 32u, 0, st>>>(
         s, a, s.lvl_bound);
-    k_adj_pgs_thread<<<grid_n(s.desc_cap, kRevThreadBlock, 148u * 16u), kRevThreadBlock, 0, side(0)>>>(s, a);
+    k_adj_pgs_packed<<<grid_n(s.desc_cap, kRevWarps, 148u * 4u), kRevWarps * 32u, 0, side(0)>>>(s, a, s.lvl_bound);
     k_adj_pgs_mid_smem<<<grid_n(s.desc_cap, kSmallIsland + 1, 148u * 4u), 128,
                          4 * (kMidIsland + 1) * sizeof(float4), side(1)>>>(s, a, s.lvl_bound);
     k_adj_pgs_block<<<grid_n(s.desc_cap, 1, 148u * 4u), 256, 0, side(2)>>>(s, a, s.lvl_bound);

@@ -1146,7 +1146,7 @@ __global__ void k_prep_joints(DevState s) {
     }
 }
 
-__global__ void k_prep_contacts(DevState s) {
+__global__ void __launch_bounds__(128, 4) k_prep_contacts(DevState s) {
     const uint32_t nm = s.counters[kCntMan];
     const uint32_t frame = s.counters[kCntFrame];
     const float inv_dt = 1.0f / s.dt;
