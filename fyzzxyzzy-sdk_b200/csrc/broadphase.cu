@@ -455,7 +455,7 @@ __device__ __forceinline__ int32_t find_key(const uint64_t* keys, uint32_t lo, u
 __global__ void k_owner_init(DevState s) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i == 0) {
-        for (int c : {int(kCntGjk), int(kCntConvex), int(kCntConvexGjk), int(kCntConvexClip), int(kCntConvexEpa)})
+        for (int c : {int(kCntRegen), int(kCntGjk), int(kCntConvex), int(kCntConvexGjk), int(kCntConvexClip), int(kCntConvexEpa)})
             s.counters[c] = 0u;
     }
     if (i >= s.n_shapes) return;

@@ -932,8 +932,8 @@ __device__ int emit_box_box(qt q1, v3 p1, float cd, const PcmCache& cache, bool 
 // Returns the emitted count, or -1 on an invalid manifold normal / overflow.
 // Sets gjk_pending (and emits nothing) when the zero-face GJK/EPA
 // continuation must complete the manifold.
-__device__ int generate_box_box(v3 h0, v3 p0, qt q0, v3 h1, v3 p1, qt q1, float cd, PcmCache& cache,
-                                ContactPt* out, bool& gjk_pending) {
+// Box/box: refreshes the cached manifold; true when it has to be regenerated.
+__device__ bool box_box_stale(v3 h0, v3 p0, qt q0, v3 h1, v3 p1, qt q1, PcmCache& cache) {
     const v3 delta = {p0.x - p1.x, p0.y - p1.y, p0.z - p1.z};
     const v3 relative = rotinv_sc(q1, delta);
     const qt rotation = qmul(qconj(q1), q0);
@@ -959,41 +959,41 @@ __device__ int generate_box_box(v3 h0, v3 p0, qt q0, v3 h1, v3 p1, qt q1, float 
         regen = a0 * sqrtf(h0.x * h0.x + h0.y * h0.y + h0.z * h0.z) > tp ||
                 a1 * sqrtf(h1.x * h1.x + h1.y * h1.y + h1.z * h1.z) > tp;
     }
-    bool direct = false;
-    const bool gjk = false;
-    const v3 gjk_n = {0, 0, 0};
-    if (regen) {
-        sv(cache.rel_p, relative);
-        cache.rel_q[0] = rotation.x; cache.rel_q[1] = rotation.y; cache.rel_q[2] = rotation.z; cache.rel_q[3] = rotation.w;
-        cache.qa[0] = q0.x; cache.qa[1] = q0.y; cache.qa[2] = q0.z; cache.qa[3] = q0.w;
-        cache.qb[0] = q1.x; cache.qb[1] = q1.y; cache.qb[2] = q1.z; cache.qb[3] = q1.w;
-        set_meta(cache, cache_count(cache), true);
-        Cand cands[kMaxBoxCandidates];
-        int count = 0;
-        const int ov = box_box_candidates(h0, p0, q0, h1, p1, q1, cd, cands, count);
-        if (ov < 0) return -1;
-        if (ov == 0) {
-            set_meta(cache, 0, true);
-            return 0;
-        }
-        if (count == 0) {
-            // Zero face contacts: the GJK/EPA continuation runs in its own
-            // kernel (k_narrowphase_gjk) over the pairs that need it, so its
-            // polytope working set stays out of this kernel.
-            gjk_pending = true;
-            return 0;
-        } else if (count <= 4) {
-            for (int i = 0; i < count; ++i) cache.pts[i] = to_pt(cands[i]);
-            set_meta(cache, uint32_t(count), true);
-        } else {
-            int sel[4];
-            batch_selection(cands, count, 1.0f, sel);
-            for (int i = 0; i < 4; ++i) cache.pts[i] = to_pt(cands[sel[i]]);
-            set_meta(cache, 4, true);
-        }
-        direct = count > 0;
+    return regen;
+}
+// A stale box/box manifold from the face candidates.
+enum : int { kBoxOverflow = -1, kBoxNone = 0, kBoxFaces = 1, kBoxGjk = 2 };
+__device__ int regenerate_box_box(v3 h0, v3 p0, qt q0, v3 h1, v3 p1, qt q1, float cd, PcmCache& cache) {
+    const v3 relative = rotinv_sc(q1, {p0.x - p1.x, p0.y - p1.y, p0.z - p1.z});
+    const qt rotation = qmul(qconj(q1), q0);
+    sv(cache.rel_p, relative);
+    cache.rel_q[0] = rotation.x; cache.rel_q[1] = rotation.y; cache.rel_q[2] = rotation.z; cache.rel_q[3] = rotation.w;
+    cache.qa[0] = q0.x; cache.qa[1] = q0.y; cache.qa[2] = q0.z; cache.qa[3] = q0.w;
+    cache.qb[0] = q1.x; cache.qb[1] = q1.y; cache.qb[2] = q1.z; cache.qb[3] = q1.w;
+    set_meta(cache, cache_count(cache), true);
+    Cand cands[kMaxBoxCandidates];
+    int count = 0;
+    const int ov = box_box_candidates(h0, p0, q0, h1, p1, q1, cd, cands, count);
+    if (ov < 0) return kBoxOverflow;
+    if (ov == 0) {
+        set_meta(cache, 0, true);
+        return kBoxNone;
     }
-    return emit_box_box(q1, p1, cd, cache, direct, gjk, gjk_n, out);
+    if (count == 0) {
+        // Zero face contacts: the GJK/EPA continuation runs in its own
+        // kernel (k_narrowphase_gjk) over the pairs that need it, so its
+        // polytope working set stays out of this kernel.
+        return kBoxGjk;
+    } else if (count <= 4) {
+        for (int i = 0; i < count; ++i) cache.pts[i] = to_pt(cands[i]);
+        set_meta(cache, uint32_t(count), true);
+    } else {
+        int sel[4];
+        batch_selection(cands, count, 1.0f, sel);
+        for (int i = 0; i < 4; ++i) cache.pts[i] = to_pt(cands[sel[i]]);
+        set_meta(cache, 4, true);
+    }
+    return kBoxFaces;
 }
 
 // Second half of the zero-face case (scene.cpp:3545-3590): GJK/EPA witness,
@@ -1058,7 +1058,8 @@ __device__ int emit_box_box(qt q1, v3 p1, float cd, const PcmCache& cache, bool 
     return emitted;
 }
 
-__device__ int generate_plane_box(v3 pp, v3 h, v3 bp, qt q, float cd, PcmCache& cache, ContactPt* out) {
+// Plane/box: refreshes the cached manifold; true when it has to be regenerated.
+__device__ bool plane_box_stale(v3 pp, v3 h, v3 bp, qt q, PcmCache& cache) {
     const v3 rel = {bp.x - pp.x, bp.y - pp.y, bp.z - pp.z};
     const float margin = pcm_box_margin(h);
     const float brk = margin * 0.2f;
@@ -1069,83 +1070,86 @@ __device__ int generate_plane_box(v3 pp, v3 h, v3 bp, qt q, float cd, PcmCache& 
     if (init)
         md = smax(smax(fabsf(rel.x - cache.rel_p[0]), fabsf(rel.y - cache.rel_p[1])), fabsf(rel.z - cache.rel_p[2]));
     const float rd = q.x * cache.rel_q[0] + q.y * cache.rel_q[1] + q.z * cache.rel_q[2] + q.w * cache.rel_q[3];
-    const bool regen = !init || cache_count(cache) != prev || md > brk || rd < 0.99996f;
-    if (regen) {
-        sv(cache.rel_p, rel);
-        cache.rel_q[0] = q.x; cache.rel_q[1] = q.y; cache.rel_q[2] = q.z; cache.rel_q[3] = q.w;
-        Cand cands[8];
-        int n = 0;
-        for (unsigned corner = 0; corner < 8u; ++corner) {
-            const v3 local = {(corner & 4u) ? -h.x : h.x, (corner & 2u) ? -h.y : h.y, (corner & 1u) ? -h.z : h.z};
-            const v3 r = rot_sc(q, local);
-            const v3 ip = {rel.x + r.x, rel.y + r.y, rel.z + r.z};
-            if (ip.y >= cd) continue;
-            cands[n++] = {local, {ip.x, 0.0f, ip.z}, {0.0f, 1.0f, 0.0f}, ip.y};
+    return !init || cache_count(cache) != prev || md > brk || rd < 0.99996f;
+}
+__device__ void regenerate_plane_box(v3 pp, v3 h, v3 bp, qt q, float cd, PcmCache& cache) {
+    const v3 rel = {bp.x - pp.x, bp.y - pp.y, bp.z - pp.z};
+    sv(cache.rel_p, rel);
+    cache.rel_q[0] = q.x; cache.rel_q[1] = q.y; cache.rel_q[2] = q.z; cache.rel_q[3] = q.w;
+    Cand cands[8];
+    int n = 0;
+    for (unsigned corner = 0; corner < 8u; ++corner) {
+        const v3 local = {(corner & 4u) ? -h.x : h.x, (corner & 2u) ? -h.y : h.y, (corner & 1u) ? -h.z : h.z};
+        const v3 r = rot_sc(q, local);
+        const v3 ip = {rel.x + r.x, rel.y + r.y, rel.z + r.z};
+        if (ip.y >= cd) continue;
+        cands[n++] = {local, {ip.x, 0.0f, ip.z}, {0.0f, 1.0f, 0.0f}, ip.y};
+    }
+    if (n <= 4) {
+        for (int i = 0; i < n; ++i) cache.pts[i] = to_pt(cands[i]);
+        set_meta(cache, uint32_t(n), true);
+    } else {
+        bool chosen[8] = {false, false, false, false, false, false, false, false};
+        int idx[4];
+        int first = 0;
+        for (int i = 1; i < n; ++i)
+            if (cands[i].sep < cands[first].sep) first = i;
+        idx[0] = first;
+        chosen[first] = true;
+        int far = 0;
+        float maxd = vlen2(vsub(cands[0].lb, cands[first].lb));
+        for (int i = 1; i < n; ++i) {
+            const float d = vlen2(vsub(cands[i].lb, cands[first].lb));
+            if (d > maxd) { maxd = d; far = i; }
         }
-        if (n <= 4) {
-            for (int i = 0; i < n; ++i) cache.pts[i] = to_pt(cands[i]);
-            set_meta(cache, uint32_t(n), true);
+        idx[1] = far;
+        chosen[far] = true;
+        const v3 seg = vsub(cands[far].lb, cands[first].lb);
+        v3 side = {-seg.z, 0.0f, seg.x};
+        const float ns = vlen2(side);
+        if (ns > 0.0f) {
+            const float inv = 1.0f / sqrtf(ns);
+            side = {side.x * inv, 0.0f, side.z * inv};
         } else {
-            bool chosen[8] = {false, false, false, false, false, false, false, false};
-            int idx[4];
-            int first = 0;
-            for (int i = 1; i < n; ++i)
-                if (cands[i].sep < cands[first].sep) first = i;
-            idx[0] = first;
-            chosen[first] = true;
-            int far = 0;
-            float maxd = vlen2(vsub(cands[0].lb, cands[first].lb));
-            for (int i = 1; i < n; ++i) {
-                const float d = vlen2(vsub(cands[i].lb, cands[first].lb));
-                if (d > maxd) { maxd = d; far = i; }
-            }
-            idx[1] = far;
-            chosen[far] = true;
-            const v3 seg = vsub(cands[far].lb, cands[first].lb);
-            v3 side = {-seg.z, 0.0f, seg.x};
-            const float ns = vlen2(side);
-            if (ns > 0.0f) {
-                const float inv = 1.0f / sqrtf(ns);
-                side = {side.x * inv, 0.0f, side.z * inv};
-            } else {
-                side = {0.0f, 1.0f, 0.0f};
-            }
-            float largest = -FLT_MAX, smallest = FLT_MAX;
-            int third = 0, fourth = 0;
+            side = {0.0f, 1.0f, 0.0f};
+        }
+        float largest = -FLT_MAX, smallest = FLT_MAX;
+        int third = 0, fourth = 0;
+        for (int i = 0; i < n; ++i) {
+            if (chosen[i]) continue;
+            const float d = vdot(vsub(cands[i].lb, cands[first].lb), side);
+            if (d > largest) { largest = d; third = i; }
+            if (d < smallest) { smallest = d; fourth = i; }
+        }
+        idx[2] = third;
+        chosen[third] = true;
+        if (smallest * largest > 0.0f) {
+            largest = -FLT_MAX;
             for (int i = 0; i < n; ++i) {
                 if (chosen[i]) continue;
                 const float d = vdot(vsub(cands[i].lb, cands[first].lb), side);
-                if (d > largest) { largest = d; third = i; }
-                if (d < smallest) { smallest = d; fourth = i; }
+                if (d > largest) { largest = d; fourth = i; }
             }
-            idx[2] = third;
-            chosen[third] = true;
-            if (smallest * largest > 0.0f) {
-                largest = -FLT_MAX;
-                for (int i = 0; i < n; ++i) {
-                    if (chosen[i]) continue;
-                    const float d = vdot(vsub(cands[i].lb, cands[first].lb), side);
-                    if (d > largest) { largest = d; fourth = i; }
-                }
-            }
-            idx[3] = fourth;
-            chosen[fourth] = true;
-            Cand centers[4];
-            for (int k = 0; k < 4; ++k) centers[k] = cands[idx[k]];
-            for (int i = 0; i < n; ++i) {
-                if (chosen[i]) continue;
-                float nearest = FLT_MAX;
-                int slot = 0;
-                for (int j = 0; j < 4; ++j) {
-                    const float d = vlen2(vsub(cands[i].lb, centers[j].lb));
-                    if (d < nearest) { nearest = d; slot = j; }
-                }
-                if (cands[i].sep < cands[idx[slot]].sep) idx[slot] = i;
-            }
-            for (int k = 0; k < 4; ++k) cache.pts[k] = to_pt(cands[idx[k]]);
-            set_meta(cache, 4, true);
         }
+        idx[3] = fourth;
+        chosen[fourth] = true;
+        Cand centers[4];
+        for (int k = 0; k < 4; ++k) centers[k] = cands[idx[k]];
+        for (int i = 0; i < n; ++i) {
+            if (chosen[i]) continue;
+            float nearest = FLT_MAX;
+            int slot = 0;
+            for (int j = 0; j < 4; ++j) {
+                const float d = vlen2(vsub(cands[i].lb, centers[j].lb));
+                if (d < nearest) { nearest = d; slot = j; }
+            }
+            if (cands[i].sep < cands[idx[slot]].sep) idx[slot] = i;
+        }
+        for (int k = 0; k < 4; ++k) cache.pts[k] = to_pt(cands[idx[k]]);
+        set_meta(cache, 4, true);
     }
+}
+__device__ int emit_plane_box(v3 pp, float cd, const PcmCache& cache, ContactPt* out) {
     int emitted = 0;
     const uint32_t n = cache_count(cache);
     for (uint32_t k = 0; k < n; ++k) {
@@ -1242,6 +1246,39 @@ __device__ __forceinline__ PairShapes pair_shapes(const DevState& s, uint64_t ke
     return p;
 }
 
+// Box and plane pairs whose cached manifold went stale (kSplit; tmp_flags is
+// free until the step's events).
+__device__ __forceinline__ uint32_t* regen_list(const DevState& s) { return s.tmp_flags; }
+// A stale pair's manifold; whether it has contacts to emit (box/box pairs
+// without face contact go on to k_narrowphase_gjk).
+__device__ __forceinline__ bool regenerate(const DevState& s, uint32_t k, const PairShapes& ps, v3 h0, v3 h1, v3 p0,
+                                           v3 p1, qt q0, qt q1, PcmCache& cache) {
+    if (ps.plane) {
+        regenerate_plane_box(p0, h1, p1, q1, ps.cd, cache);
+        return true;
+    }
+    const int r = regenerate_box_box(h0, p0, q0, h1, p1, q1, ps.cd, cache);
+    if (r == kBoxGjk) s.gjk_list[atomicAdd(&s.counters[kCntGjk], 1u)] = k;
+    if (r == kBoxOverflow) atomicOr(s.err, kErrContactOverflow);
+    return r == kBoxFaces;
+}
+__device__ __forceinline__ int emit_box_pair(const PairShapes& ps, v3 p0, v3 p1, qt q1, const PcmCache& cache,
+                                             bool fresh, ContactPt* out) {
+    return ps.plane ? emit_plane_box(p0, ps.cd, cache, out)
+                    : emit_box_box(q1, p1, ps.cd, cache, fresh, false, {0, 0, 0}, out);
+}
+
+// One thread a pair: sphere pairs, the refresh of box manifolds, and (kSplit
+// false) the regeneration of stale ones.  kSplit lists those instead for
+// k_narrowphase_regen: in one kernel the clipping of a few pairs holds up
+// nearly every warp (11 of 32 lanes active).  That pays where the pairs fill
+// the device many times over -- 1.3 million pairs 866 against 350 + 270 us,
+// 380,000 pairs 187 against 116 + 28 us -- while a small world only gets a
+// second kernel as long as one regeneration: 57,000 pairs 44 against 49 us,
+// 200 pairs 16 against 22 us.  The line is drawn by the pair budget, which
+// the host knows (kSplitPairs, about three live pairs a budgeted ten).
+constexpr uint32_t kSplitPairs = 1u << 20;
+template <bool kSplit>
 __global__ void __launch_bounds__(128) k_narrowphase(DevState s) {
     const uint32_t n = *s.cur.n;
     const uint32_t stride = gridDim.x * blockDim.x;
@@ -1268,13 +1305,13 @@ __global__ void __launch_bounds__(128) k_narrowphase(DevState s) {
         const v3 p0 = ld3(s.s_wp[first]), p1 = ld3(s.s_wp[second]);
         const qt q0 = ldq(s.s_wq[first]), q1 = ldq(s.s_wq[second]);
         const float4 g0 = s.s_geom[first], g1 = s.s_geom[second];
-        if (plane && !sphere) {
-            count = generate_plane_box(p0, {g1.x, g1.y, g1.z}, p1, q1, cd, cache, out);
-        } else if (!plane && !sphere) {
-            bool gjk_pending = false;
-            count = generate_box_box({g0.x, g0.y, g0.z}, p0, q0, {g1.x, g1.y, g1.z}, p1, q1, cd, cache, out,
-                                     gjk_pending);
-            if (gjk_pending) s.gjk_list[atomicAdd(&s.counters[kCntGjk], 1u)] = k;
+        bool stale = false;
+        if (!sphere) {
+            const v3 h0 = {g0.x, g0.y, g0.z}, h1 = {g1.x, g1.y, g1.z};
+            stale = plane ? plane_box_stale(p0, h1, p1, q1, cache) : box_box_stale(h0, p0, q0, h1, p1, q1, cache);
+            bool emit = !stale;
+            if (!kSplit && stale) emit = regenerate(s, k, ps, h0, h1, p0, p1, q0, q1, cache);
+            if (emit) count = emit_box_pair(ps, p0, p1, q1, cache, stale, out);
         } else {
             const uint32_t sp = ta == kSphere ? sa : sb;
             const v3 c = ld3(s.s_wp[sp]);
@@ -1292,15 +1329,35 @@ __global__ void __launch_bounds__(128) k_narrowphase(DevState s) {
                 }
             }
         }
-        if (count < 0) {
-            atomicOr(s.err, kErrContactOverflow);
-            count = 0;
-        }
         if (pcm) s.cur.cache[k] = cache;
+        if (kSplit && stale) {
+            regen_list(s)[atomicAdd(&s.counters[kCntRegen], 1u)] = k;
+            continue;
+        }
         s.cur.count[k] = uint32_t(count);
         for (int i = 0; i < count; ++i) s.pts[4 * size_t(k) + i] = out[i];
         // friction histories are not carried here: row preparation reads a
         // touching manager's history from the previous generation
+    }
+}
+
+// The listed stale pairs, one thread each.
+__global__ void __launch_bounds__(128) k_narrowphase_regen(DevState s) {
+    const uint32_t n = s.counters[kCntRegen];
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint32_t k = regen_list(s)[i];
+        const PairShapes ps = pair_shapes(s, s.cur.key[k]);
+        const v3 p0 = ld3(s.s_wp[ps.first]), p1 = ld3(s.s_wp[ps.second]);
+        const qt q0 = ldq(s.s_wq[ps.first]), q1 = ldq(s.s_wq[ps.second]);
+        const float4 g0 = s.s_geom[ps.first], g1 = s.s_geom[ps.second];
+        PcmCache cache = s.cur.cache[k];
+        ContactPt out[4];
+        int count = 0;
+        if (regenerate(s, k, ps, {g0.x, g0.y, g0.z}, {g1.x, g1.y, g1.z}, p0, p1, q0, q1, cache))
+            count = emit_box_pair(ps, p0, p1, q1, cache, true, out);
+        s.cur.cache[k] = cache;
+        s.cur.count[k] = uint32_t(count);
+        for (int j = 0; j < count; ++j) s.pts[4 * size_t(k) + j] = out[j];
     }
 }
 
@@ -2087,7 +2144,13 @@ void enqueue_narrowphase(const DevState& s, cudaStream_t st, const StageHook& ho
     const int T = 128;
     hook(kStNarrow, st);
     const uint32_t blocks = (s.pair_cap + T - 1) / T;
-    k_narrowphase<<<blocks < 148u * 16u ? blocks : 148u * 16u, T, 0, st>>>(s);
+    const uint32_t grid = blocks < 148u * 16u ? blocks : 148u * 16u;
+    if (s.pair_cap >= kSplitPairs) {
+        k_narrowphase<true><<<grid, T, 0, st>>>(s);
+        k_narrowphase_regen<<<grid, T, 0, st>>>(s);
+    } else {
+        k_narrowphase<false><<<grid, T, 0, st>>>(s);
+    }
     const uint32_t gb = (s.pair_cap + kGjkWarps - 1) / kGjkWarps;
     k_narrowphase_gjk<<<gb < 148u * 8u ? gb : 148u * 8u, kGjkWarps * 32, 0, st>>>(s);
     if (s.n_meshes) {

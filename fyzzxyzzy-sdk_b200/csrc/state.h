@@ -374,7 +374,7 @@ enum : int { kCntMan = 0, kCntDesc = 1, kCntIsl = 2, kCntFrame = 3, kCntLevels =
              kCntThCommon = 23 /* pairs exceeding in this step and the previous one */,
              kCntList4 = 24 /* lengths of island lists 4 .. kIslLists - 1 */,
              kCntQueue = kCntList4 + DevState::kIslLists - 4 /* work-queue ticket of the small islands' solver */,
-             kCntSlots = kCntQueue + 1 };
+             kCntRegen = kCntQueue + 1 /* stale box and plane manifolds */, kCntSlots = kCntRegen + 1 };
 // Counter slot of island list c.
 __host__ __device__ constexpr int list_counter(int c) { return c < 4 ? kCntList + c : kCntList4 + (c - 4); }
 // Each list holds islands of more than this many descriptors (its capacity
