@@ -17,12 +17,13 @@
 //
 // B200 mapping.  Descriptors are the distance joints (constraint slot
 // descending) followed by the touching managers in pair order.  A lock-free
-// union-find groups them into islands; a stable radix sort by island root
-// keeps each island's descriptors in that order, so the per-island greedy
+// union-find groups them into islands; a stable radix sort by each island's
+// smallest body keeps its descriptors in that order, so the per-island greedy
 // partition is exactly the reference's per-task greedy (islands share no
-// dynamic body).  PGS runs one warp (small islands) or one CTA (large
-// islands) per island, sweeping its partitions in order with warp / block
-// barriers only: no grid-wide synchronisation and no host round trip.
+// dynamic body).  PGS runs on one CTA per group of small islands, one CTA per
+// larger island or a cluster of CTAs per large one, sweeping the partitions in
+// order with block / cluster barriers only: no grid-wide synchronisation and
+// no host round trip.
 #include "solver_common.cuh"
 #include "lookback.cuh"
 #include <cfloat>
@@ -2037,12 +2038,13 @@ __global__ void __launch_bounds__(kGroupThreads, 4) k_pgs_group(DevState s) {
 // list).  An island has about ten levels, so a class's threads cover the
 // descriptors of a level; its records fill shared memory.
 template <class F> void for_island_solvers(F f) {
-    f(k_pgs_island<512, 128, 8>, 128u, 8u, Unit<512, 513, 128, 8>::kBytes, 9);
-    f(k_pgs_island<256, 64, 8>, 64u, 8u, Unit<256, 257, 64, 8>::kBytes, 8);
-    f(k_pgs_island<128, 32, 8>, 32u, 8u, Unit<128, 129, 32, 8>::kBytes, 7);
-    f(k_pgs_island<512, 128, 1>, 128u, 1u, Unit<512, 513, 128, 1>::kBytes, 6);
-    f(k_pgs_island<256, 64, 1>, 64u, 1u, Unit<256, 257, 64, 1>::kBytes, 5);
-    f(k_pgs_island<112, 64, 1>, 64u, 1u, Unit<112, 113, 64, 1>::kBytes, 4);
+    f(k_pgs_island<512, 128, 8>, 128u, 8u, Unit<512, 513, 128, 8>::kBytes, 10);
+    f(k_pgs_island<256, 64, 8>, 64u, 8u, Unit<256, 257, 64, 8>::kBytes, 9);
+    f(k_pgs_island<128, 32, 8>, 32u, 8u, Unit<128, 129, 32, 8>::kBytes, 8);
+    f(k_pgs_island<512, 128, 1>, 128u, 1u, Unit<512, 513, 128, 1>::kBytes, 7);
+    f(k_pgs_island<256, 64, 1>, 64u, 1u, Unit<256, 257, 64, 1>::kBytes, 6);
+    f(k_pgs_island<128, 64, 1>, 64u, 1u, Unit<128, 129, 64, 1>::kBytes, 5);
+    f(k_pgs_island<64, 64, 1>, 64u, 1u, Unit<64, 65, 64, 1>::kBytes, 4);
 }
 
 // One CTA per island beyond kBigIsland descriptors: deltas in global memory.

@@ -170,10 +170,10 @@ struct DevState {
     // Islands by size class (descriptors), listed each step by
     // k_island_classes: 0 (32, 512] shared-memory partition, 1 (isl_warp,
     // isl_mid] the rollout's 128-thread reverse sweep, 2 (512, 4096]
-    // shared-memory partition, 3 beyond 4096 global-memory paths, 4-9 the
+    // shared-memory partition, 3 beyond 4096 global-memory paths, 4-10 the
     // CTA and cluster solvers, kSmallList + c the small islands of
     // (2^(c-1), 2^c] descriptors (pgs_list).
-    static constexpr int kSmallList = 10, kSmallClasses = 6, kIslLists = kSmallList + kSmallClasses;
+    static constexpr int kSmallList = 11, kSmallClasses = 6, kIslLists = kSmallList + kSmallClasses;
     uint32_t* isl_list[kIslLists] = {};
 
     // step scratch
@@ -289,7 +289,7 @@ struct StageHook {
 // back into the main stream through events, so inside a stream capture they
 // become parallel branches of the step's graph.
 struct Branches {
-    static constexpr int kN = 6;
+    static constexpr int kN = 7;
     cudaStream_t st[kN] = {};
     cudaEvent_t fork = nullptr;
     cudaEvent_t join[kN] = {};
@@ -379,14 +379,14 @@ enum : int { kCntMan = 0, kCntDesc = 1, kCntIsl = 2, kCntFrame = 3, kCntLevels =
 __host__ __device__ constexpr int list_counter(int c) { return c < 4 ? kCntList + c : kCntList4 + (c - 4); }
 // Each list holds islands of more than this many descriptors (its capacity
 // is descriptors / (bound + 1) + 2).
-constexpr uint32_t kListMinDesc[DevState::kIslLists] = {32,  32,   512,  4096, 32, 112, 256, 512,
-                                                            1024, 2048, 0,    1,    2,  4,   8,   16};
+constexpr uint32_t kListMinDesc[DevState::kIslLists] = {32,  32,   512,  4096, 32, 64, 128, 256, 512,
+                                                            1024, 2048, 0,    1,    2,  4,  8,   16};
 // The solver list of an island of n descriptors (-1: beyond kBigIsland,
 // list 3 holds it).
 __host__ __device__ constexpr int pgs_list(uint32_t n) {
     if (n > kBigIsland) return -1;
-    if (n > 512u) return n <= 1024u ? 7 : n <= 2048u ? 8 : 9;
-    if (n > 32u) return n <= 112u ? 4 : n <= 256u ? 5 : 6;
+    if (n > 512u) return n <= 1024u ? 8 : n <= 2048u ? 9 : 10;
+    if (n > 32u) return n <= 64u ? 4 : n <= 128u ? 5 : n <= 256u ? 6 : 7;
     int c = 0;
     while ((1u << c) < n) ++c;
     return DevState::kSmallList + c;
