@@ -11,8 +11,8 @@
 //
 // The radix sort with 8-bit digits (the default) is a one-sweep LSD sort
 // (Adinets and Merrill, "Onesweep: A Faster Least Significant Digit Radix
-// Sort for GPUs", 2022), in 8- or 9-bit digits, whichever needs fewer
-// passes: one launch counts the digits of every pass at once, then
+// Sort for GPUs", 2022), in the narrowest of 8- to 10-bit digits with the
+// fewest passes: one launch counts the digits of every pass at once, then
 // each pass is one launch whose tiles (taken in ticket order) rank their
 // keys, publish their digit counts and find the counts of the tiles before
 // them by the same bounded, epoch-tagged look-back as the scan.  Other
@@ -208,14 +208,20 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_scatter(const uint32_t* 
     }
 }
 
-// ---- one-sweep passes (8- or 9-bit digits) ----
-// Scratch (zeroed when allocated): [0] epoch, [1] tile ticket, [2] finished
-// blocks, [3] pad, then kOsMaxPasses x 512 digit totals, then one 64-bit
-// state per tile and digit (512 a tile): epoch (30 bits) | status (2 bits:
-// 1 count of the tile, 2 inclusive count) | value (32 bits).
-constexpr int kOsMaxPasses = 4, kOsMaxDigits = 512;
-constexpr uint32_t kOsHeader = 4, kOsHist = kOsMaxPasses * kOsMaxDigits;
+// ---- one-sweep passes (8- to 10-bit digits) ----
+// Scratch (zeroed when allocated): [0] epoch, [1] finished blocks of a sort's
+// last pass, [2 + p] tile ticket of pass p, then kOsMaxPasses x 1024 digit
+// totals, then one 64-bit state per tile and digit (1024 a tile): epoch (30
+// bits) | status (2 bits: 1 count of the tile, 2 inclusive count) | value (32
+// bits).  Pass p of a sort runs under epoch + p.
+constexpr int kOsMaxPasses = 4, kOsMaxDigits = 1024;
+constexpr uint32_t kOsHeader = 8, kOsHist = kOsMaxPasses * kOsMaxDigits;
 constexpr int kOsLook = 8;   // predecessors read together in the look-back
+// A pass is latency from end to end (ticket, ranking rounds, look-back), so a
+// tile's 2,048 keys go to 16 warps of four rounds rather than 8 of eight.
+constexpr int kOsThreads = 512, kOsItems = 4, kOsWarps = kOsThreads / 32;
+static_assert(kOsThreads * kOsItems == kSortTile, "one tile size for every sort");
+template <int B> constexpr size_t os_smem() { return (size_t(kOsWarps) * ((1u << B) + 1u) + (1u << B)) * 4; }
 
 // Digit totals of every pass (ghist is zero between sorts).
 template <int B>
@@ -228,92 +234,97 @@ __global__ void __launch_bounds__(kSortThreads) k_os_hist(const uint32_t* __rest
     __syncthreads();
     const uint32_t lim = n_dev ? min(n, *n_dev) : n;
     for (uint32_t idx = blockIdx.x * kSortThreads + threadIdx.x; idx < lim; idx += gridDim.x * kSortThreads) {
-        const uint32_t k = keys[idx];
-        for (int p = 0; p < passes; ++p) atomicAdd(&h[p * R + ((k >> (begin_bit + B * p)) & (R - 1u))], 1u);
+        const uint32_t k = keys[idx] >> begin_bit;
+        for (int p = 0; p < passes; ++p) atomicAdd(&h[p * R + ((k >> (B * p)) & (R - 1u))], 1u);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < passes * int(R); i += kSortThreads)
         if (h[i]) atomicAdd(&ghist[i], h[i]);
 }
 
-// One pass: ranks a tile's keys by digit (stable), then places them at the
-// digit's global offset + the counts of the digit in earlier tiles + the
-// rank.  Thread t looks after digits t, t + 256, ...
+// Pass `pass` of `passes`: ranks a tile's keys by digit (stable), then places
+// them at the digit's global offset + the counts of the digit in earlier
+// tiles + the rank.  Thread t looks after digits t * DPT .. t * DPT + DPT - 1.
 template <int B>
-__global__ void __launch_bounds__(kSortThreads) k_os_scatter(const uint32_t* __restrict__ kin,
-                                                            const uint32_t* __restrict__ vin,
-                                                            uint32_t* __restrict__ kout,
-                                                            uint32_t* __restrict__ vout, uint32_t n,
-                                                            const uint32_t* n_dev, int shift,
-                                                            const uint32_t* __restrict__ ghist, uint32_t* ctl,
-                                                            unsigned long long* state, uint32_t* err,
-                                                            uint32_t* clear, uint32_t clear_n) {
-    constexpr uint32_t R = 1u << B, DPT = R / kSortThreads;   // digits a thread looks after
-    __shared__ uint32_t wcount[kSortWarps][R + 1];
-    __shared__ uint32_t wofs[kSortWarps][R + 1];
-    __shared__ uint32_t base_d[R];
-    __shared__ uint32_t sm_scan[kSortThreads / 32 + 1];
+__global__ void __launch_bounds__(kOsThreads, 2) k_os_scatter(const uint32_t* __restrict__ kin,
+                                                          const uint32_t* __restrict__ vin,
+                                                          uint32_t* __restrict__ kout, uint32_t* __restrict__ vout,
+                                                          uint32_t n, const uint32_t* n_dev, int shift, int pass,
+                                                          int passes, uint32_t* ghist, uint32_t* ctl,
+                                                          unsigned long long* state, uint32_t* err) {
+    constexpr uint32_t R = 1u << B, DPT = R > kOsThreads ? R / kOsThreads : 1u;
+    extern __shared__ uint32_t os_sm[];
+    uint32_t* wcount = os_sm;                          // kOsWarps x (R + 1): counts, then offsets inside the tile
+    uint32_t* base_d = os_sm + kOsWarps * (R + 1u);    // R
+    __shared__ uint32_t sm_scan[kOsThreads / 32 + 1];
     __shared__ uint32_t s_tile;
     // blocks beyond the live tiles leave before taking a ticket
     const uint32_t lim = n_dev ? min(n, *n_dev) : n;
     const uint32_t live = uint32_t((uint64_t(lim) + kSortTile - 1) / kSortTile);
     if (blockIdx.x >= live) return;
-    const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(&ctl[0]) & 0x3fffffffu;
+    const uint32_t epoch = (*reinterpret_cast<volatile uint32_t*>(&ctl[0]) + uint32_t(pass)) & 0x3fffffffu;
     const unsigned long long tag = (unsigned long long)epoch << 34;
-    if (threadIdx.x == 0) s_tile = atomicAdd(&ctl[1], 1u);
+    if (threadIdx.x == 0) s_tile = atomicAdd(&ctl[2 + pass], 1u);
+    for (uint32_t i = threadIdx.x; i < kOsWarps * (R + 1u); i += kOsThreads) wcount[i] = 0u;
     __syncthreads();
     const uint32_t tile = s_tile;
-    {
-        const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-        for (uint32_t i = threadIdx.x; i < kSortWarps * (R + 1); i += kSortThreads) (&wcount[0][0])[i] = 0u;
-        __syncthreads();
-        const uint32_t wbase = tile * kSortTile + warp * 32 * kSortItems;
-        uint32_t key[kSortItems], val[kSortItems], dig[kSortItems], rank[kSortItems];
-        const uint32_t lt = (1u << lane) - 1u;
-        uint32_t* wc = wcount[warp];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t wbase = tile * kSortTile + warp * 32 * kOsItems;
+    uint32_t key[kOsItems], val[kOsItems], dig[kOsItems], rank[kOsItems];
+    const uint32_t lt = (1u << lane) - 1u;
+    uint32_t* wc = wcount + warp * (R + 1u);
 #pragma unroll
-        for (int r = 0; r < kSortItems; ++r) {
-            const uint32_t idx = wbase + r * 32 + lane;
-            const bool valid = idx < lim;
-            key[r] = valid ? kin[idx] : 0u;
-            val[r] = valid ? vin[idx] : 0u;
-            dig[r] = valid ? ((key[r] >> shift) & (R - 1u)) : R;
-            const uint32_t peers = __match_any_sync(0xffffffffu, dig[r]);
-            const int leader = __ffs(peers) - 1;
-            const uint32_t base = wc[dig[r]];
-            __syncwarp();
-            if (lane == leader) wc[dig[r]] = base + __popc(peers);
-            __syncwarp();
-            rank[r] = base + __popc(peers & lt);
-        }
-        __syncthreads();
-        // thread t: digits t * DPT .. t * DPT + DPT - 1 (consecutive, so the
-        // block scan of their totals gives each its global offset)
-        uint32_t cnt[DPT], gtot = 0, gsum[DPT];
+    for (int r = 0; r < kOsItems; ++r) {
+        const uint32_t idx = wbase + r * 32 + lane;
+        const bool valid = idx < lim;
+        key[r] = valid ? kin[idx] : 0u;
+        val[r] = valid ? vin[idx] : 0u;
+        dig[r] = valid ? ((key[r] >> shift) & (R - 1u)) : R;
+    }
 #pragma unroll
-        for (uint32_t e = 0; e < DPT; ++e) {
-            const uint32_t d = threadIdx.x * DPT + e;
-            uint32_t c = 0;
-            for (int w = 0; w < kSortWarps; ++w) {
-                wofs[w][d] = c;
-                c += wcount[w][d];
+    for (int r = 0; r < kOsItems; ++r) {
+        const uint32_t peers = __match_any_sync(0xffffffffu, dig[r]);
+        const int leader = __ffs(peers) - 1;
+        const uint32_t base = wc[dig[r]];
+        __syncwarp();
+        if (lane == leader) wc[dig[r]] = base + __popc(peers);
+        __syncwarp();
+        rank[r] = base + __popc(peers & lt);
+    }
+    __syncthreads();
+    // this thread's digits (consecutive, so the block scan of their totals
+    // gives each its global offset): the warps' offsets and the tile's count
+    const uint32_t d0 = threadIdx.x * DPT;
+    const bool mine = d0 < R;
+    uint32_t cnt[DPT], gtot = 0, gsum[DPT];
+#pragma unroll
+    for (uint32_t e = 0; e < DPT; ++e) {
+        uint32_t c = 0;
+        if (mine) {
+            uint32_t w[kOsWarps];
+#pragma unroll
+            for (int k = 0; k < kOsWarps; ++k) w[k] = wcount[k * (R + 1u) + d0 + e];
+#pragma unroll
+            for (int k = 0; k < kOsWarps; ++k) {
+                wcount[k * (R + 1u) + d0 + e] = c;
+                c += w[k];
             }
-            cnt[e] = c;
-            gsum[e] = gtot;
-            gtot += ghist[d];
         }
-        uint32_t gx;
-        block_excl_scan<kSortThreads>(gtot, gx, sm_scan);
-        bool failed = false;
+        cnt[e] = c;
+        gsum[e] = gtot;
+        gtot += mine ? ghist[uint32_t(pass) * R + d0 + e] : 0u;
+    }
+    if (mine)
+#pragma unroll
+        for (uint32_t e = 0; e < DPT; ++e)
+            os_state_store(state + size_t(tile) * R + d0 + e, tag | ((tile == 0 ? 2ull : 1ull) << 32) | cnt[e]);
+    uint32_t gx;
+    block_excl_scan<kOsThreads>(gtot, gx, sm_scan);
+    bool failed = false;
+    if (mine)
 #pragma unroll
         for (uint32_t e = 0; e < DPT; ++e) {
-            const uint32_t d = threadIdx.x * DPT + e;
-            unsigned long long* my = state + size_t(tile) * R + d;
-            os_state_store(my, tag | ((tile == 0 ? 2ull : 1ull) << 32) | cnt[e]);
-        }
-#pragma unroll
-        for (uint32_t e = 0; e < DPT; ++e) {
-            const uint32_t d = threadIdx.x * DPT + e;
+            const uint32_t d = d0 + e;
             // look-back over kOsLook predecessors at a time (their loads in
             // flight together): sum tile counts until an inclusive count
             uint32_t prefix = 0;
@@ -339,40 +350,41 @@ __global__ void __launch_bounds__(kSortThreads) k_os_scatter(const uint32_t* __r
             if (tile != 0) os_state_store(state + size_t(tile) * R + d, tag | (2ull << 32) | (prefix + cnt[e]));
             base_d[d] = gx + gsum[e] + prefix;
         }
-        if (failed && err) atomicOr(err, kErrLogic);
-        __syncthreads();
-        // a look-back that gave up leaves the offsets unknown: the step
-        // reports the error and nothing lands outside the output
+    if (failed && err) atomicOr(err, kErrLogic);
+    __syncthreads();
+    // a look-back that gave up leaves the offsets unknown: the step
+    // reports the error and nothing lands outside the output
 #pragma unroll
-        for (int r = 0; r < kSortItems; ++r) {
-            if (dig[r] < R) {
-                const uint32_t pos = base_d[dig[r]] + wofs[warp][dig[r]] + rank[r];
-                if (pos < lim) {
-                    kout[pos] = key[r];
-                    vout[pos] = val[r];
-                } else if (err) {
-                    atomicOr(err, kErrLogic);
-                }
+    for (int r = 0; r < kOsItems; ++r) {
+        if (dig[r] < R) {
+            const uint32_t pos = base_d[dig[r]] + wc[dig[r]] + rank[r];
+            if (pos < lim) {
+                kout[pos] = key[r];
+                vout[pos] = val[r];
+            } else if (err) {
+                atomicOr(err, kErrLogic);
             }
         }
     }
-    // the last live block to finish opens the next epoch, resets the ticket
-    // and, in the sort's last pass, clears the digit totals for the next sort
-    // (a memset before every sort cost its chain about 6 us)
+    if (pass + 1 != passes) return;
+    // the last live block of the sort's last pass opens the next sort's
+    // epochs, resets the tickets and clears the digit totals (a memset before
+    // every sort cost its chain about 6 us, this fence and count in every
+    // pass about 1 us each)
     __shared__ bool last;
     if (threadIdx.x == 0) {
         __threadfence();
-        last = atomicAdd(&ctl[2], 1u) == live - 1;
+        last = atomicAdd(&ctl[1], 1u) == live - 1;
         if (last) {
             ctl[0] = (epoch + 1u) & 0x3fffffffu;
             ctl[1] = 0u;
-            ctl[2] = 0u;
+            for (int p = 0; p < passes; ++p) ctl[2 + p] = 0u;
             __threadfence();
         }
     }
     __syncthreads();
     if (last)
-        for (uint32_t i = threadIdx.x; i < clear_n; i += kSortThreads) clear[i] = 0u;
+        for (uint32_t i = threadIdx.x; i < uint32_t(passes) * R; i += kOsThreads) ghist[i] = 0u;
 }
 
 // The live entries of a sort that ended in the alternate buffers, copied
@@ -396,9 +408,8 @@ void onesweep_sort(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32_t*
                                                                          ghist);
     uint32_t *ki = keys, *vi = vals, *ko = keys_alt, *vo = vals_alt;
     for (int p = 0; p < passes; ++p) {
-        k_os_scatter<B><<<ntiles, kSortThreads, 0, st>>>(ki, vi, ko, vo, n_cap, n_dev, begin_bit + B * p,
-                                                          ghist + (1u << B) * p, os_scratch, state, err, ghist,
-                                                          p + 1 == passes ? uint32_t(passes) << B : 0u);
+        k_os_scatter<B><<<ntiles, kOsThreads, os_smem<B>(), st>>>(ki, vi, ko, vo, n_cap, n_dev, begin_bit + B * p, p,
+                                                                  passes, ghist, os_scratch, state, err);
         uint32_t* t = ki; ki = ko; ko = t;
         t = vi; vi = vo; vo = t;
     }
@@ -453,6 +464,7 @@ size_t radix_hist_words(uint32_t n_cap) {
 }
 
 void init_primitive_kernels() {
+    cudaFuncSetAttribute(k_os_scatter<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(os_smem<10>()));
     cudaFuncSetAttribute(k_radix_scatter<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(scatter_smem<10>()));
     cudaFuncSetAttribute(k_radix_scatter<11>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(scatter_smem<11>()));
 }
@@ -467,17 +479,21 @@ void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32
     const uint32_t ntiles = (n_cap + kSortTile - 1) / kSortTile;
     if (ntiles == 0) return;
     const int B = digit_bits >= 8 && digit_bits <= kRadixMaxBits ? digit_bits : 8;
-    // one-sweep passes: 8- or 9-bit digits, whichever needs fewer passes
+    // one-sweep passes: the narrowest of 8- to 10-bit digits with the fewest passes
     const int width = end_bit - begin_bit;
-    const int os_b = (width + 8) / 9 < (width + 7) / 8 ? 9 : 8;
+    int os_b = 8;
+    for (int b = 9; b <= 10; ++b)
+        if ((width + b - 1) / b < (width + os_b - 1) / os_b) os_b = b;
     const int os_passes = (width + os_b - 1) / os_b;
     if (B == 8 && os_scratch && os_passes <= kOsMaxPasses) {
         if (onesweep_words(n_cap) > os_words) {   // never: the world sizes the scratch for its largest sort
             if (err) cudaMemsetAsync(err, 0xff, 4, st);
             return;
         }
-        if (os_b == 9) onesweep_sort<9>(keys, vals, keys_alt, vals_alt, n_cap, n_dev, begin_bit, os_passes, ntiles,
-                                        os_scratch, st, err);
+        if (os_b == 10) onesweep_sort<10>(keys, vals, keys_alt, vals_alt, n_cap, n_dev, begin_bit, os_passes, ntiles,
+                                          os_scratch, st, err);
+        else if (os_b == 9) onesweep_sort<9>(keys, vals, keys_alt, vals_alt, n_cap, n_dev, begin_bit, os_passes,
+                                             ntiles, os_scratch, st, err);
         else onesweep_sort<8>(keys, vals, keys_alt, vals_alt, n_cap, n_dev, begin_bit, os_passes, ntiles,
                               os_scratch, st, err);
         return;
