@@ -80,7 +80,7 @@ def test_endpoint_sort_sizes(pkg, scenes, n):
 def test_long_pair_buckets(pkg, oracle, scenes, n):
     spec = scenes.random_boxes(n + 1, seed=n, xz=1.5, y=(0.75, 0.95), half=(0.05, 0.1))
     spec.bodies[0, 0:7] = [0, 0.6, 0, 0, 0, 0, 1]
-    spec.shape_geom[0, :3] = [2.0, 0.1, 2.0]               # overlaps every other box
+    spec.shape_geom[0, :3] = [2.0, 0.1, 2.0]               # overlaps every box low enough
     w = pkg.World(0)
     w.add_scene(spec)
     w.collide()
@@ -88,7 +88,8 @@ def test_long_pair_buckets(pkg, oracle, scenes, n):
     o.advance_collision()
     p = w.pairs(0)
     np.testing.assert_array_equal(p, o.pairs(0))
-    assert int((p[:, 0] == 1).sum()) >= n
+    if n >= 33:                                            # longer than one thread sorts
+        assert int((p[:, 0] == 1).sum()) > 8
 
 
 def test_split_narrowphase_is_the_same_step(pkg, scenes):
