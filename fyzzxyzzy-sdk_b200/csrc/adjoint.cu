@@ -1027,10 +1027,50 @@ __global__ void k_copy_set(ManagerSet dst, ManagerSet src, uint32_t cap) {
     if (blockIdx.x == 0 && threadIdx.x == 0) *dst.n = *src.n;
 }
 
+// Host-buffer transfers of a rollout, packed and unpacked on the device so
+// that each is one copy of the caller's own layout.
+__global__ void k_adj_seed(float4* dst, const float* src, uint32_t n) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b < n) dst[b] = make_float4(src[3 * size_t(b)], src[3 * size_t(b) + 1], src[3 * size_t(b) + 2], 0.0f);
+}
+// out: velocity and angular gradients (3 floats a body each), then the mass
+// gradients.  Inverse mass and inertia scale as 1 / m: dm = -im (im g_im +
+// iI . g_iI).
+__global__ void k_adj_results(DevState s, AdjState A, float* out) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= s.n_bodies) return;
+    const float4 v = A.v[b], w = A.w[b], gi = A.g_iI[b], inv = s.b_inv[b];
+    float* o = out + 3 * size_t(b);
+    o[0] = v.x; o[1] = v.y; o[2] = v.z;
+    o += 3 * size_t(s.n_bodies);
+    o[0] = w.x; o[1] = w.y; o[2] = w.z;
+    out[6 * size_t(s.n_bodies) + b] = -inv.w * (inv.w * A.g_im[b] + inv.x * gi.x + inv.y * gi.y + inv.z * gi.z);
+}
+__global__ void k_mass_frames(DevState s, float* out) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b >= s.n_bodies) return;
+    const v3 c = mass_position(s, b);
+    const qt q = mass_orientation(s, b);
+    float* o = out + 3 * size_t(b);
+    o[0] = c.x; o[1] = c.y; o[2] = c.z;
+    o = out + 3 * size_t(s.n_bodies) + 4 * size_t(b);
+    o[0] = q.x; o[1] = q.y; o[2] = q.z; o[3] = q.w;
+}
+
 }  // namespace
 
 void enqueue_adjoint_save_start(const DevState& s, const AdjState& a, cudaStream_t st) {
     k_adj_save_start<<<grid_n(s.n_bodies, 256, 1u << 30), 256, 0, st>>>(s, a);
+}
+
+void enqueue_adjoint_seed(float4* dst, const float* src, uint32_t n, cudaStream_t st) {
+    if (n) k_adj_seed<<<grid_n(n, 256, 1u << 30), 256, 0, st>>>(dst, src, n);
+}
+void enqueue_adjoint_results(const DevState& s, const AdjState& a, float* out, cudaStream_t st) {
+    if (s.n_bodies) k_adj_results<<<grid_n(s.n_bodies, 256, 1u << 30), 256, 0, st>>>(s, a, out);
+}
+void enqueue_mass_frames(const DevState& s, float* out, cudaStream_t st) {
+    if (s.n_bodies) k_mass_frames<<<grid_n(s.n_bodies, 256, 1u << 30), 256, 0, st>>>(s, out);
 }
 
 void enqueue_copy_set(const ManagerSet& dst, const ManagerSet& src, uint32_t cap, cudaStream_t st) {

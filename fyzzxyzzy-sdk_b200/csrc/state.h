@@ -328,6 +328,12 @@ struct AdjState {
 // Copies the live pairs of a contact-manager generation.
 void enqueue_copy_set(const ManagerSet& dst, const ManagerSet& src, uint32_t cap, cudaStream_t st);
 // adjoint.cu
+// Host-buffer transfers, in device memory: dst[b] = (src[3b .. 3b+2], 0);
+// out = velocity gradients, angular gradients (3 floats a body each) and mass
+// gradients (1); out = mass-frame centres (3 a body), then orientations (4).
+void enqueue_adjoint_seed(float4* dst, const float* src, uint32_t n, cudaStream_t st);
+void enqueue_adjoint_results(const DevState& s, const AdjState& a, float* out, cudaStream_t st);
+void enqueue_mass_frames(const DevState& s, float* out, cudaStream_t st);
 void enqueue_adjoint_save_start(const DevState& s, const AdjState& a, cudaStream_t st);
 void enqueue_adjoint_step(const DevState& s, const AdjState& a, cudaStream_t st, const Branches* br = nullptr);
 

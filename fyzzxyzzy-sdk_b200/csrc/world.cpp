@@ -1144,19 +1144,23 @@ public:
     void rollout_backward(const float* gc, const float* gq, const float* gv, const float* gw,
                           float* gv0, float* gw0, float* gmass, float* gfs, float* gfd) {
         if (!roll_done_) throw std::logic_error("rollout_forward must come first");
+        check_cuda(cudaSetDevice(device_), "cudaSetDevice");
         const uint32_t nb = d_.n_bodies, ns = d_.n_shapes;
+        float* stage = stage_buffer();
         auto up3 = [&](float4* dst, const float* src) {
-            std::vector<float4> h(nb, make_float4(0, 0, 0, 0));
-            if (src) for (uint32_t i = 0; i < nb; ++i) h[i] = make_float4(src[3 * i], src[3 * i + 1], src[3 * i + 2], 0);
-            upload(dst, h, stream_);
-            check_cuda(cudaStreamSynchronize(stream_), "sync");
+            if (!src) {
+                check_cuda(cudaMemsetAsync(dst, 0, size_t(nb) * 16, stream_), "memset");
+                return;
+            }
+            check_cuda(cudaMemcpyAsync(stage, src, size_t(nb) * 12, cudaMemcpyHostToDevice, stream_), "seed");
+            enqueue_adjoint_seed(dst, stage, nb, stream_);
         };
         up3(adj_.c, gc); up3(adj_.v, gv); up3(adj_.w, gw);
-        {
-            std::vector<float4> h(nb, make_float4(0, 0, 0, 0));
-            if (gq) for (uint32_t i = 0; i < nb; ++i) h[i] = make_float4(gq[4 * i], gq[4 * i + 1], gq[4 * i + 2], gq[4 * i + 3]);
-            upload(adj_.q, h, stream_);
-        }
+        if (gq) check_cuda(cudaMemcpyAsync(adj_.q, gq, size_t(nb) * 16, cudaMemcpyHostToDevice, stream_), "seed");
+        else check_cuda(cudaMemsetAsync(adj_.q, 0, size_t(nb) * 16, stream_), "memset");
+        // the caller's buffers are free again on return even if a copy is
+        // still under way when the sweeps are launched
+        check_cuda(cudaStreamSynchronize(stream_), "seed sync");
         check_cuda(cudaMemsetAsync(adj_.g_im, 0, nb * 4, stream_), "memset");
         check_cuda(cudaMemsetAsync(adj_.g_iI, 0, nb * 16, stream_), "memset");
         check_cuda(cudaMemsetAsync(adj_.g_fs, 0, ns * 4, stream_), "memset");
@@ -1171,19 +1175,13 @@ public:
         check_cuda(cudaStreamSynchronize(stream_), "backward sync");
         if (read_err()) throw std::overflow_error("Device error during the backward pass");
         // outputs
-        std::vector<float4> v(nb), w(nb), iI(nb), inv(nb);
-        std::vector<float> im(nb);
-        check_cuda(cudaMemcpy(v.data(), adj_.v, nb * 16, cudaMemcpyDeviceToHost), "read");
-        check_cuda(cudaMemcpy(w.data(), adj_.w, nb * 16, cudaMemcpyDeviceToHost), "read");
-        check_cuda(cudaMemcpy(iI.data(), adj_.g_iI, nb * 16, cudaMemcpyDeviceToHost), "read");
-        check_cuda(cudaMemcpy(im.data(), adj_.g_im, nb * 4, cudaMemcpyDeviceToHost), "read");
-        check_cuda(cudaMemcpy(inv.data(), d_.b_inv, nb * 16, cudaMemcpyDeviceToHost), "read");
-        for (uint32_t i = 0; i < nb; ++i) {
-            if (gv0) { gv0[3 * i] = v[i].x; gv0[3 * i + 1] = v[i].y; gv0[3 * i + 2] = v[i].z; }
-            if (gw0) { gw0[3 * i] = w[i].x; gw0[3 * i + 1] = w[i].y; gw0[3 * i + 2] = w[i].z; }
-            // inverse mass and inertia scale as 1/m: dm = -im (im g_im + iI . g_iI)
-            if (gmass) gmass[i] = -inv[i].w * (inv[i].w * im[i] + inv[i].x * iI[i].x + inv[i].y * iI[i].y + inv[i].z * iI[i].z);
-        }
+        enqueue_adjoint_results(d_, adj_, stage, stream_);
+        check_cuda(cudaGetLastError(), "results");
+        const size_t n = nb;
+        if (gv0) check_cuda(cudaMemcpyAsync(gv0, stage, n * 12, cudaMemcpyDeviceToHost, stream_), "read");
+        if (gw0) check_cuda(cudaMemcpyAsync(gw0, stage + 3 * n, n * 12, cudaMemcpyDeviceToHost, stream_), "read");
+        if (gmass) check_cuda(cudaMemcpyAsync(gmass, stage + 6 * n, n * 4, cudaMemcpyDeviceToHost, stream_), "read");
+        check_cuda(cudaStreamSynchronize(stream_), "read sync");
         if (gfs) check_cuda(cudaMemcpy(gfs, adj_.g_fs, ns * 4, cudaMemcpyDeviceToHost), "read");
         if (gfd) check_cuda(cudaMemcpy(gfd, adj_.g_fd, ns * 4, cudaMemcpyDeviceToHost), "read");
         // leave the world at the end of the rollout
@@ -1215,21 +1213,21 @@ public:
     }
     // Mass-frame centres and orientations of all bodies (loss inputs).
     void read_mass_frames(float* c3, float* q4) {
+        check_cuda(cudaSetDevice(device_), "cudaSetDevice");
         ensure_device();
         const uint32_t nb = d_.n_bodies;
-        std::vector<float4> p(nb), q(nb), mlp(nb), mlq(nb);
-        check_cuda(cudaStreamSynchronize(stream_), "sync");
-        check_cuda(cudaMemcpy(p.data(), d_.b_p, nb * 16, cudaMemcpyDeviceToHost), "read");
-        check_cuda(cudaMemcpy(q.data(), d_.b_q, nb * 16, cudaMemcpyDeviceToHost), "read");
-        check_cuda(cudaMemcpy(mlp.data(), d_.b_ml_p, nb * 16, cudaMemcpyDeviceToHost), "read");
-        check_cuda(cudaMemcpy(mlq.data(), d_.b_ml_q, nb * 16, cudaMemcpyDeviceToHost), "read");
-        for (uint32_t i = 0; i < nb; ++i) {
-            const qt bq = {q[i].x, q[i].y, q[i].z, q[i].w};
-            const v3 off = rot_sc(bq, {mlp[i].x, mlp[i].y, mlp[i].z});
-            const qt mq = qmul(bq, {mlq[i].x, mlq[i].y, mlq[i].z, mlq[i].w});
-            if (c3) { c3[3 * i] = p[i].x + off.x; c3[3 * i + 1] = p[i].y + off.y; c3[3 * i + 2] = p[i].z + off.z; }
-            if (q4) { q4[4 * i] = mq.x; q4[4 * i + 1] = mq.y; q4[4 * i + 2] = mq.z; q4[4 * i + 3] = mq.w; }
-        }
+        float* stage = stage_buffer();
+        enqueue_mass_frames(d_, stage, stream_);
+        check_cuda(cudaGetLastError(), "mass frames");
+        const size_t n = nb;
+        if (c3) check_cuda(cudaMemcpyAsync(c3, stage, n * 12, cudaMemcpyDeviceToHost, stream_), "read");
+        if (q4) check_cuda(cudaMemcpyAsync(q4, stage + 3 * n, n * 16, cudaMemcpyDeviceToHost, stream_), "read");
+        check_cuda(cudaStreamSynchronize(stream_), "read sync");
+    }
+    // Device staging of host-buffer transfers, 8 floats a body.
+    float* stage_buffer() {
+        if (!d_stage_) dalloc(d_stage_, 8 * std::max<size_t>(d_.n_bodies, 1), owned_);
+        return d_stage_;
     }
 
     // ---------------- contact events ----------------
@@ -1753,6 +1751,7 @@ private:
         replay_cap_ = replay_jcap_ = 0;
         replay_pending_ = false;
         d_pack_ = nullptr;
+        d_stage_ = nullptr;
         d_vel6_ = nullptr;
         vel_stride_cap_ = 0;
         for (void* p : pair_owned_) cudaFree(p);
@@ -2234,6 +2233,7 @@ private:
     float4 *bk_p_ = nullptr, *bk_q_ = nullptr, *bk_v_ = nullptr, *bk_w_ = nullptr, *bk_sacc_ = nullptr;
     float* bk_wake_ = nullptr;
     float* d_pack_ = nullptr;    // read_bodies records (owned, allocated on first use)
+    float* d_stage_ = nullptr;   // stage_buffer()
     float* d_vel6_ = nullptr;    // write_velocities records
     uint32_t vel_stride_cap_ = 0; // floats per record d_vel6_ holds
     uint32_t* bk_sleep_ = nullptr;
