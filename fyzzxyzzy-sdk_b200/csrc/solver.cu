@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kScanThreads) k_touch_compact(DevState s) {
 // linking", SODA 2014): trees then stay some log n deep.  Linking by the
 // index itself made chains of neighbours, about a hundred hops deep in a
 // 1,900-descriptor island, and the find that walked one set the length of the
-// key pass (32 us; 36 us on the 131,072-body pile).
+// key pass (32 us, 5 now; 36 us on the 131,072-body pile, 11 now).
 __device__ __forceinline__ uint32_t uf_rank(uint32_t x) { return x * 0x9E3779B1u; }   // odd factor: no two alike
 __device__ uint32_t uf_find(uint32_t* parent, uint32_t x) {
     uint32_t cur = parent[x];
@@ -826,7 +826,7 @@ template <uint32_t MAXN> struct PartSmem {
     static constexpr size_t kBytes = (2 * size_t(kTable) + 2 * size_t(MAXN)) * 4;
     // A round is a few dependent shared-memory accesses a descriptor: above
     // 512 descriptors, 256 threads took eight turns at them (61 us for an
-    // island of 1,923, 35 rounds).
+    // island of 1,923, 35 rounds; 29 us with 1,024).
     static constexpr uint32_t kThreads = MAXN > kMidIsland ? 1024u : 256u;
 };
 
@@ -2306,6 +2306,7 @@ void init_solver_kernels() {
     cudaFuncSetAttribute(k_pgs_group, cudaFuncAttributeMaxDynamicSharedMemorySize, int(GroupUnit::kBytes));
 }
 
+constexpr uint32_t kWidePrepPairs = 1u << 20;   // pair budget; see enqueue_solver's row preparation
 void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, const Branches* br) {
     uint32_t* lvl_bound = s.lvl_bound;
     const uint32_t T = s.elem_block;   // elementwise kernels (at most 56 registers, no launch bounds)
@@ -2330,6 +2331,18 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     }
     if (s.n_kinematic) k_kinematic_velocities<<<grid_for(s.n_bodies, T, 1u << 30), T, 0, st>>>(s);
     k_bodies_velocity<<<grid_for(s.n_bodies, T, 1u << 30), T, 0, st>>>(s);
+    // Row preparation needs the touching managers and the solver bodies, not
+    // the islands: it runs beside their sort and partition, which are latency
+    // and leave most of the device idle.  Contacts and joints one after the
+    // other beside the partitions only: 300 mechanisms 846 us for four steps
+    // against 778, 131,072-body pile 4,085 against 3,925, 4,096 scenes 8,870
+    // against 8,595.  Below the pair budget where preparation outlasts that
+    // chain it gets two CTAs an SM: at eight its registers keep the sort's
+    // CTAs waiting (32,768 hulls 1,826 us, with two 1,812).
+    const uint32_t prep_blocks = s.pair_cap >= kWidePrepPairs ? cap_blocks : 148u * 2u;
+    fork_branches(br, st, 2);
+    k_prep_contacts<<<grid_for(s.desc_cap, 128, prep_blocks), 128, 0, side(0)>>>(s);
+    if (s.n_joints) k_prep_joints<<<grid_for(s.n_joints, 128, 1u << 30), 128, 0, side(1)>>>(s);   // ~150 registers
     k_desc_keys<<<grid_for(s.desc_cap, T, cap_blocks), T, 0, st>>>(s);
     if (s.replay) {
         int rbits = 1;
@@ -2346,19 +2359,17 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
                      s.sort_hist, s.sort_hist_words, s.scan_tmp, s.scan_tmp_words, st, s.err, s.radix_bits, s.sort_os, s.sort_os_words);
     k_island_compact<<<lookback_grid(s.desc_cap), kScanThreads, 0, st>>>(s);
     k_island_classes<<<grid_for(s.desc_cap, T, cap_blocks), T, 0, st>>>(s);
-    // partitions by island size class, and row preparation: independent
+    // partitions by island size class: independent
     hook(kStPrep, st);
-    fork_branches(br, st, 3);
+    fork_branches(br, st, 4);
     launch(k_partition_smem<kBigIsland>, grid_for(s.desc_cap, kMidIsland + 1, 148u * 2u), PartSmem<kBigIsland>::kThreads,
-                PartSmem<kBigIsland>::kBytes, 1u, g_high_priority, side(1), s, lvl_bound, 2);
-    launch(k_partition_large, grid_for(s.desc_cap, kBigIsland + 1, 148u), 256u, size_t(0), 1u, g_high_priority, side(1), s,
+                PartSmem<kBigIsland>::kBytes, 1u, g_high_priority, side(2), s, lvl_bound, 2);
+    launch(k_partition_large, grid_for(s.desc_cap, kBigIsland + 1, 148u), 256u, size_t(0), 1u, g_high_priority, side(2), s,
                 lvl_bound);
     k_partition<<<grid_for(s.desc_cap, kPartWarps, 148u * 16u), kPartWarps * 32, 0, st>>>(s, lvl_bound);
     k_partition_smem<kMidIsland><<<grid_for(s.desc_cap, kSerialIsland + 1, 148u * 8u), 256,
-                                   PartSmem<kMidIsland>::kBytes, side(0)>>>(s, lvl_bound, 0);
-    if (s.n_joints) k_prep_joints<<<grid_for(s.n_joints, 128, 1u << 30), 128, 0, side(2)>>>(s);   // ~150 registers
-    k_prep_contacts<<<grid_for(s.desc_cap, 128, cap_blocks), 128, 0, side(2)>>>(s);
-    join_branches(br, st, 3);
+                                   PartSmem<kMidIsland>::kBytes, side(3)>>>(s, lvl_bound, 0);
+    join_branches(br, st, 4);
     // PGS: islands by size class, independent.  The clusters' eight CTAs
     // need room in one part of the chip at once: they go first and with
     // priority, or they wait until the other classes have drained (127 us of
