@@ -3,15 +3,16 @@
 Sweeps, on a B200, the parameters that change how a step runs but not what
 it computes (every setting gives bit-identical results):
 
-  island_thread   islands of at most this many descriptors: one thread each
-  island_warp     ... up to this many: one warp each
-  island_cta      ... up to this many: one 128-thread CTA (larger: 384 threads)
+  island_thread   accepted, without effect (small islands are solved in groups)
+  island_warp     rollouts' reverse sweep: islands of 33 to this many
+                  descriptors by one warp each
+  island_cta      ... up to this many by one 128-thread CTA
   radix_bits      digit width of the device-wide radix sorts (endpoint sort of
                   large scenes, island sort of the descriptors)
   elem_block      threads a block of the elementwise kernels
-  work_queue      warp / CTA solvers take islands round-robin (0) or from a
-                  device work queue, a per-step counter each worker draws
-                  the next island from (1)
+  work_queue      the small islands' solver takes its groups round-robin (0)
+                  or from a device work queue, a per-step counter each CTA
+                  draws the next group from (1)
 
 for each world class the library distinguishes -- "large_scene" (some scene
 above 2,048 finite shapes: the 131,072-body plain scene from its settled

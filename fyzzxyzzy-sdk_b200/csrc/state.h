@@ -43,16 +43,16 @@ struct DevState {
     uint32_t pair_cap = 0, desc_cap = 0;
     uint32_t max_small_scene = 2048;   // finite shapes sorted inside one CTA
     // Performance parameters (fyzz_b200_tuning_t; every choice gives the same
-    // results): islands of at most isl_thread descriptors are solved by one
-    // thread, up to isl_warp by one warp, up to isl_mid by a 128-thread CTA,
-    // up to kBigIsland by the 384-thread CTA; radix sorts take digits of
-    // radix_bits; elementwise kernels run elem_block threads a block.
+    // results): a rollout's reverse sweep solves islands of (32, isl_warp]
+    // descriptors by one warp, up to isl_mid by a 128-thread CTA; radix sorts
+    // take digits of radix_bits; elementwise kernels run elem_block threads a
+    // block.  isl_thread has no effect.
     uint32_t isl_thread = 8, isl_warp = 96, isl_mid = 512;
     int radix_bits = 8;
     uint32_t elem_block = 256;
-    // Island scheduling of the warp and CTA solvers: false = static (worker
-    // w takes list entries w, w + W, ...), true = a work queue (each worker
-    // takes the next entry from a per-step device counter).
+    // Scheduling of the small islands' groups: false = static (CTA w takes
+    // groups w, w + W, ...), true = a work queue (each CTA takes the next
+    // group from a per-step device counter).
     bool work_queue = false;
     int pos_iters = 4, vel_iters = 1;
     uint64_t neg_zero2 = 0x8000000080000000ull;   // {-0, -0}, opaque to the kernels' compiler
@@ -269,7 +269,7 @@ void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t* keys_alt, uint32
                       uint32_t* os_scratch = nullptr, size_t os_words = 0);
 constexpr int kRadixMaxBits = 11;   // widest radix digit
 size_t radix_hist_words(uint32_t n_cap);
-// One-sweep scratch of radix_sort_pairs (8-bit digits); zero when allocated.
+// One-sweep scratch of radix_sort_pairs (8- to 10-bit digits); zero when allocated.
 size_t onesweep_words(uint32_t n_cap);
 void init_primitive_kernels();
 size_t scan_tmp_words_for(uint32_t n_cap);
@@ -361,9 +361,9 @@ void enqueue_unpack_velocities(const DevState& s, const float* rec, uint32_t str
                                cudaStream_t st);
 void init_solver_kernels();
 // Island size classes (descriptors per island).
-constexpr uint32_t kSmallIsland = 96;     // one warp
-constexpr uint32_t kMidIsland = 512;      // one CTA, shared-memory deltas
-constexpr uint32_t kBigIsland = 4096;     // one CTA, shared-memory deltas (1 CTA / SM)
+constexpr uint32_t kSmallIsland = 96;     // reverse sweep: one warp
+constexpr uint32_t kMidIsland = 512;      // partition: 256 threads up to here, 1,024 above
+constexpr uint32_t kBigIsland = 4096;     // beyond: partition and PGS in global memory
 // counters[] slots
 enum : int { kCntMan = 0, kCntDesc = 1, kCntIsl = 2, kCntFrame = 3, kCntLevels = 4, kCntGjk = 5,
              kCntAwake = 6 /* descriptors of awake islands */, kCntSleeping = 7 /* asleep at step start */,

@@ -212,14 +212,14 @@ int fyzz_b200_profile_step(fyzz_b200_world* w, float seconds, float* stage_ms, u
  * when some scene has more than 2,048 finite shapes, else "many_scenes".
  * fyzz_b200_set_tuning overrides it for the world. */
 typedef struct {
-    uint32_t island_thread;  /* islands of at most this many descriptors are solved by one thread (0..8; 8) */
-    uint32_t island_warp;    /* ... up to this many by one warp (32..96; 96) */
-    uint32_t island_cta;     /* ... up to this many by one 128-thread CTA (128..512; 512); larger islands up to
-                                4,096 by one 384-thread CTA, beyond that from global memory */
+    uint32_t island_thread;  /* accepted, without effect since small islands are solved in groups (0..8; 8) */
+    uint32_t island_warp;    /* rollouts' reverse sweep: islands of 33 to this many descriptors by one warp (32..96; 96) */
+    uint32_t island_cta;     /* ... up to this many by one 128-thread CTA (128..512; 512), larger ones from global
+                                memory.  The forward solver's classes are fixed by shared-memory sizes */
     uint32_t radix_bits;     /* digit width of the device-wide radix sorts (8..11; 8) */
     uint32_t elem_block;     /* threads a block of the elementwise kernels (64..1024, multiple of 32; 256) */
-    uint32_t work_queue;     /* warp and CTA solvers take islands round-robin (0) or from a device work
-                                queue, the next list entry per worker from a per-step counter (1); 0 */
+    uint32_t work_queue;     /* the small islands' solver takes its groups round-robin (0) or from a device
+                                work queue, the next group per CTA from a per-step counter (1); 0 */
 } fyzz_b200_tuning_t;
 int fyzz_b200_set_tuning(fyzz_b200_world* w, const fyzz_b200_tuning_t* tuning);
 int fyzz_b200_get_tuning(fyzz_b200_world* w, fyzz_b200_tuning_t* tuning);
