@@ -44,7 +44,7 @@ EXPORTS = (
     "fyzz_b200_cook_convex_mesh", "fyzz_b200_convex_mesh_release", "fyzz_b200_cook_error",
     "fyzz_b200_convex_mesh_info", "fyzz_b200_attach_convex_shape", "fyzz_b200_add_scene_ex",
     "fyzz_b200_write_velocities_strided", "fyzz_b200_remove_constraint",
-    "fyzz_b200_set_pair_budget", "fyzz_b200_test_scan",
+    "fyzz_b200_set_pair_budget", "fyzz_b200_test_scan", "fyzz_b200_test_clear_normals",
     "fyzz_b200_set_body_contact_report_threshold", "fyzz_b200_force_threshold_changes",
     "fyzz_b200_read_islands", "fyzz_b200_set_caller_validated_transforms",
     "fyzz_b200_set_descriptor_order", "fyzz_b200_set_tuning", "fyzz_b200_get_tuning",
@@ -191,6 +191,7 @@ def lib():
         L.fyzz_b200_set_body_contact_report_threshold.argtypes = [vp, u32, f32]
         L.fyzz_b200_force_threshold_changes.argtypes = [vp, P(P(ForceThresholdReport)), P(u64)]
         L.fyzz_b200_test_scan.argtypes = [vp, u32, i32, P(u32), P(u64)]
+        L.fyzz_b200_test_clear_normals.argtypes = [vp, u32, u32]
         L.fyzz_b200_rollout_forward.argtypes = [vp, f32]
         L.fyzz_b200_rollout_backward.argtypes = [vp] + [vp] * 9
         L.fyzz_b200_read_mass_frames.argtypes = [vp, vp, vp]
@@ -584,6 +585,10 @@ class World:
         self.last_scan = (bits.value, bad.value)
         self._check(rc)
         return bits.value, bad.value
+
+    def test_clear_normals(self, shape_a: int, shape_b: int):
+        """Test hook: zeroes the cached contact normals of a pair of boxes."""
+        self._check(lib().fyzz_b200_test_clear_normals(self.h, shape_a, shape_b))
 
     def rollout_begin(self, steps: int, checkpoint_every: int):
         self._check(lib().fyzz_b200_rollout_begin(self.h, steps, checkpoint_every))

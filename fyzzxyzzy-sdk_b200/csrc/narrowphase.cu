@@ -929,9 +929,6 @@ __device__ __forceinline__ float pcm_box_margin(v3 h) { return smin(0.15f * smin
 __device__ int emit_box_box(qt q1, v3 p1, float cd, const PcmCache& cache, bool direct, bool gjk, v3 gjk_n,
                             ContactPt* out);
 
-// Returns the emitted count, or -1 on an invalid manifold normal / overflow.
-// Sets gjk_pending (and emits nothing) when the zero-face GJK/EPA
-// continuation must complete the manifold.
 // Box/box: refreshes the cached manifold; true when it has to be regenerated.
 __device__ bool box_box_stale(v3 h0, v3 p0, qt q0, v3 h1, v3 p1, qt q1, PcmCache& cache) {
     const v3 delta = {p0.x - p1.x, p0.y - p1.y, p0.z - p1.z};
@@ -1028,6 +1025,8 @@ __device__ int finish_box_box_gjk(v3 h0, v3 h1, v3 p1, qt q1, float cd, PcmCache
     return emit_box_box(q1, p1, cd, cache, false, true, w.nb, out);
 }
 
+// Returns the emitted count, or -1 when the manifold's normal is zero or not
+// finite (cached normals that cancel).
 __device__ int emit_box_box(qt q1, v3 p1, float cd, const PcmCache& cache, bool direct, bool gjk, v3 gjk_n,
                             ContactPt* out) {
     const uint32_t n = cache_count(cache);
@@ -1246,6 +1245,21 @@ __device__ __forceinline__ PairShapes pair_shapes(const DevState& s, uint64_t ke
     return p;
 }
 
+// Pair k's contacts, and its cache (sphere pairs keep none).  Every
+// generator ends here: a negative count is an invalid manifold, which raises
+// the step's error and leaves the pair without contacts (the kernels that
+// read cur.count trust it to be at most four).
+__device__ __forceinline__ void store_manifold(const DevState& s, uint32_t k, const PcmCache* cache, int count,
+                                               const ContactPt* out) {
+    if (count < 0) {
+        atomicOr(s.err, kErrContactOverflow);
+        count = 0;
+    }
+    if (cache) s.cur.cache[k] = *cache;
+    s.cur.count[k] = uint32_t(count);
+    for (int j = 0; j < count; ++j) s.pts[4 * size_t(k) + j] = out[j];
+}
+
 // Box and plane pairs whose cached manifold went stale (kSplit; tmp_flags is
 // free until the step's events).
 __device__ __forceinline__ uint32_t* regen_list(const DevState& s) { return s.tmp_flags; }
@@ -1329,13 +1343,12 @@ __global__ void __launch_bounds__(128) k_narrowphase(DevState s) {
                 }
             }
         }
-        if (pcm) s.cur.cache[k] = cache;
         if (kSplit && stale) {
+            s.cur.cache[k] = cache;
             regen_list(s)[atomicAdd(&s.counters[kCntRegen], 1u)] = k;
             continue;
         }
-        s.cur.count[k] = uint32_t(count);
-        for (int i = 0; i < count; ++i) s.pts[4 * size_t(k) + i] = out[i];
+        store_manifold(s, k, pcm ? &cache : nullptr, count, out);
         // friction histories are not carried here: row preparation reads a
         // touching manager's history from the previous generation
     }
@@ -1355,9 +1368,7 @@ __global__ void __launch_bounds__(128) k_narrowphase_regen(DevState s) {
         int count = 0;
         if (regenerate(s, k, ps, {g0.x, g0.y, g0.z}, {g1.x, g1.y, g1.z}, p0, p1, q0, q1, cache))
             count = emit_box_pair(ps, p0, p1, q1, cache, true, out);
-        s.cur.cache[k] = cache;
-        s.cur.count[k] = uint32_t(count);
-        for (int j = 0; j < count; ++j) s.pts[4 * size_t(k) + j] = out[j];
+        store_manifold(s, k, &cache, count, out);
     }
 }
 
@@ -1395,14 +1406,8 @@ __global__ void __launch_bounds__(kGjkWarps * 32, 3) k_narrowphase_gjk(DevState 
             have = have && w.sep <= ps.cd;
             PcmCache cache = s.cur.cache[k];
             ContactPt out[4];
-            int count = finish_box_box_gjk(h0, h1, p1, q1, ps.cd, cache, have, w, out);
-            if (count < 0) {
-                atomicOr(s.err, kErrContactOverflow);
-                count = 0;
-            }
-            s.cur.cache[k] = cache;
-            s.cur.count[k] = uint32_t(count);
-            for (int j = 0; j < count; ++j) s.pts[4 * size_t(k) + j] = out[j];
+            const int count = finish_box_box_gjk(h0, h1, p1, q1, ps.cd, cache, have, w, out);
+            store_manifold(s, k, &cache, count, out);
         }
         __syncwarp();
     }
@@ -1943,16 +1948,6 @@ __device__ int convex_emit(const Fin& f1, float cd, const PcmCache& cache, Conta
     }
     return count;
 }
-__device__ __forceinline__ void store_manifold(const DevState& s, uint32_t k, const PcmCache& cache, int count,
-                                               const ContactPt* out) {
-    if (count < 0) {
-        atomicOr(s.err, kErrContactOverflow);
-        count = 0;
-    }
-    s.cur.cache[k] = cache;
-    s.cur.count[k] = uint32_t(count);
-    for (int j = 0; j < count; ++j) s.pts[4 * size_t(k) + j] = out[j];
-}
 
 // Pairs with a cooked hull, one thread each: hull vertices against the
 // floor, and finite pairs whose cached manifold stays valid.  Finite pairs
@@ -1967,7 +1962,7 @@ __global__ void __launch_bounds__(128) k_narrowphase_convex(DevState s) {
         ContactPt out[4];
         if (ps.plane) {
             const int count = plane_hull(s, ps, cache, out);
-            store_manifold(s, k, cache, count, out);
+            store_manifold(s, k, &cache, count, out);
             continue;
         }
         const Fin f0 = load_fin(s, ps.first), f1 = load_fin(s, ps.second);
@@ -1977,7 +1972,7 @@ __global__ void __launch_bounds__(128) k_narrowphase_convex(DevState s) {
             s.cvx_gjk_list[atomicAdd(&s.counters[kCntConvexGjk], 1u)] = k;
             continue;
         }
-        store_manifold(s, k, cache, convex_emit(f1, ps.cd, cache, out), out);
+        store_manifold(s, k, &cache, convex_emit(f1, ps.cd, cache, out), out);
     }
 }
 
@@ -2028,7 +2023,7 @@ __device__ void convex_finish(const DevState& s, uint32_t k, bool have, Cand w, 
     }
     if (lane == 0) {
         ContactPt out[4];
-        store_manifold(s, k, cache, convex_emit(f1, cd, cache, out), out);
+        store_manifold(s, k, &cache, convex_emit(f1, cd, cache, out), out);
     }
 }
 __global__ void __launch_bounds__(kCvxWarps * 32, 3) k_narrowphase_convex_gjk(DevState s) {
@@ -2132,7 +2127,7 @@ __global__ void __launch_bounds__(kCvxWarps * 32) k_narrowphase_convex_clip(DevS
                 set_meta(cache, 1, true);
             }
             ContactPt out[4];
-            store_manifold(s, k, cache, convex_emit(f1, ps.cd, cache, out), out);
+            store_manifold(s, k, &cache, convex_emit(f1, ps.cd, cache, out), out);
         }
         __syncwarp();
     }

@@ -889,6 +889,25 @@ public:
         if (mismatches) *mismatches = bad;
         return bits;
     }
+    void clear_cached_normals(uint32_t a, uint32_t b) {
+        check_cuda(cudaSetDevice(device_), "cudaSetDevice");
+        ensure_device();
+        check_cuda(cudaStreamSynchronize(stream_), "sync");
+        const ManagerSet& set = sets_[last_cur_];
+        uint32_t n = 0;
+        check_cuda(cudaMemcpy(&n, set.n, 4, cudaMemcpyDeviceToHost), "read");
+        std::vector<uint64_t> keys(n);
+        if (n) check_cuda(cudaMemcpy(keys.data(), set.key, size_t(n) * 8, cudaMemcpyDeviceToHost), "read");
+        const auto at = std::find(keys.begin(), keys.end(), uint64_t(std::min(a, b)) << 32 | std::max(a, b));
+        if (at == keys.end()) throw std::out_of_range("Not an overlapping pair");
+        if (shapes_[a].type != kBox || shapes_[b].type != kBox) throw std::invalid_argument("Not a pair of boxes");
+        PcmCache* slot = set.cache + (at - keys.begin());
+        PcmCache cache;
+        check_cuda(cudaMemcpy(&cache, slot, sizeof cache, cudaMemcpyDeviceToHost), "read");
+        if ((cache.meta & 255u) == 0) throw std::invalid_argument("The pair has no cached contacts");
+        for (PcmPoint& p : cache.pts) p.nb[0] = p.nb[1] = p.nb[2] = 0.0f;
+        check_cuda(cudaMemcpy(slot, &cache, sizeof cache, cudaMemcpyHostToDevice), "write");
+    }
     // ---------------- differentiable rollouts ----------------
     // A rollout of `steps` steps keeps a full-state checkpoint every `every`
     // steps.  The backward pass walks the segments in reverse: it restores
@@ -2678,6 +2697,9 @@ int fyzz_b200_test_scan(fyzz_b200_world* w, uint32_t n, int skip_first_tile, uin
         if (bits & fyzz::b200::kErrLogic)
             throw std::logic_error("Scan look-back wait gave up (error bits " + std::to_string(bits) + ")");
     });
+}
+int fyzz_b200_test_clear_normals(fyzz_b200_world* w, uint32_t shape_a, uint32_t shape_b) {
+    return guarded(w, [&](auto& W) { W.clear_cached_normals(shape_a, shape_b); });
 }
 int fyzz_b200_rollout_begin(fyzz_b200_world* w, uint32_t steps, uint32_t checkpoint_every) {
     return guarded(w, [&](auto& W) { W.rollout_begin(steps, checkpoint_every); });

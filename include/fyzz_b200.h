@@ -411,6 +411,11 @@ int fyzz_b200_set_descriptor_order(fyzz_b200_world* w, const uint32_t* pairs, ui
  * scans and steps run normally. */
 int fyzz_b200_test_scan(fyzz_b200_world* w, uint32_t n, int skip_first_tile, uint32_t* error_bits,
                         uint64_t* mismatches);
+/* Test hook (no reference counterpart): zeroes the cached contact normals of
+ * an overlapping pair of boxes, as normals that cancel would leave their sum.
+ * The next step finds the manifold invalid: it reports the contact error bit
+ * (FYZZ_B200_OVERFLOW) and rolls back. */
+int fyzz_b200_test_clear_normals(fyzz_b200_world* w, uint32_t shape_a, uint32_t shape_b);
 
 /* ---- broadphase / narrowphase views (Scene::pairs, found_pairs,
  *      lost_pairs, contacts: scene.h:827-833) ---- */
