@@ -1245,52 +1245,58 @@ __device__ __forceinline__ PairShapes pair_shapes(const DevState& s, uint64_t ke
     return p;
 }
 
-// Pair k's contacts, and its cache (sphere pairs keep none).  Every
-// generator ends here: a negative count is an invalid manifold, which raises
-// the step's error and leaves the pair without contacts (the kernels that
-// read cur.count trust it to be at most four).
-__device__ __forceinline__ void store_manifold(const DevState& s, uint32_t k, const PcmCache* cache, int count,
-                                               const ContactPt* out) {
+// Pair k's contacts.  Every generator ends here: a negative count is an
+// invalid manifold, which raises the step's error and leaves the pair without
+// contacts (the kernels that read cur.count trust it to be at most four).
+__device__ __forceinline__ void store_contacts(const DevState& s, uint32_t k, int count, const ContactPt* out) {
     if (count < 0) {
         atomicOr(s.err, kErrContactOverflow);
         count = 0;
     }
-    if (cache) s.cur.cache[k] = *cache;
     s.cur.count[k] = uint32_t(count);
     for (int j = 0; j < count; ++j) s.pts[4 * size_t(k) + j] = out[j];
+}
+__device__ __forceinline__ void store_manifold(const DevState& s, uint32_t k, const PcmCache& cache, int count,
+                                               const ContactPt* out) {
+    s.cur.cache[k] = cache;
+    store_contacts(s, k, count, out);
 }
 
 // Box and plane pairs whose cached manifold went stale (kSplit; tmp_flags is
 // free until the step's events).
 __device__ __forceinline__ uint32_t* regen_list(const DevState& s) { return s.tmp_flags; }
-// A stale pair's manifold; whether it has contacts to emit (box/box pairs
-// without face contact go on to k_narrowphase_gjk).
-__device__ __forceinline__ bool regenerate(const DevState& s, uint32_t k, const PairShapes& ps, v3 h0, v3 h1, v3 p0,
-                                           v3 p1, qt q0, qt q1, PcmCache& cache) {
-    if (ps.plane) {
-        regenerate_plane_box(p0, h1, p1, q1, ps.cd, cache);
-        return true;
+// A box pair's refresh, the regeneration of a stale manifold and its
+// contacts in one call, for the one-kernel narrowphase.  Written into the
+// kernel as one refresh, regeneration and emission for both kinds of pair they
+// took, a step, 104 us for 1,024 scenes of 64 boxes, 22.0 for 1,000 boxes, 26.4
+// for 1,200 jointed ones, 39.6 for a pile of 20,011; a call for each kind takes
+// 91, 17.9, 20.2 and 37.5.  The registers (122) are not what it gains by:
+// bounded to 80 it takes 103, 19.3, 21.4 and 41.3.
+__device__ __noinline__ int generate_box_box(v3 h0, v3 p0, qt q0, v3 h1, v3 p1, qt q1, float cd, PcmCache& cache,
+                                             ContactPt* out, bool& gjk) {
+    const bool stale = box_box_stale(h0, p0, q0, h1, p1, q1, cache);
+    if (stale) {
+        const int r = regenerate_box_box(h0, p0, q0, h1, p1, q1, cd, cache);
+        gjk = r == kBoxGjk;
+        if (r != kBoxFaces) return r == kBoxOverflow ? -1 : 0;
     }
-    const int r = regenerate_box_box(h0, p0, q0, h1, p1, q1, ps.cd, cache);
-    if (r == kBoxGjk) s.gjk_list[atomicAdd(&s.counters[kCntGjk], 1u)] = k;
-    if (r == kBoxOverflow) atomicOr(s.err, kErrContactOverflow);
-    return r == kBoxFaces;
+    return emit_box_box(q1, p1, cd, cache, stale, false, {0, 0, 0}, out);
 }
-__device__ __forceinline__ int emit_box_pair(const PairShapes& ps, v3 p0, v3 p1, qt q1, const PcmCache& cache,
-                                             bool fresh, ContactPt* out) {
-    return ps.plane ? emit_plane_box(p0, ps.cd, cache, out)
-                    : emit_box_box(q1, p1, ps.cd, cache, fresh, false, {0, 0, 0}, out);
+__device__ __noinline__ int generate_plane_box(v3 pp, v3 h, v3 bp, qt q, float cd, PcmCache& cache, ContactPt* out) {
+    if (plane_box_stale(pp, h, bp, q, cache)) regenerate_plane_box(pp, h, bp, q, cd, cache);
+    return emit_plane_box(pp, cd, cache, out);
 }
 
 // One thread a pair: sphere pairs, the refresh of box manifolds, and (kSplit
 // false) the regeneration of stale ones.  kSplit lists those instead for
 // k_narrowphase_regen: in one kernel the clipping of a few pairs holds up
-// nearly every warp (11 of 32 lanes active).  That pays where the pairs fill
-// the device many times over -- 1.3 million pairs 866 against 350 + 270 us,
-// 380,000 pairs 187 against 116 + 28 us -- while a small world only gets a
-// second kernel as long as one regeneration: 57,000 pairs 44 against 49 us,
-// 200 pairs 16 against 22 us.  The line is drawn by the pair budget, which
-// the host knows (kSplitPairs, about three live pairs a budgeted ten).
+// nearly every warp (11 of 32 lanes active), while two kernels are at least
+// as long as one regeneration each.  One kernel against two: 57,600 live
+// pairs 34 us against 22 + 22, 159,000 64 against 45 + 29, 323,000 120
+// against 80 + 28, 674,000 274 against 158 + 32 (batched scenes), 381,000 118
+// against 94 + 30 (one pile; its step 1,005 against 982).  The line, near
+// 315,000 live pairs, is drawn by the pair budget, which the host knows
+// (kSplitPairs: a default budget holds three live pairs in ten).
 constexpr uint32_t kSplitPairs = 1u << 20;
 template <bool kSplit>
 __global__ void __launch_bounds__(128) k_narrowphase(DevState s) {
@@ -1319,13 +1325,21 @@ __global__ void __launch_bounds__(128) k_narrowphase(DevState s) {
         const v3 p0 = ld3(s.s_wp[first]), p1 = ld3(s.s_wp[second]);
         const qt q0 = ldq(s.s_wq[first]), q1 = ldq(s.s_wq[second]);
         const float4 g0 = s.s_geom[first], g1 = s.s_geom[second];
+        const v3 h0 = {g0.x, g0.y, g0.z}, h1 = {g1.x, g1.y, g1.z};
         bool stale = false;
-        if (!sphere) {
-            const v3 h0 = {g0.x, g0.y, g0.z}, h1 = {g1.x, g1.y, g1.z};
+        if (!sphere && kSplit) {
+            // both kinds in one branch: a record's loads are then in flight
+            // together (126 registers); a branch each, as below, takes 56 and
+            // 368 us for 1.3 million pairs against 300
             stale = plane ? plane_box_stale(p0, h1, p1, q1, cache) : box_box_stale(h0, p0, q0, h1, p1, q1, cache);
-            bool emit = !stale;
-            if (!kSplit && stale) emit = regenerate(s, k, ps, h0, h1, p0, p1, q0, q1, cache);
-            if (emit) count = emit_box_pair(ps, p0, p1, q1, cache, stale, out);
+            if (!stale) count = plane ? emit_plane_box(p0, cd, cache, out)
+                                      : emit_box_box(q1, p1, cd, cache, false, false, {0, 0, 0}, out);
+        } else if (!sphere && plane) {
+            count = generate_plane_box(p0, h1, p1, q1, cd, cache, out);
+        } else if (!sphere) {
+            bool gjk = false;
+            count = generate_box_box(h0, p0, q0, h1, p1, q1, cd, cache, out, gjk);
+            if (gjk) s.gjk_list[atomicAdd(&s.counters[kCntGjk], 1u)] = k;
         } else {
             const uint32_t sp = ta == kSphere ? sa : sb;
             const v3 c = ld3(s.s_wp[sp]);
@@ -1343,12 +1357,12 @@ __global__ void __launch_bounds__(128) k_narrowphase(DevState s) {
                 }
             }
         }
+        if (pcm) s.cur.cache[k] = cache;
         if (kSplit && stale) {
-            s.cur.cache[k] = cache;
             regen_list(s)[atomicAdd(&s.counters[kCntRegen], 1u)] = k;
             continue;
         }
-        store_manifold(s, k, pcm ? &cache : nullptr, count, out);
+        store_contacts(s, k, count, out);
         // friction histories are not carried here: row preparation reads a
         // touching manager's history from the previous generation
     }
@@ -1365,10 +1379,18 @@ __global__ void __launch_bounds__(128) k_narrowphase_regen(DevState s) {
         const float4 g0 = s.s_geom[ps.first], g1 = s.s_geom[ps.second];
         PcmCache cache = s.cur.cache[k];
         ContactPt out[4];
+        const v3 h0 = {g0.x, g0.y, g0.z}, h1 = {g1.x, g1.y, g1.z};
         int count = 0;
-        if (regenerate(s, k, ps, {g0.x, g0.y, g0.z}, {g1.x, g1.y, g1.z}, p0, p1, q0, q1, cache))
-            count = emit_box_pair(ps, p0, p1, q1, cache, true, out);
-        store_manifold(s, k, &cache, count, out);
+        if (ps.plane) {
+            regenerate_plane_box(p0, h1, p1, q1, ps.cd, cache);
+            count = emit_plane_box(p0, ps.cd, cache, out);
+        } else {
+            const int r = regenerate_box_box(h0, p0, q0, h1, p1, q1, ps.cd, cache);
+            if (r == kBoxGjk) s.gjk_list[atomicAdd(&s.counters[kCntGjk], 1u)] = k;
+            if (r == kBoxOverflow) count = -1;
+            if (r == kBoxFaces) count = emit_box_box(q1, p1, ps.cd, cache, true, false, {0, 0, 0}, out);
+        }
+        store_manifold(s, k, cache, count, out);
     }
 }
 
@@ -1407,7 +1429,7 @@ __global__ void __launch_bounds__(kGjkWarps * 32, 3) k_narrowphase_gjk(DevState 
             PcmCache cache = s.cur.cache[k];
             ContactPt out[4];
             const int count = finish_box_box_gjk(h0, h1, p1, q1, ps.cd, cache, have, w, out);
-            store_manifold(s, k, &cache, count, out);
+            store_manifold(s, k, cache, count, out);
         }
         __syncwarp();
     }
@@ -1962,7 +1984,7 @@ __global__ void __launch_bounds__(128) k_narrowphase_convex(DevState s) {
         ContactPt out[4];
         if (ps.plane) {
             const int count = plane_hull(s, ps, cache, out);
-            store_manifold(s, k, &cache, count, out);
+            store_manifold(s, k, cache, count, out);
             continue;
         }
         const Fin f0 = load_fin(s, ps.first), f1 = load_fin(s, ps.second);
@@ -1972,7 +1994,7 @@ __global__ void __launch_bounds__(128) k_narrowphase_convex(DevState s) {
             s.cvx_gjk_list[atomicAdd(&s.counters[kCntConvexGjk], 1u)] = k;
             continue;
         }
-        store_manifold(s, k, &cache, convex_emit(f1, ps.cd, cache, out), out);
+        store_manifold(s, k, cache, convex_emit(f1, ps.cd, cache, out), out);
     }
 }
 
@@ -2023,7 +2045,7 @@ __device__ void convex_finish(const DevState& s, uint32_t k, bool have, Cand w, 
     }
     if (lane == 0) {
         ContactPt out[4];
-        store_manifold(s, k, &cache, convex_emit(f1, cd, cache, out), out);
+        store_manifold(s, k, cache, convex_emit(f1, cd, cache, out), out);
     }
 }
 __global__ void __launch_bounds__(kCvxWarps * 32, 3) k_narrowphase_convex_gjk(DevState s) {
@@ -2127,7 +2149,7 @@ __global__ void __launch_bounds__(kCvxWarps * 32) k_narrowphase_convex_clip(DevS
                 set_meta(cache, 1, true);
             }
             ContactPt out[4];
-            store_manifold(s, k, &cache, convex_emit(f1, ps.cd, cache, out), out);
+            store_manifold(s, k, cache, convex_emit(f1, ps.cd, cache, out), out);
         }
         __syncwarp();
     }
