@@ -1294,10 +1294,10 @@ __device__ __noinline__ int generate_plane_box(v3 pp, v3 h, v3 bp, qt q, float c
 // as long as one regeneration each.  One kernel against two: 57,600 live
 // pairs 34 us against 22 + 22, 159,000 64 against 45 + 29, 323,000 120
 // against 80 + 28, 674,000 274 against 158 + 32 (batched scenes), 381,000 118
-// against 94 + 30 (one pile; its step 1,005 against 982).  The line, near
-// 315,000 live pairs, is drawn by the pair budget, which the host knows
-// (kSplitPairs: a default budget holds three live pairs in ten).
-constexpr uint32_t kSplitPairs = 1u << 20;
+// against 94 + 30 (one pile; its step 1,005 against 982); rollouts, 127,000
+// pairs 93 against 85, 180,000 85 against 91.  The line is drawn by the live
+// pairs that the host's budget was made for (DevState::pairs_expected).
+constexpr uint32_t kSplitPairs = 300000;
 template <bool kSplit>
 __global__ void __launch_bounds__(128) k_narrowphase(DevState s) {
     const uint32_t n = *s.cur.n;
@@ -2162,7 +2162,7 @@ void enqueue_narrowphase(const DevState& s, cudaStream_t st, const StageHook& ho
     hook(kStNarrow, st);
     const uint32_t blocks = (s.pair_cap + T - 1) / T;
     const uint32_t grid = blocks < 148u * 16u ? blocks : 148u * 16u;
-    if (s.pair_cap >= kSplitPairs) {
+    if (s.pairs_expected >= kSplitPairs) {
         k_narrowphase<true><<<grid, T, 0, st>>>(s);
         k_narrowphase_regen<<<grid, T, 0, st>>>(s);
     } else {

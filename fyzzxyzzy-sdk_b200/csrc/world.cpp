@@ -733,7 +733,7 @@ public:
         const uint64_t want = uint64_t(double(std::max(live[0], live[1])) * headroom) + 4096;
         const uint32_t cap = uint32_t(std::min<uint64_t>(want, 0x7fffffffull));
         if (cap < std::max(live[0], live[1])) throw std::overflow_error("Pair budget below the live pairs");
-        resize_pairs_keeping(cap, live);
+        resize_pairs_keeping(cap, live, std::max(live[0], live[1]));
     }
     // Sets the pair budget to `cap` pairs (at least the live pairs of both
     // generations), keeping the contact-manager history.
@@ -751,7 +751,7 @@ public:
     // Re-allocates the pair arrays for `cap` pairs; both generations' live
     // records (keys, PCM caches, friction histories, touch counts) are
     // carried over, so the next step continues exactly as it would have.
-    void resize_pairs_keeping(uint32_t cap, const uint32_t live[2]) {
+    void resize_pairs_keeping(uint32_t cap, const uint32_t live[2], uint32_t expected = 0) {
         std::vector<void*> tmp;
         ManagerSet keep[2];
         for (int k = 0; k < 2; ++k) {
@@ -772,7 +772,7 @@ public:
             }
         check_cuda(cudaStreamSynchronize(stream_), "sync");
         const int parity = parity_, last = last_cur_;
-        alloc_pairs(cap);
+        alloc_pairs(cap, expected);
         for (int k = 0; k < 2; ++k) enqueue_copy_set(sets_[k], keep[k], live[k], stream_);
         if (d_.thresholds)
             for (int k = 0; k < 2; ++k) enqueue_copy_threshold_set(th_sets_[k], keep_th[k], live_th[k], stream_);
@@ -1778,7 +1778,9 @@ private:
         uploaded_ = false;
     }
 
-    void alloc_pairs(uint32_t cap) {
+    // expected: the live pairs a budget fits; the others (nine a body and
+    // their doublings) come to hold some three live pairs in ten.
+    void alloc_pairs(uint32_t cap, uint32_t expected = 0) {
         for (void* p : pair_owned_) cudaFree(p);
         pair_owned_.clear();
         bk_set_ = ManagerSet{};
@@ -1787,6 +1789,7 @@ private:
         for (auto& g : graphs_) if (g) { cudaGraphExecDestroy(g); g = nullptr; }
         release_segment_graphs();
         d_.pair_cap = cap;
+        d_.pairs_expected = expected ? expected : uint32_t(uint64_t(cap) * 3 / 10);
         d_.desc_cap = cap + d_.n_joints + kJointReserve;
         for (int k = 0; k < 2; ++k) {
             dalloc(sets_[k].key, cap, pair_owned_);
