@@ -3,10 +3,6 @@
 Sweeps, on a B200, the parameters that change how a step runs but not what
 it computes (every setting gives bit-identical results):
 
-  island_thread   accepted, without effect (small islands are solved in groups)
-  island_warp     rollouts' reverse sweep: islands of 33 to this many
-                  descriptors by one warp each
-  island_cta      ... up to this many by one 128-thread CTA
   radix_bits      digit width of the device-wide radix sorts (endpoint sort of
                   large scenes, island sort of the descriptors)
   elem_block      threads a block of the elementwise kernels
@@ -14,10 +10,19 @@ it computes (every setting gives bit-identical results):
                   or from a device work queue, a per-step counter each CTA
                   draws the next group from (1)
 
-for each world class the library distinguishes -- "large_scene" (some scene
+timed on forward steps, and
+
+  island_warp     rollouts' reverse sweep: islands of 33 to this many
+                  descriptors by one warp each
+  island_cta      ... up to this many by one 128-thread CTA
+
+timed on a rollout's backward pass, the only place they act
+(island_thread, the table's first column, has no effect and keeps its
+default), for each world class the library distinguishes -- "large_scene" (some scene
 above 2,048 finite shapes: the 131,072-body plain scene from its settled
-state, timed over steps 6-25 like the bench's headline) and "many_scenes"
-(the 4,096-scene batched world, timed over steps 61-80).  Every setting
+state, timed over steps 6-25 like the bench's headline, and a rollout of 8
+steps from there) and "many_scenes" (the 4,096-scene batched world, timed over
+steps 61-80, and a rollout of the 1,024 x 64 boxes after 60 steps).  Every setting
 computes the same trajectory, so each candidate is timed on a fresh world
 over exactly the same steps (CUDA events on the world's stream, the better
 of two worlds); one round of coordinate descent keeps a candidate when it
@@ -33,8 +38,8 @@ import argparse
 import datetime
 import importlib
 import os
-import statistics
 import sys
+import time
 
 import numpy as np
 
@@ -45,12 +50,13 @@ DEFAULTS = {"island_thread": 8, "island_warp": 96, "island_cta": 512, "radix_bit
             "work_queue": 0}
 CANDIDATES = {
     "radix_bits": [8, 9, 10, 11],
-    "island_thread": [0, 4, 8],
     "island_warp": [32, 64, 96],
     "island_cta": [128, 256, 512],
     "elem_block": [128, 256, 512],
     "work_queue": [0, 1],
 }
+STEP_PARAMS = ["work_queue", "radix_bits", "elem_block"]
+REVERSE_PARAMS = ["island_warp", "island_cta"]
 FIELDS = ["island_thread", "island_warp", "island_cta", "radix_bits", "elem_block", "work_queue"]
 
 
@@ -77,6 +83,11 @@ def many_scenes_specs(scenes):
     return scenes.batched_scenes(4096), 60
 
 
+def rollout_specs(scenes):
+    """The differentiable 1,024 x 64 boxes, after 60 steps."""
+    return scenes.loose_piles(1024), 60
+
+
 def measure(torch, pkg, specs, settle: int, params: dict, steps: int) -> float:
     """ms per step of a fresh world under `params`, over steps settle+1 ..
     settle+steps.  Every setting computes the same trajectory, so every
@@ -99,21 +110,43 @@ def measure(torch, pkg, specs, settle: int, params: dict, steps: int) -> float:
     return ms
 
 
-def tune(torch, pkg, specs, settle, steps: int, log) -> tuple[dict, float, float]:
-    """One round of coordinate descent: each parameter's candidates timed on
+def measure_reverse(pkg, specs, settle: int, params: dict, steps: int = 8) -> float:
+    """ms per step of a rollout's backward pass (recompute and adjoint) of a
+    fresh world under `params`; the first backward captures its graph."""
+    w = pkg.World(0)
+    for s in specs:
+        w.add_scene(s)
+    w.set_tuning(**params)
+    w.step(DT, settle)
+    w.fit_pair_budget(1.5)
+    grad = np.ones((w.counts()["bodies"], 3), np.float32)
+    ms = []
+    for run in range(3):
+        if run:
+            w.rollout_rewind()
+        w.rollout_begin(steps, steps)
+        w.rollout_forward(DT)
+        w.synchronize()
+        t = time.perf_counter()
+        w.rollout_backward(grad)
+        ms.append((time.perf_counter() - t) * 1e3 / steps)
+    w.close()
+    return min(ms[1:])
+
+
+def descend(timed, names, best: dict, log) -> tuple[dict, float, float]:
+    """One round of coordinate descent over `names`: each candidate timed on
     fresh worlds (the better of two), the fastest kept when at least 1%
     ahead of the incumbent."""
-    def timed(params):
-        return min(measure(torch, pkg, specs, settle, params, steps) for _ in range(2))
-    best = dict(DEFAULTS)
-    base = best_ms = timed(best)
-    log(f"  defaults {best}: {base:.4f} ms/step")
-    for name in ["work_queue", "radix_bits", "island_thread", "island_warp", "island_cta", "elem_block"]:
+    twice = lambda params: min(timed(params) for _ in range(2))  # noqa: E731
+    base = best_ms = twice(best)
+    log(f"  start {best}: {base:.4f} ms/step")
+    for name in names:
         for v in CANDIDATES[name]:
             if v == best[name]:
                 continue
             trial = dict(best, **{name: v})
-            ms = timed(trial)
+            ms = twice(trial)
             log(f"  {name}={v}: {ms:.4f} ms/step (incumbent {best_ms:.4f})")
             if ms < best_ms * 0.99:
                 best, best_ms = trial, ms
@@ -133,13 +166,17 @@ def main():
     def log(msg):
         print(msg, flush=True)
 
-    for cls, make in (("large_scene", large_scene_specs), ("many_scenes", many_scenes_specs)):
-        log(f"{cls}:")
-        specs, settle = make(scenes)
-        best, best_ms, base = tune(torch, pkg, specs, settle, args.steps, log)
+    for cls, make, make_rollout in (("large_scene", large_scene_specs, large_scene_specs),
+                                    ("many_scenes", many_scenes_specs, rollout_specs)):
+        best = dict(DEFAULTS)
+        for what, names, (specs, settle), timed in (
+                ("step", STEP_PARAMS, make(scenes), lambda p: measure(torch, pkg, specs, settle, p, args.steps)),
+                ("backward", REVERSE_PARAMS, make_rollout(scenes), lambda p: measure_reverse(pkg, specs, settle, p))):
+            log(f"{cls}, {what}:")
+            best, best_ms, base = descend(timed, names, best, log)
+            notes.append(f"# {cls} {what}: defaults {base:.4f} ms/step, tuned {best_ms:.4f} ms/step")
         lines.append(f"{cls} " + " ".join(str(best[f]) for f in FIELDS))
-        notes.append(f"# {cls}: defaults {base:.4f} ms/step, tuned {best_ms:.4f} ms/step")
-        log(f"  -> {best} ({base:.4f} -> {best_ms:.4f} ms/step)")
+        log(f"  -> {best}")
     gpu = torch.cuda.get_device_name(0)
     with open(args.out, "w") as f:
         f.write(f"# Step tuning table (fyzz_b200_tuning_t per world class), written by autotune.py on {gpu},\n")

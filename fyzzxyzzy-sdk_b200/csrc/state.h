@@ -47,8 +47,8 @@ struct DevState {
     // results): a rollout's reverse sweep solves islands of (32, isl_warp]
     // descriptors by one warp, up to isl_mid by a 128-thread CTA; radix sorts
     // take digits of radix_bits; elementwise kernels run elem_block threads a
-    // block.  isl_thread has no effect.
-    uint32_t isl_thread = 8, isl_warp = 96, isl_mid = 512;
+    // block.
+    uint32_t isl_warp = 96, isl_mid = 512;
     int radix_bits = 8;
     uint32_t elem_block = 256;
     // Scheduling of the small islands' groups: false = static (CTA w takes

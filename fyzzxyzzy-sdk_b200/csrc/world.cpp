@@ -2019,7 +2019,6 @@ private:
         check_cuda(cudaStreamSynchronize(stream_), "joint upload");
     }
     void apply_tuning() {
-        d_.isl_thread = tuning_.island_thread;
         d_.isl_warp = tuning_.island_warp;
         d_.isl_mid = tuning_.island_cta;
         d_.radix_bits = int(tuning_.radix_bits);
@@ -2099,7 +2098,6 @@ private:
             }
             tuning_ = t;
         }
-        d.isl_thread = tuning_.island_thread;
         d.isl_warp = tuning_.island_warp;
         d.isl_mid = tuning_.island_cta;
         d.radix_bits = int(tuning_.radix_bits);
