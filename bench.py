@@ -224,6 +224,7 @@ def step_bytes(c: dict, iters: int = 5) -> dict:
 def roofline_of(counts: dict, ms_per_step: float, stages: dict, peak: float, peak_kind: str) -> dict:
     """Whole-step roofline (all algorithmic bytes of a step / device time of
     a step) plus per-stage fractions for the stages the accounting covers;
+    row preparation runs beside the islands and is timed on its own branch;
     the island / partition stage has no algorithmic bytes (latency-bound
     integer work) and is listed with its time only."""
     per = step_bytes(counts)

@@ -394,7 +394,8 @@ class World:
 
     def profile_step(self, seconds: float = 1.0 / 120.0) -> dict:
         """One eagerly launched step; per-stage device milliseconds from CUDA
-        events the library records on its stream."""
+        events the library records on its streams.  "prep" runs beside the
+        later part of "islands"; the others follow one another."""
         out = np.zeros(len(STAGES), np.float32)
         self._check(lib().fyzz_b200_profile_step(self.h, seconds, _p(out), out.size))
         return dict(zip(STAGES, out.tolist()))

@@ -2340,8 +2340,13 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     // 1,776 against 1,798 with runs 1 % apart) and slower in large worlds
     // (131,072-body pile 4,005 against 3,925).
     fork_branches(br, st, 2);
+    hook(kStPrep, side(0));
     k_prep_contacts<<<grid_for(s.desc_cap, 128, cap_blocks), 128, 0, side(0)>>>(s);
-    if (s.n_joints) k_prep_joints<<<grid_for(s.n_joints, 128, 1u << 30), 128, 0, side(1)>>>(s);   // ~150 registers
+    hook(kStPrepEnd, side(0));
+    if (s.n_joints) {
+        k_prep_joints<<<grid_for(s.n_joints, 128, 1u << 30), 128, 0, side(1)>>>(s);   // ~150 registers
+        hook(kStPrepJointsEnd, side(1));
+    }
     k_desc_keys<<<grid_for(s.desc_cap, T, cap_blocks), T, 0, st>>>(s);
     if (s.replay) {
         int rbits = 1;
@@ -2359,7 +2364,6 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     k_island_compact<<<lookback_grid(s.desc_cap), kScanThreads, 0, st>>>(s);
     k_island_classes<<<grid_for(s.desc_cap, T, cap_blocks), T, 0, st>>>(s);
     // partitions by island size class: independent
-    hook(kStPrep, st);
     fork_branches(br, st, 4);
     launch(k_partition_smem<kBigIsland>, grid_for(s.desc_cap, kMidIsland + 1, 148u * 2u), PartSmem<kBigIsland>::kThreads,
                 PartSmem<kBigIsland>::kBytes, 1u, g_high_priority, side(2), s, lvl_bound, 2);

@@ -278,7 +278,10 @@ size_t scan_tmp_words_for(uint32_t n_cap);
 // Stage boundaries of one step, reported to an optional hook (the world uses
 // it to bracket stages with CUDA events when profiling).
 enum Stage : int {
-    kStBounds = 0, kStSort, kStPairs, kStNarrow, kStIslands, kStPrep, kStPgs, kStIntegrate, kStEnd
+    kStBounds = 0, kStSort, kStPairs, kStNarrow, kStIslands, kStPrep, kStPgs, kStIntegrate, kStEnd,
+    // Row preparation runs on side streams beside the islands: begun at
+    // kStPrep, its contacts done at kStPrepEnd, its joints at kStPrepJointsEnd.
+    kStPrepEnd, kStPrepJointsEnd, kStEvents
 };
 struct StageHook {
     void (*fn)(void* ctx, int stage, cudaStream_t st) = nullptr;

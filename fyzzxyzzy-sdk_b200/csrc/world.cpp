@@ -1382,8 +1382,8 @@ public:
         if (!std::isfinite(dt) || dt <= 0.0f) throw std::invalid_argument("timestep must be finite and positive");
         check_cuda(cudaSetDevice(device_), "cudaSetDevice");
         ensure_device();
-        struct Ctx { cudaEvent_t ev[kStEnd + 1]; bool seen[kStEnd + 1]; } ctx{};
-        for (int i = 0; i <= kStEnd; ++i) check_cuda(cudaEventCreate(&ctx.ev[i]), "event");
+        struct Ctx { cudaEvent_t ev[kStEvents]; bool seen[kStEvents]; } ctx{};
+        for (cudaEvent_t& e : ctx.ev) check_cuda(cudaEventCreate(&e), "event");
         StageHook hook;
         hook.ctx = &ctx;
         hook.fn = [](void* c, int stage, cudaStream_t st) {
@@ -1402,12 +1402,16 @@ public:
         const uint32_t err = read_err();
         last_cur_ = parity_;
         parity_ ^= 1;
-        for (uint32_t i = 0; i < n && i < uint32_t(kStEnd); ++i) {
+        const auto between = [&](int a, int b) {
             float t = 0.0f;
-            if (ctx.seen[i] && ctx.seen[i + 1]) cudaEventElapsedTime(&t, ctx.ev[i], ctx.ev[i + 1]);
-            ms[i] = t;
-        }
-        for (int i = 0; i <= kStEnd; ++i) cudaEventDestroy(ctx.ev[i]);
+            if (ctx.seen[a] && ctx.seen[b]) cudaEventElapsedTime(&t, ctx.ev[a], ctx.ev[b]);
+            return t;
+        };
+        for (uint32_t i = 0; i < n && i < uint32_t(kStEnd); ++i)
+            ms[i] = i == kStIslands ? between(kStIslands, kStPgs)
+                  : i == kStPrep    ? std::max(between(kStPrep, kStPrepEnd), between(kStPrep, kStPrepJointsEnd))
+                                    : between(int(i), int(i) + 1);
+        for (cudaEvent_t& e : ctx.ev) cudaEventDestroy(e);
         if (err) {
             restore();
             th_device_valid_ = false;

@@ -198,9 +198,10 @@ int fyzz_b200_collide(fyzz_b200_world* w);
 int fyzz_b200_synchronize(fyzz_b200_world* w);
 /* One step launched without the graph, with CUDA events on the world's
  * stream at each stage boundary.  stage_ms receives up to n stage times:
- * 0 bounds, 1 endpoint sort, 2 pairs, 3 narrowphase, 4 islands,
- * 5 partitions and row preparation (concurrent graph branches), 6 PGS,
- * 7 integration.  (Counterpart of the reference's
+ * 0 bounds, 1 endpoint sort, 2 pairs, 3 narrowphase, 4 islands and their
+ * partitions, 5 row preparation (on branches of its own beside the later part
+ * of stage 4, so its time is also in that one's), 6 PGS, 7 integration.
+ * (Counterpart of the reference's
  * Context::profile_batch_gpu_nanoseconds, compute.h:299.) */
 int fyzz_b200_profile_step(fyzz_b200_world* w, float seconds, float* stage_ms, uint32_t n);
 /* ---- performance parameters (no reference counterpart) ----
