@@ -2,13 +2,16 @@
 
 Islands of exactly n descriptors (towers of n touching cubes) around every
 class of the island solvers -- the groups of small ones, one CTA, a cluster
-of CTAs, global memory -- and chains of joints across the classes: partition
-levels exact, velocities and poses within 1e-4 (the step's tolerance).
+of CTAs, global memory -- with their partition levels exact, and chains of
+joints across the classes: velocities and poses within 1e-4 (the step's
+tolerance).
 Endpoint sorts around the widths of the one-CTA sort, long pair buckets
 under one body, and the split narrowphase of large pair budgets: exact.
 """
 import numpy as np
 import pytest
+
+from test_gpu_parity import oracle_levels
 
 pytestmark = pytest.mark.gpu
 
@@ -42,14 +45,15 @@ def check_step(pkg, oracle, spec):
     assert rel_err(ws[:, 3:6], os_[:, 3:6]) <= VEL_RTOL
     assert rel_err(ws[:, 10:13], os_[:, 10:13]) <= VEL_RTOL
     assert rel_err(ws[:, 0:3], os_[:, 0:3], floor=1.0) <= VEL_RTOL
-    return w
+    return w, o
 
 
 @pytest.mark.parametrize("sizes", [
     [1, 2, 3, 4, 5, 8, 9, 15, 16, 17, 31, 32, 33, 2, 1, 7], [63, 64, 65, 127, 128, 129, 1], [255, 256, 257],
     [511, 512, 513], [1023, 1024, 1025], [2047, 2048, 2049], [4095, 4096, 4097]])
 def test_islands_of_every_class(pkg, oracle, scenes, sizes):
-    w = check_step(pkg, oracle, towers(scenes, sizes))
+    w, o = check_step(pkg, oracle, towers(scenes, sizes))
+    np.testing.assert_array_equal(w.levels(), oracle_levels(o, 0))
     assert sorted(w.islands()[0].tolist()) == sorted(sizes)
 
 
