@@ -251,102 +251,37 @@ __device__ __forceinline__ void rel_adj(v3 n, v3 ra, v3 rb, v3 av, v3 aw, v3 bv,
     g.rb = vsub(g.rb, vmul(bw, gb));
 }
 
-// The 64-byte row records move as 256-bit accesses (sm_100): a lane's record
-// lies apart from its neighbours', so an access costs an L1 wavefront a lane
-// whatever its width.  In volatile assembly, so that a descriptor's loads
-// stay where they are issued and a sum's load behind the store before it.
-__device__ __forceinline__ void load256(const float4* p, float4* r) {
-    asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                 : "=f"(r[0].x), "=f"(r[0].y), "=f"(r[0].z), "=f"(r[0].w), "=f"(r[1].x), "=f"(r[1].y), "=f"(r[1].z),
-                   "=f"(r[1].w)
-                 : "l"(p));
+// Adds a row-gradient increment to its accumulator: reductions of 128 bits
+// without a reply.  One thread at a time owns a row (its descriptor's), so
+// the sum is that of a load, an add and a store, but no row waits for the
+// previous row's accumulator to come back.
+template <class T> __device__ __forceinline__ void add_row(T& dst, const T& inc) {
+    static_assert(sizeof(T) % 16 == 0 && alignof(T) == 16, "16-byte row record");
+    float4* d = reinterpret_cast<float4*>(&dst);
+    const float4* a = reinterpret_cast<const float4*>(&inc);
+#pragma unroll
+    for (int k = 0; k < int(sizeof(T) / 16); ++k)
+        asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(d + k), "f"(a[k].x), "f"(a[k].y),
+                     "f"(a[k].z), "f"(a[k].w)
+                     : "memory");
 }
-__device__ __forceinline__ void store256(float4* p, const float4* r) {
-    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(r[0].x), "f"(r[0].y),
-                 "f"(r[0].z), "f"(r[0].w), "f"(r[1].x), "f"(r[1].y), "f"(r[1].z), "f"(r[1].w));
-}
+// A row of the forward step (read-only here, so the loads of all a
+// manager's rows can be in flight before the first is used).
 template <class T> __device__ __forceinline__ T load_row(const T* row) {
     static_assert(sizeof(T) == 64 && alignof(T) == 16, "64-byte row record");
     T r;
-    load256(reinterpret_cast<const float4*>(row), reinterpret_cast<float4*>(&r));
-    load256(reinterpret_cast<const float4*>(row) + 2, reinterpret_cast<float4*>(&r) + 2);
+    const float4* s = reinterpret_cast<const float4*>(row);
+    float4* d = reinterpret_cast<float4*>(&r);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) d[k] = __ldg(s + k);
     return r;
 }
-__device__ __forceinline__ float4 add4(float4 a, float4 b) {
-    return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
-}
-// The sums of a descriptor's row gradients over the passes: four vectors of
-// each normal row (or of a joint's row), the first three of each friction row
-// and the manager's coefficients.  One thread at a time owns a descriptor.
-// Every sum is a plain add: reductions to global memory (red.add), which need
-// no load, flush subnormals.
-constexpr uint32_t kSumVecs = 4 * 4 + 4 * 3 + 1;
-__device__ __forceinline__ constexpr uint32_t sum_normal(int j) { return 4u * uint32_t(j); }
-__device__ __forceinline__ constexpr uint32_t sum_friction(int k) { return 16u + 3u * uint32_t(k); }
-constexpr uint32_t kSumHeader = 28;
-// In the sums' own arrays (islands beyond isl_warp descriptors).
-struct GlobalSums {
-    __device__ __forceinline__ float4* at(float4* global, uint32_t) const { return global; }
-    template <int N> __device__ __forceinline__ void load(const float4* p, float4 (&v)[N]) const {
-#pragma unroll
-        for (int k = 0; k + 1 < N; k += 2) load256(p + k, v + k);
-        if (N & 1) v[N - 1] = p[N - 1];
-    }
-    template <int N> __device__ __forceinline__ void add(float4* p, const float4 (&v)[N], const float4* inc) const {
-        float4 r[N];
-#pragma unroll
-        for (int k = 0; k < N; ++k) r[k] = add4(v[k], inc[k]);
-#pragma unroll
-        for (int k = 0; k + 1 < N; k += 2) store256(p + k, r + k);
-        if (N & 1) p[N - 1] = r[N - 1];
-    }
-};
-// In shared memory, `stride` vectors apart, until publish: a row's sum is
-// then never waited for, and leaves once instead of with every pass.  The two
-// sweeps of the 1,024 x 64 boxes rollout take 234 + 219 us a step, with the
-// sums in global memory 238 + 287; the flushing reductions took 193 + 242.
-struct SharedSums {
-    float4* mine;
-    uint32_t stride;
-    bool fresh;   // the first pass: nothing summed yet
-    __device__ __forceinline__ float4* at(float4*, uint32_t q) const { return mine + q * stride; }
-    template <int N> __device__ __forceinline__ void load(const float4* p, float4 (&v)[N]) const {
-#pragma unroll
-        for (int k = 0; k < N; ++k) v[k] = fresh ? make_float4(0, 0, 0, 0) : p[k * stride];
-    }
-    template <int N> __device__ __forceinline__ void add(float4* p, const float4 (&v)[N], const float4* inc) const {
-#pragma unroll
-        for (int k = 0; k < N; ++k) p[k * stride] = add4(v[k], inc[k]);
-    }
-    // The sums of descriptor d to their arrays (cleared before the sweep).
-    __device__ __forceinline__ void publish(const DevState& s, const AdjState& A, uint32_t d) const {
-        const auto put = [&](void* row, uint32_t q, int n) {
-            float4 v[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) v[k] = k < n ? mine[(q + k) * stride] : make_float4(0, 0, 0, 0);
-            store256(static_cast<float4*>(row), v);
-            store256(static_cast<float4*>(row) + 2, v + 2);
-        };
-        if (d < s.n_joints) {
-            put(A.jrow + d, 0, 4);
-            return;
-        }
-        const uint32_t m = d - s.n_joints;
-        const ManagerHeader hd = s.mh[m];
-        for (int j = 0; j < int(hd.count); ++j) put(A.nrow + 4 * size_t(m) + j, sum_normal(j), 4);
-        for (int k = 0; k < int(2 * hd.anchors); ++k) put(A.frow + 4 * size_t(m) + k, sum_friction(k), 3);
-        A.hd[m] = mine[kSumHeader * stride];
-    }
-};
-template <class R, class S>
+template <class R>
 __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, uint32_t lid, int it, int pos,
-                             const R& D, const S& sums) {
+                             const R& D) {
     const size_t cap = s.pair_cap;
     if (d < s.n_joints) {
         const JointRow r = s.jrow[d];
-        float4* const at = sums.at(reinterpret_cast<float4*>(A.jrow + d), 0u);
-        float4 sum[4];
-        sums.load(at, sum);
         int32_t b0, b1;
         if constexpr (R::kLocal) {
             b0 = local_handle(lid & 0xffffu); b1 = local_handle(lid >> 16);
@@ -373,7 +308,7 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
         o.ima = g.ima; o.imb = g.imb;
         o.vel_mult = nd * ynb;
         if (it < pos) o.constant = ynb; else o.unbiased = ynb;
-        sums.add(at, sum, reinterpret_cast<const float4*>(&o));
+        add_row(A.jrow[d], o);
         A.yj[d] = ynb - dlb;
         D.store(b0, av, aw, avb, awb);
         D.store(b1, bv, bw, bvb, bwb);
@@ -414,9 +349,6 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
     float yv[4] = {y4.x, y4.y, y4.z, y4.w};
     RowAdj hg = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, 0.0f, 0.0f};
     float nsumb = 0.0f, dfb = 0.0f;
-    float4* const hat = sums.at(A.hd + m, kSumHeader);
-    float4 hsum[1];
-    sums.load(hat, hsum);
     const float4 yo4 = it > 0 ? tn4[slot - cap] : zero4;
     if (friction) {
         const bool prev_friction = it > 0 && (it - 1 >= pos || pos - (it - 1) <= 3);
@@ -435,9 +367,6 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
         for (int k = 3; k >= 0; --k) {
             if (k >= int(2 * hd.anchors)) continue;
             const FrictionRow& f = frow[k];
-            float4* const at = sums.at(reinterpret_cast<float4*>(A.frow + 4 * size_t(m) + k), sum_friction(k));
-            float4 sum[3];
-            sums.load(at, sum);
             const v3 t = lv(f.t), ra = lv(f.ra), rb = lv(f.rb);
             const float xn = xt[k];
             const float xo = xto[k];
@@ -465,7 +394,7 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
             o.t[0] = g.n.x; o.t[1] = g.n.y; o.t[2] = g.n.z;
             o.ra[0] = g.ra.x; o.ra[1] = g.ra.y; o.ra[2] = g.ra.z;
             o.rb[0] = g.rb.x; o.rb[1] = g.rb.y; o.rb[2] = g.rb.z;
-            sums.add(at, sum, reinterpret_cast<const float4*>(&o));
+            add_row(A.frow[4 * size_t(m) + k], o);
             hg.ima += g.ima; hg.imb += g.imb;
             fv[k] = xob;
         }
@@ -478,9 +407,6 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
     for (int j = 3; j >= 0; --j) {
         if (j >= int(hd.count)) continue;
         const NormalRow& r = nrow[j];
-        float4* const at = sums.at(reinterpret_cast<float4*>(A.nrow + 4 * size_t(m) + j), sum_normal(j));
-        float4 sum[4];
-        sums.load(at, sum);
         const v3 n = lv(r.n), ra = lv(r.ra), rb = lv(r.rb);
         const float yn = tn[j];
         const float yo = tno[j];
@@ -501,13 +427,14 @@ __device__ void reverse_desc(const DevState& s, const AdjState& A, uint32_t d, u
         o.n[0] = g.n.x; o.n[1] = g.n.y; o.n[2] = g.n.z;
         o.ra[0] = g.ra.x; o.ra[1] = g.ra.y; o.ra[2] = g.ra.z;
         o.rb[0] = g.rb.x; o.rb[1] = g.rb.y; o.rb[2] = g.rb.z;
-        sums.add(at, sum, reinterpret_cast<const float4*>(&o));
+        add_row(A.nrow[4 * size_t(m) + j], o);
         hg.ima += g.ima; hg.imb += g.imb;
         yv[j] = yob;
     }
     reinterpret_cast<float4*>(A.yn)[m] = make_float4(yv[0], yv[1], yv[2], yv[3]);
-    const float4 hinc = make_float4(hg.ima, hg.imb, 0.0f, dfb);
-    sums.add(hat, hsum, &hinc);
+    asm volatile("red.relaxed.gpu.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(A.hd + m), "f"(hg.ima), "f"(hg.imb),
+                 "f"(0.0f), "f"(dfb)
+                 : "memory");
     D.store(h0, av, aw, avb, awb);
     D.store(h1, bv, bw, bvb, bwb);
 }
@@ -537,19 +464,17 @@ constexpr uint32_t kRevWarps = 4;
 // Islands of at most kRevSmall descriptors, several to a warp: an island of
 // (2^(c-1), 2^c] descriptors (the forward's list kSmallList + c) takes 2^c
 // lanes, one descriptor each, and the warp steps through its islands' levels
-// together, in reverse.  One thread an island of up to 8 (its descriptors one
-// after another, each a few round trips to memory) and one warp an island of
-// up to 96 (most lanes idle) took 276 + 462 us a step of the 1,024 x 64 boxes
-// rollout; this and the next take 234 + 219, side by side.
+// together, in reverse.  One thread an island of up to 8 took 198 us a step
+// (its descriptors one after another, each a few round trips to memory), one
+// warp an island of up to 96 328 us (most lanes idle).  In the 1,024 x 64
+// boxes rollout the two classes' kernels took 462 + 276 us a step; now 244 +
+// 195, side by side.
 constexpr uint32_t kRevSmall = 32;
-constexpr uint32_t kPackedVecs = 4 * 2 * 32 + kSumVecs * 32;   // shared memory of a warp
 __global__ void __launch_bounds__(kRevWarps * 32) k_adj_pgs_packed(DevState s, AdjState A, const uint32_t* lvl_bound) {
-    extern __shared__ float4 shp[];
+    __shared__ float4 sh[kRevWarps][4 * 2 * 32];
     const uint32_t lane = threadIdx.x & 31u, wib = threadIdx.x >> 5;
     const int pos = s.pos_iters, vel = s.vel_iters < 1 ? 1 : s.vel_iters;
-    float4* const deltas = shp + wib * kPackedVecs;   // 64 bodies, then 32 descriptors' sums
-    const RevLocal D{deltas};
-    SharedSums sums{deltas + 4 * 2 * 32 + lane, 32u, true};
+    const RevLocal D{sh[wib]};
     uint32_t units[DevState::kSmallClasses], total = 0;   // warps' worth of islands per class
 #pragma unroll
     for (int c = 0; c < DevState::kSmallClasses; ++c) {
@@ -574,7 +499,7 @@ __global__ void __launch_bounds__(kRevWarps * 32) k_adj_pgs_packed(DevState s, A
             nb = s.isl_nbod[isl];
         }
         const int32_t* ib = s.isl_bod + begin + isl;
-        float4* my = deltas + 4 * (sub * 2u * g);   // g + 1 bodies at most
+        float4* my = sh[wib] + 4 * (sub * 2u * g);   // g + 1 bodies at most
         for (uint32_t l = i; l < nb; l += g) {
             const int32_t b = ib[l];
             my[4 * l] = s.sb_dv[b]; my[4 * l + 1] = s.sb_dw[b];
@@ -606,69 +531,54 @@ __global__ void __launch_bounds__(kRevWarps * 32) k_adj_pgs_packed(DevState s, A
                 __syncwarp();
             }
             for (int l = levels - 1; l >= 0; --l) {
-                if (level == l) reverse_desc(s, A, d, lid, it, pos, D, sums);
+                if (level == l) reverse_desc(s, A, d, lid, it, pos, D);
                 __syncwarp();
             }
-            sums.fresh = false;
         }
-        sums.fresh = true;
-        if (i < n) sums.publish(s, A, d);
         __syncwarp();
     }
 }
 
-// One warp (and CTA) per island of (kRevSmall, isl_warp] descriptors, from
-// the forward's lists of (32, 64] and (64, 128].
-constexpr uint32_t kRevWarpVecs = 4 * (kSmallIsland + 1) + kSumVecs * kSmallIsland;
-__global__ void __launch_bounds__(32) k_adj_pgs_warp_smem(DevState s, AdjState A, const uint32_t* lvl_bound) {
-    extern __shared__ float4 shw[];
-    constexpr int kLists = 2;
-    const int lists[kLists] = {pgs_list(kSmallIsland), pgs_list(kRevSmall + 1)};   // the longer chains first
-    const uint32_t lane = threadIdx.x;
+// One warp per island of (kRevSmall, isl_warp] descriptors.
+__global__ void __launch_bounds__(kRevWarps * 32) k_adj_pgs_warp_smem(DevState s, AdjState A,
+                                                                     const uint32_t* lvl_bound) {
+    __shared__ float4 sh[kRevWarps][4 * (kSmallIsland + 1)];
+    const uint32_t ni = *s.n_isl;
+    const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     const int pos = s.pos_iters, vel = s.vel_iters < 1 ? 1 : s.vel_iters;
-    const RevLocal D{shw};
-    const uint32_t n0 = s.counters[list_counter(lists[0])], total = n0 + s.counters[list_counter(lists[1])];
-    for (uint32_t k = blockIdx.x; k < total; k += gridDim.x) {
-        const uint32_t isl = k < n0 ? s.isl_list[lists[0]][k] : s.isl_list[lists[1]][k - n0];
-        const uint32_t begin = s.isl_begin[isl], n = s.isl_begin[isl + 1] - begin;
-        if (n > s.isl_warp) continue;
+    const RevLocal D{sh[wib]};
+    for (uint32_t isl = warp; isl < ni; isl += nwarps) {
+        const uint32_t begin = s.isl_begin[isl], end = s.isl_begin[isl + 1];
+        if (end - begin > s.isl_warp || end - begin <= kRevSmall) continue;
         const uint32_t nlev = s.isl_end[isl];
         const uint32_t nb = s.isl_nbod[isl];
         const int32_t* ib = s.isl_bod + begin + isl;
         const uint32_t* bound = lvl_bound + begin + isl;
         for (uint32_t l = lane; l < nb; l += 32) {
             const int32_t g = ib[l];
-            shw[4 * l] = s.sb_dv[g]; shw[4 * l + 1] = s.sb_dw[g];
-            shw[4 * l + 2] = A.dv[g]; shw[4 * l + 3] = A.dw[g];
+            sh[wib][4 * l] = s.sb_dv[g]; sh[wib][4 * l + 1] = s.sb_dw[g];
+            sh[wib][4 * l + 2] = A.dv[g]; sh[wib][4 * l + 3] = A.dw[g];
         }
         __syncwarp();
-        SharedSums sums{shw + 4 * (kSmallIsland + 1), kSmallIsland, true};
-        float4* const first = sums.mine;
         for (int it = pos + vel - 1; it >= 0; --it) {
             if (it == pos - 1) {
                 for (uint32_t l = lane; l < nb; l += 32) {
                     const int32_t g = ib[l];
-                    float4 v = shw[4 * l + 2], w = shw[4 * l + 3];
+                    float4 v = sh[wib][4 * l + 2], w = sh[wib][4 * l + 3];
                     const float4 mv = A.dvm[g], mw = A.dwm[g];
                     v.x += mv.x; v.y += mv.y; v.z += mv.z;
                     w.x += mw.x; w.y += mw.y; w.z += mw.z;
-                    shw[4 * l + 2] = v; shw[4 * l + 3] = w;
+                    sh[wib][4 * l + 2] = v; sh[wib][4 * l + 3] = w;
                 }
                 __syncwarp();
             }
             for (int l = int(nlev) - 1; l >= 0; --l) {
                 const uint32_t lb = bound[l], le = bound[l + 1];
-                for (uint32_t i = lb + lane; i < le; i += 32) {
-                    sums.mine = first + (i - begin);
-                    reverse_desc(s, A, s.d_val2[i], s.d_lbod[i], it, pos, D, sums);
-                }
+                for (uint32_t i = lb + lane; i < le; i += 32) reverse_desc(s, A, s.d_val2[i], s.d_lbod[i], it, pos, D);
                 __syncwarp();
             }
-            sums.fresh = false;
-        }
-        for (uint32_t i = lane; i < n; i += 32) {
-            sums.mine = first + i;
-            sums.publish(s, A, s.d_val2[begin + i]);
         }
         __syncwarp();
     }
@@ -709,7 +619,7 @@ __global__ void __launch_bounds__(128) k_adj_pgs_mid_smem(DevState s, AdjState A
             for (int l = int(nlev) - 1; l >= 0; --l) {
                 const uint32_t lb = bound[l], le = bound[l + 1];
                 for (uint32_t i = lb + threadIdx.x; i < le; i += blockDim.x)
-                    reverse_desc(s, A, s.d_val2[i], s.d_lbod[i], it, pos, D, GlobalSums{});
+                    reverse_desc(s, A, s.d_val2[i], s.d_lbod[i], it, pos, D);
                 __syncthreads();
             }
         }
@@ -736,7 +646,7 @@ __global__ void __launch_bounds__(256) k_adj_pgs_block(DevState s, AdjState A, c
             for (int l = int(nlev) - 1; l >= 0; --l) {
                 const uint32_t lb = bound[l], le = bound[l + 1];
                 for (uint32_t i = lb + threadIdx.x; i < le; i += blockDim.x)
-                    reverse_desc(s, A, s.d_val2[i], 0u, it, pos, RevGlobal{A}, GlobalSums{});
+                    reverse_desc(s, A, s.d_val2[i], 0u, it, pos, RevGlobal{A});
                 __syncthreads();
             }
         }
@@ -1153,13 +1063,6 @@ __global__ void k_mass_frames(DevState s, float* out) {
 
 }  // namespace
 
-void init_adjoint_kernels() {
-    cudaFuncSetAttribute(k_adj_pgs_packed, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(kRevWarps * kPackedVecs * sizeof(float4)));
-    cudaFuncSetAttribute(k_adj_pgs_warp_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(kRevWarpVecs * sizeof(float4)));
-}
-
 void enqueue_adjoint_save_start(const DevState& s, const AdjState& a, cudaStream_t st) {
     k_adj_save_start<<<grid_n(s.n_bodies, 256, 1u << 30), 256, 0, st>>>(s, a);
 }
@@ -1189,10 +1092,9 @@ void enqueue_adjoint_step(const DevState& s, const AdjState& a, cudaStream_t st,
     k_adj_integrate<<<grid_n(s.n_bodies, T, 1u << 30), T, 0, st>>>(s, a);
     fork_branches(br, st, 3);
     auto side = [&](int i) { return br ? br->st[i] : st; };
-    k_adj_pgs_warp_smem<<<grid_n(s.desc_cap, kRevSmall + 1, 148u * 4u), 32, kRevWarpVecs * sizeof(float4), st>>>(
+    k_adj_pgs_warp_smem<<<grid_n(s.desc_cap * 32u, kRevWarps * 32u, 148u * 8u), kRevWarps * 32u, 0, st>>>(
         s, a, s.lvl_bound);
-    k_adj_pgs_packed<<<grid_n(s.desc_cap, kRevWarps, 148u * 4u), kRevWarps * 32u,
-                       kRevWarps * kPackedVecs * sizeof(float4), side(0)>>>(s, a, s.lvl_bound);
+    k_adj_pgs_packed<<<grid_n(s.desc_cap, kRevWarps, 148u * 4u), kRevWarps * 32u, 0, side(0)>>>(s, a, s.lvl_bound);
     k_adj_pgs_mid_smem<<<grid_n(s.desc_cap, kSmallIsland + 1, 148u * 4u), 128,
                          4 * (kMidIsland + 1) * sizeof(float4), side(1)>>>(s, a, s.lvl_bound);
     k_adj_pgs_block<<<grid_n(s.desc_cap, 1, 148u * 4u), 256, 0, side(2)>>>(s, a, s.lvl_bound);

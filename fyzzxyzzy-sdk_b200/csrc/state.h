@@ -332,7 +332,6 @@ struct AdjState {
 // Copies the live pairs of a contact-manager generation.
 void enqueue_copy_set(const ManagerSet& dst, const ManagerSet& src, uint32_t cap, cudaStream_t st);
 // adjoint.cu
-void init_adjoint_kernels();
 // Host-buffer transfers, in device memory: dst[b] = (src[3b .. 3b+2], 0);
 // out = velocity gradients, angular gradients (3 floats a body each) and mass
 // gradients (1); out = mass-frame centres (3 a body), then orientations (4).

@@ -264,7 +264,6 @@ public:
         }
         check_cuda(cudaEventCreateWithFlags(&br_.fork, cudaEventDisableTiming), "cudaEventCreate");
         init_solver_kernels();
-        init_adjoint_kernels();
         check_cuda(cudaGetLastError(), "kernel attributes");
         check_cuda(cudaMallocHost(reinterpret_cast<void**>(&host_err_), 64), "cudaMallocHost");
         scene_body_begin_.push_back(0);
