@@ -253,8 +253,13 @@ __device__ __forceinline__ void rel_adj(v3 n, v3 ra, v3 rb, v3 av, v3 aw, v3 bv,
 
 // Adds a row-gradient increment to its accumulator: reductions of 128 bits
 // without a reply.  One thread at a time owns a row (its descriptor's), so
-// the sum is that of a load, an add and a store, but no row waits for the
-// previous row's accumulator to come back.
+// the sum is that of a load, an add and a store except that a reduction
+// flushes subnormals (k_adj_scale keeps the seeds far above them), but no row
+// waits for the previous row's accumulator to come back.  Loads and stores
+// instead took 331 + 284 us a step against 243 + 194 in the two largest sweeps
+// of the 1,024 x 64 boxes rollout, sums kept in shared memory 219 + 234 there
+// but 1,549 against 760 in the islands beyond 512 descriptors of the
+// 131,072-body pile, whose sums have no room there.
 template <class T> __device__ __forceinline__ void add_row(T& dst, const T& inc) {
     static_assert(sizeof(T) % 16 == 0 && alignof(T) == 16, "16-byte row record");
     float4* d = reinterpret_cast<float4*>(&dst);
@@ -464,11 +469,10 @@ constexpr uint32_t kRevWarps = 4;
 // Islands of at most kRevSmall descriptors, several to a warp: an island of
 // (2^(c-1), 2^c] descriptors (the forward's list kSmallList + c) takes 2^c
 // lanes, one descriptor each, and the warp steps through its islands' levels
-// together, in reverse.  One thread an island of up to 8 took 198 us a step
-// (its descriptors one after another, each a few round trips to memory), one
-// warp an island of up to 96 328 us (most lanes idle).  In the 1,024 x 64
-// boxes rollout the two classes' kernels took 462 + 276 us a step; now 244 +
-// 195, side by side.
+// together, in reverse.  One thread an island of up to 8 (its descriptors one
+// after another, each a few round trips to memory) and one warp an island of
+// up to 96 (most lanes idle) took 276 + 462 us a step of the 1,024 x 64 boxes
+// rollout; this and the next take 194 + 243, side by side.
 constexpr uint32_t kRevSmall = 32;
 __global__ void __launch_bounds__(kRevWarps * 32) k_adj_pgs_packed(DevState s, AdjState A, const uint32_t* lvl_bound) {
     __shared__ float4 sh[kRevWarps][4 * 2 * 32];
@@ -1037,18 +1041,51 @@ __global__ void k_adj_seed(float4* dst, const float* src, uint32_t n) {
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
     if (b < n) dst[b] = make_float4(src[3 * size_t(b)], src[3 * size_t(b) + 1], src[3 * size_t(b) + 2], 0.0f);
 }
+// The sweeps are linear in their seeds, and their sums are reductions, which
+// flush subnormals.  Seeds whose largest is below 2^-40 are therefore scaled
+// to it by a power of two, exactly, and the gradients back: seeds of 2^-100
+// gave velocity gradients 2.5e-6 off the unscaled ones without this (1.8e-8
+// with sums that do not flush, exact now).  Not further, to leave a long
+// rollout's growth its room.
+constexpr uint32_t kSeedFloor = (127u - 40u) << 23;   // bits of 2^-40
+__device__ __forceinline__ float seed_scale(uint32_t peak) {
+    return peak && peak < kSeedFloor ? ldexpf(1.0f, -40 - ilogbf(__uint_as_float(peak))) : 1.0f;
+}
+__global__ void k_adj_peak(AdjState A, uint32_t n) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t peak = 0;
+    if (b < n)
+        for (const float4 x : {A.c[b], A.q[b], A.v[b], A.w[b]})
+            for (const float f : {x.x, x.y, x.z, x.w}) peak = max(peak, __float_as_uint(f) & 0x7fffffffu);
+    peak = __reduce_max_sync(0xffffffffu, peak);
+    if ((threadIdx.x & 31u) == 0 && peak) atomicMax(A.peak, peak);
+}
+__global__ void k_adj_scale(AdjState A, uint32_t n) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    const float k = seed_scale(*A.peak);
+    if (b >= n || k == 1.0f) return;
+    for (float4* p : {A.c + b, A.q + b, A.v + b, A.w + b}) {
+        const float4 x = *p;
+        *p = make_float4(x.x * k, x.y * k, x.z * k, x.w * k);
+    }
+}
 // out: velocity and angular gradients (3 floats a body each), then the mass
-// gradients.  Inverse mass and inertia scale as 1 / m: dm = -im (im g_im +
+// gradients; the friction gradients in place.  All scaled back.  Inverse mass and inertia scale as 1 / m: dm = -im (im g_im +
 // iI . g_iI).
 __global__ void k_adj_results(DevState s, AdjState A, float* out) {
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    const float k = 1.0f / seed_scale(*A.peak);   // a power of two
+    if (b < s.n_shapes) {
+        A.g_fs[b] *= k;
+        A.g_fd[b] *= k;
+    }
     if (b >= s.n_bodies) return;
     const float4 v = A.v[b], w = A.w[b], gi = A.g_iI[b], inv = s.b_inv[b];
     float* o = out + 3 * size_t(b);
-    o[0] = v.x; o[1] = v.y; o[2] = v.z;
+    o[0] = v.x * k; o[1] = v.y * k; o[2] = v.z * k;
     o += 3 * size_t(s.n_bodies);
-    o[0] = w.x; o[1] = w.y; o[2] = w.z;
-    out[6 * size_t(s.n_bodies) + b] = -inv.w * (inv.w * A.g_im[b] + inv.x * gi.x + inv.y * gi.y + inv.z * gi.z);
+    o[0] = w.x * k; o[1] = w.y * k; o[2] = w.z * k;
+    out[6 * size_t(s.n_bodies) + b] = -inv.w * (inv.w * A.g_im[b] + inv.x * gi.x + inv.y * gi.y + inv.z * gi.z) * k;
 }
 __global__ void k_mass_frames(DevState s, float* out) {
     const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1070,8 +1107,14 @@ void enqueue_adjoint_save_start(const DevState& s, const AdjState& a, cudaStream
 void enqueue_adjoint_seed(float4* dst, const float* src, uint32_t n, cudaStream_t st) {
     if (n) k_adj_seed<<<grid_n(n, 256, 1u << 30), 256, 0, st>>>(dst, src, n);
 }
+void enqueue_adjoint_scale(const AdjState& a, uint32_t n, cudaStream_t st) {
+    if (!n) return;
+    k_adj_peak<<<grid_n(n, 256, 1u << 30), 256, 0, st>>>(a, n);
+    k_adj_scale<<<grid_n(n, 256, 1u << 30), 256, 0, st>>>(a, n);
+}
 void enqueue_adjoint_results(const DevState& s, const AdjState& a, float* out, cudaStream_t st) {
-    if (s.n_bodies) k_adj_results<<<grid_n(s.n_bodies, 256, 1u << 30), 256, 0, st>>>(s, a, out);
+    const uint32_t n = s.n_bodies > s.n_shapes ? s.n_bodies : s.n_shapes;
+    if (n) k_adj_results<<<grid_n(n, 256, 1u << 30), 256, 0, st>>>(s, a, out);
 }
 void enqueue_mass_frames(const DevState& s, float* out, cudaStream_t st) {
     if (s.n_bodies) k_mass_frames<<<grid_n(s.n_bodies, 256, 1u << 30), 256, 0, st>>>(s, out);

@@ -328,6 +328,7 @@ struct AdjState {
     float *yn = nullptr, *yf = nullptr, *yj = nullptr;   // applied-impulse adjoints
     uint32_t* mark = nullptr;                     // per body: last step it was visited
     uint32_t* epoch = nullptr;                    // step counter of the reverse pass
+    uint32_t* peak = nullptr;                     // bits of the largest seed's magnitude
 };
 // Copies the live pairs of a contact-manager generation.
 void enqueue_copy_set(const ManagerSet& dst, const ManagerSet& src, uint32_t cap, cudaStream_t st);
@@ -338,6 +339,9 @@ void enqueue_copy_set(const ManagerSet& dst, const ManagerSet& src, uint32_t cap
 void enqueue_adjoint_seed(float4* dst, const float* src, uint32_t n, cudaStream_t st);
 void enqueue_adjoint_results(const DevState& s, const AdjState& a, float* out, cudaStream_t st);
 void enqueue_mass_frames(const DevState& s, float* out, cudaStream_t st);
+// Lifts small seeds clear of the subnormals (a.peak must be zero);
+// enqueue_adjoint_results scales the gradients back.
+void enqueue_adjoint_scale(const AdjState& a, uint32_t n, cudaStream_t st);
 void enqueue_adjoint_save_start(const DevState& s, const AdjState& a, cudaStream_t st);
 void enqueue_adjoint_step(const DevState& s, const AdjState& a, cudaStream_t st, const Branches* br = nullptr);
 

@@ -1066,7 +1066,7 @@ public:
         dalloc(A.yn, 4 * cap, roll_owned_); dalloc(A.yf, 4 * cap, roll_owned_);
         dalloc(A.yj, std::max<size_t>(d_.n_jrows, 1), roll_owned_);
         dalloc(A.mark, nb, roll_owned_);
-        dalloc(A.epoch, 1, roll_owned_);
+        dalloc(A.epoch, 1, roll_owned_); dalloc(A.peak, 1, roll_owned_);
         check_cuda(cudaMemsetAsync(A.mark, 0, nb * 4, stream_), "memset");
         check_cuda(cudaMemsetAsync(A.epoch, 0, 4, stream_), "memset");
         check_cuda(cudaStreamSynchronize(stream_), "sync");
@@ -1177,6 +1177,9 @@ public:
         up3(adj_.c, gc); up3(adj_.v, gv); up3(adj_.w, gw);
         if (gq) check_cuda(cudaMemcpyAsync(adj_.q, gq, size_t(nb) * 16, cudaMemcpyHostToDevice, stream_), "seed");
         else check_cuda(cudaMemsetAsync(adj_.q, 0, size_t(nb) * 16, stream_), "memset");
+        check_cuda(cudaMemsetAsync(adj_.peak, 0, 4, stream_), "memset");
+        enqueue_adjoint_scale(adj_, nb, stream_);
+        check_cuda(cudaGetLastError(), "seed scale");
         // the caller's buffers are free again on return even if a copy is
         // still under way when the sweeps are launched
         check_cuda(cudaStreamSynchronize(stream_), "seed sync");
