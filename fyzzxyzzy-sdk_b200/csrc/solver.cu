@@ -1361,10 +1361,12 @@ __global__ void __launch_bounds__(128, 4) k_prep_contacts(DevState s) {
 }
 
 // ---------------- PGS ----------------
-// Velocity deltas of the solver bodies in global memory, addressed by body
-// (islands beyond kBigIsland descriptors).  Handle -1 is the static world
-// (zero delta, never written).
+// Velocity deltas of the solver bodies for the solvers that read their rows
+// from global memory: there too, addressed by body (islands beyond kBigIsland
+// descriptors), or in shared memory by the island's local body.  Handle -1 is
+// the static world (zero delta, never written).
 struct GlobalDeltas {
+    static constexpr bool kLocal = false;
     const DevState& s;
     __device__ __forceinline__ void load(int32_t b, v3& dv, v3& dw) const {
         if (b < 0) { dv = dw = {0, 0, 0}; return; }
@@ -1377,6 +1379,28 @@ struct GlobalDeltas {
         s.sb_dw[b] = st4(dw, 0.0f);
     }
 };
+struct LocalDeltas {
+    static constexpr bool kLocal = true;
+    float4 *v, *w;
+    __device__ __forceinline__ void load(int32_t l, v3& dv, v3& dw) const {
+        if (l < 0) { dv = dw = {0, 0, 0}; return; }
+        dv = ld3(v[l]);
+        dw = ld3(w[l]);
+    }
+    __device__ __forceinline__ void store(int32_t l, v3 dv, v3 dw) const {
+        if (l < 0) return;
+        v[l] = st4(dv, 0.0f);
+        w[l] = st4(dw, 0.0f);
+    }
+};
+// Slot word: local bodies in bits 0-12 and 13-25 (0x1fff: the static
+// world), contact points or joint rows in bits 26-28, anchors in bits
+// 29-30, bit 31 a joint.
+constexpr uint32_t kNoBody = 0x1fffu;
+__device__ __forceinline__ uint32_t slot_word(uint32_t la, uint32_t lb, uint32_t count, uint32_t anchors, bool joint) {
+    return (la & kNoBody) | ((lb & kNoBody) << 13) | (count << 26) | (anchors << 29) | (joint ? 1u << 31 : 0u);
+}
+__device__ __forceinline__ int32_t word_body(uint32_t bits) { return (bits & kNoBody) == kNoBody ? -1 : int32_t(bits & kNoBody); }
 // 32 bytes per thread in one load (sm_100's 256-bit global loads): a solver
 // row is two loads instead of four 128-bit ones.  Scattered rows (one
 // manager per thread) cost one L1 wavefront per thread and load instruction,
@@ -1393,8 +1417,9 @@ __device__ __forceinline__ void ldg256(const void* p, float4& a, float4& b) {
 
 // A joint's rows in order (scene.cpp:8905-8945) between bodies b0 / b1
 // (-1: the static world).
+template <class D>
 __device__ __forceinline__ void solve_joint(const DevState& s, uint32_t d, int32_t b0, int32_t b1, int it, int pos,
-                                            const GlobalDeltas& D_) {
+                                            const D& D_) {
     v3 av, aw, bv, bw;
     D_.load(b0, av, aw);
     D_.load(b1, bv, bw);
@@ -1420,12 +1445,16 @@ __device__ __forceinline__ void solve_joint(const DevState& s, uint32_t d, int32
 }
 
 // One descriptor's rows for pass `it` (scene.cpp:8853-9148), read from the
-// per-manager arrays prep writes (islands beyond kBigIsland descriptors).
-__device__ void solve_desc(const DevState& s, uint32_t d, int it, int pos, int vel, const GlobalDeltas& D_) {
+// per-manager arrays prep writes.  word: its slot word, where D addresses
+// shared memory.
+template <class D>
+__device__ void solve_desc(const DevState& s, uint32_t d, uint32_t word, int it, int pos, int vel, const D& D_) {
     if (d < s.n_joints) {
-        const int32_t b0 = is_dyn(s, s.j_a[d]) ? int32_t(s.j_a[d]) : -1;
-        const int32_t b1 = is_dyn(s, s.j_b[d]) ? int32_t(s.j_b[d]) : -1;
-        solve_joint(s, d, b0, b1, it, pos, D_);
+        if constexpr (D::kLocal)
+            solve_joint(s, d, word_body(word), word_body(word >> 13), it, pos, D_);
+        else
+            solve_joint(s, d, is_dyn(s, s.j_a[d]) ? int32_t(s.j_a[d]) : -1, is_dyn(s, s.j_b[d]) ? int32_t(s.j_b[d]) : -1,
+                        it, pos, D_);
         return;
     }
     const uint32_t m = d - s.n_joints;
@@ -1448,22 +1477,25 @@ __device__ void solve_desc(const DevState& s, uint32_t d, int it, int pos, int v
     const float4* fq = reinterpret_cast<const float4*>(s.frow + 4 * size_t(m));
     float4 n0[4], n1[4], n2[4], n3[4], f0[4], f1[4], f2[4];
     float fa[4];
-    // All four row slots of the manager are read without waiting for the
-    // header (unused slots are never consumed), so the row loads and the
-    // header load are in flight together.
+    // The rows are read without waiting for the header, so that their loads
+    // and the header's are in flight together: those the slot word counts, or
+    // all four slots (unused ones are never consumed).
     const bool friction_pass = it >= pos || pos - it <= 3;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-        ldg256(nr + 4 * j, n0[j], n1[j]);
-        ldg256(nr + 4 * j + 2, n2[j], n3[j]);
-        if (friction_pass) {
+        if (!D::kLocal || uint32_t(j) < ((word >> 26) & 7u)) {
+            ldg256(nr + 4 * j, n0[j], n1[j]);
+            ldg256(nr + 4 * j + 2, n2[j], n3[j]);
+        }
+        if (friction_pass && (!D::kLocal || uint32_t(j) < 2u * ((word >> 29) & 3u))) {
             float4 f3;
             ldg256(fq + 4 * j, f0[j], f1[j]);
             ldg256(fq + 4 * j + 2, f2[j], f3);
             fa[j] = f3.x;
         }
     }
-    const int32_t h0 = hd.b0, h1 = hd.b1;
+    const int32_t h0 = D::kLocal ? word_body(word) : hd.b0;
+    const int32_t h1 = D::kLocal ? word_body(word >> 13) : hd.b1;
     v3 av, aw, bv, bw;
     D_.load(h0, av, aw);
     D_.load(h1, bv, bw);
@@ -1603,14 +1635,6 @@ __device__ __forceinline__ uint64_t dot2(const Pairs& j, const Pairs& v, uint64_
 __device__ __forceinline__ Pairs axpy2(const Pairs& v, const Pairs& j, uint64_t k, uint64_t nz) {
     return {add2(v.x, mul2(j.x, k, nz)), add2(v.y, mul2(j.y, k, nz)), add2(v.z, mul2(j.z, k, nz))};
 }
-// Slot word: local bodies in bits 0-12 and 13-25 (0x1fff: the static
-// world), contact points or joint rows in bits 26-28, anchors in bits
-// 29-30, bit 31 a joint.
-constexpr uint32_t kNoBody = 0x1fffu;
-__device__ __forceinline__ uint32_t slot_word(uint32_t la, uint32_t lb, uint32_t count, uint32_t anchors, bool joint) {
-    return (la & kNoBody) | ((lb & kNoBody) << 13) | (count << 26) | (anchors << 29) | (joint ? 1u << 31 : 0u);
-}
-
 // Shared memory of a unit of at most CAP descriptors and NBOD bodies a CTA
 // on a cluster of CL CTAs (slot i on CTA i % CL, body l on CTA l % CL).
 template <uint32_t CAP, uint32_t NBOD, uint32_t NT, uint32_t CL> struct Unit {
@@ -1923,6 +1947,24 @@ template <uint32_t CAP, uint32_t NBOD, uint32_t NT, uint32_t CL> struct Unit {
     }
 };
 
+// The cluster classes hold their islands' rows in the shared memory of eight
+// SMs' worth of CTAs, so only 18, 37 or 74 of their islands are on the chip at
+// once.  Beyond half as many again they would go in waves, and k_pgs_crowd,
+// with its rows in global memory and an island a CTA, is the faster form; if
+// one class is that crowded all three take it, since clusters beside it starve.
+// Scenes of one heap each, a step with clusters / crowded: 48 x 1,000 boxes
+// (islands up to 2,048) 731 / 779 us, 64 906 / 861, 256 2,640 / 1,915; 24 x 1,500
+// (up to 4,096) 769 / 860, 32 957 / 958, 256 5,502 / 3,190; 64 x 500 (up to 1,024)
+// 490 / 527, 96 611 / 595, 256 1,218 / 926.
+template <uint32_t CAP, uint32_t NT> constexpr uint32_t kCrowdLimit =
+    148u * uint32_t(232448u / Unit<CAP, CAP + 1, NT, 8>::kBytes) / 8u * 3u / 2u;
+static_assert(pgs_list(1024) == 8 && pgs_list(2048) == 9 && pgs_list(4096) == 10, "lists of the cluster classes");
+__device__ __forceinline__ bool crowded(const DevState& s) {
+    return s.crowds && (s.counters[list_counter(8)] > kCrowdLimit<128, 32> ||
+                        s.counters[list_counter(9)] > kCrowdLimit<256, 64> ||
+                        s.counters[list_counter(10)] > kCrowdLimit<512, 128>);
+}
+
 // One island of a size class of at most CAP x CL descriptors (n descriptors
 // have n + 1 bodies at most) on a CTA, or on a cluster of CL CTAs sharing
 // the deltas through distributed shared memory.
@@ -1931,6 +1973,7 @@ __global__ void __launch_bounds__(NT) k_pgs_island(DevState s, int list_class) {
     extern __shared__ float4 shb[];
     const Unit<CAP, CAP + 1, NT, CL> U(shb);
     const uint32_t n_list = s.counters[list_counter(list_class)];
+    if (CL > 1 && crowded(s)) return;   // k_pgs_crowd takes them
     const uint32_t* list = s.isl_list[list_class];
     const uint32_t rank = CL == 1 ? 0u : blockIdx.x % CL;
     for (uint32_t k = blockIdx.x / CL; k < n_list; k += gridDim.x / CL) {
@@ -2054,6 +2097,65 @@ template <class F> void for_island_solvers(F f) {
     f(k_pgs_island<64, 64, 1>, 64u, 1u, Unit<64, 65, 64, 1>::kBytes, 4);
 }
 
+// The islands of a crowded cluster class (at most MAXN descriptors), one CTA
+// each: deltas, descriptors and slot words in shared memory, rows in global
+// memory, where each of the five passes reads them again.
+template <uint32_t MAXN> constexpr size_t crowd_smem() {
+    return (MAXN + 1) * 2 * sizeof(float4) + (2 * MAXN + kMaxLevels + 1) * 4;
+}
+template <uint32_t MAXN, uint32_t NT>
+__global__ void __launch_bounds__(NT) k_pgs_crowd(DevState s, int list_class) {
+    extern __shared__ float4 shb[];
+    const LocalDeltas D{shb, shb + (MAXN + 1)};
+    uint32_t* desc = reinterpret_cast<uint32_t*>(shb + 2 * (MAXN + 1));
+    uint32_t *word = desc + MAXN, *level = word + MAXN;
+    if (!crowded(s)) return;
+    const uint32_t n_list = s.counters[list_counter(list_class)];
+    const int pos = s.pos_iters, vel = s.vel_iters < 1 ? 1 : s.vel_iters;
+    for (uint32_t k = blockIdx.x; k < n_list; k += gridDim.x) {
+        const uint32_t isl = s.isl_list[list_class][k], begin = s.isl_begin[isl], n = s.isl_begin[isl + 1] - begin;
+        const uint32_t nlev = s.isl_end[isl], nb = s.isl_nbod[isl];
+        const int32_t* ib = s.isl_bod + begin + isl;
+        for (uint32_t l = threadIdx.x; l < nb; l += NT) D.v[l] = D.w[l] = make_float4(0, 0, 0, 0);
+        for (uint32_t l = threadIdx.x; l <= nlev; l += NT) level[l] = s.lvl_bound[begin + isl + l] - begin;
+        for (uint32_t i = threadIdx.x; i < n; i += NT) {
+            const uint32_t d = s.d_val2[begin + i], lid = s.d_lbod[begin + i];
+            const bool joint = d < s.n_joints;
+            uint32_t count = 0, anchors = 0;
+            if (!joint) {
+                const ManagerHeader& hd = s.mh[d - s.n_joints];
+                count = min(hd.count, 4u);
+                anchors = min(hd.anchors, 2u);
+            }
+            desc[i] = d;
+            word[i] = slot_word(lid, lid >> 16, count, anchors, joint);
+        }
+        __syncthreads();
+        for (int it = 0; it < pos + vel; ++it) {
+            for (uint32_t l = 0; l < nlev; ++l) {
+                for (uint32_t i = level[l] + threadIdx.x; i < level[l + 1]; i += NT)
+                    solve_desc(s, desc[i], word[i], it, pos, vel, D);
+                __syncthreads();
+            }
+            if (it + 1 != pos && it + 1 != pos + vel) continue;
+            const bool moved = it + 1 == pos;
+            for (uint32_t l = threadIdx.x; l < nb; l += NT) {
+                (moved ? s.sb_mdv : s.sb_dv)[ib[l]] = D.v[l];
+                (moved ? s.sb_mdw : s.sb_dw)[ib[l]] = D.w[l];
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// f(kernel, threads, shared memory, CTAs an SM, island list), largest first
+// like the cluster classes.
+template <class F> void for_crowd_solvers(F f) {
+    f(k_pgs_crowd<4096, 384>, 384u, crowd_smem<4096>(), 1u, 10);
+    f(k_pgs_crowd<2048, 192>, 192u, crowd_smem<2048>(), 2u, 9);
+    f(k_pgs_crowd<1024, 128>, 128u, crowd_smem<1024>(), 3u, 8);
+}
+
 // One CTA per island beyond kBigIsland descriptors: deltas in global memory.
 __global__ void __launch_bounds__(256) k_pgs_block(DevState s, const uint32_t* lvl_bound) {
     const uint32_t n_list = s.counters[kCntList + 3];
@@ -2068,7 +2170,7 @@ __global__ void __launch_bounds__(256) k_pgs_block(DevState s, const uint32_t* l
             for (uint32_t l = 0; l < nlev; ++l) {
                 const uint32_t lb = bound[l], le = bound[l + 1];
                 for (uint32_t i = lb + threadIdx.x; i < le; i += blockDim.x)
-                    solve_desc(s, s.d_val2[i], it, pos, vel, D);
+                    solve_desc(s, s.d_val2[i], 0u, it, pos, vel, D);
                 __syncthreads();
             }
             if (it + 1 == pos) {
@@ -2310,6 +2412,9 @@ void init_solver_kernels() {
     for_island_solvers([](auto kernel, uint32_t, uint32_t, size_t smem, int) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
     });
+    for_crowd_solvers([](auto kernel, uint32_t, size_t smem, uint32_t, int) {
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    });
     cudaFuncSetAttribute(k_pgs_group, cudaFuncAttributeMaxDynamicSharedMemorySize, int(GroupUnit::kBytes));
 }
 
@@ -2387,6 +2492,14 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     hook(kStPgs, st);
     fork_branches(br, st, Branches::kN);
     int branch = 0;
+    // A crowd's solvers come before the clusters': at the stage's start they
+    // find room to leave again at once (after them 10 to 18 us a step).
+    if (s.crowds)
+        for_crowd_solvers([&](auto kernel, uint32_t nt, size_t smem, uint32_t per_sm, int list) {
+            launch(kernel, grid_for(s.desc_cap, kListMinDesc[list] + 1, 148u * per_sm), nt, smem, 1u, g_high_priority,
+                   side(branch++), s, list);
+        });
+    branch = 0;
     for_island_solvers([&](auto kernel, uint32_t nt, uint32_t cl, size_t smem, int list) {
         const uint32_t islands = grid_for(s.desc_cap, kListMinDesc[list] + 1, 148u * uint32_t(232448u / smem) / cl);
         launch(kernel, islands * cl, nt, smem, cl, cl > 1 ? g_high_priority : 0, side(branch++), s, list);

@@ -42,6 +42,7 @@ struct DevState {
     uint32_t n_scenes = 0, n_bodies = 0, n_shapes = 0, n_finite = 0, n_joints = 0;
     uint32_t pair_cap = 0, desc_cap = 0;
     uint32_t pairs_expected = 0;   // live pairs the budget was made for
+    bool crowds = false;           // so many large islands are possible that the step carries k_pgs_crowd
     uint32_t max_small_scene = 2048;   // finite shapes sorted inside one CTA
     // Performance parameters (fyzz_b200_tuning_t; every choice gives the same
     // results): a rollout's reverse sweep solves islands of (32, isl_warp]

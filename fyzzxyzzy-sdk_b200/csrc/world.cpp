@@ -1797,6 +1797,11 @@ private:
         release_segment_graphs();
         d_.pair_cap = cap;
         d_.pairs_expected = expected ? expected : uint32_t(uint64_t(cap) * 3 / 10);
+        // dozens of scenes that may each hold an island of more than 512
+        // descriptors, or a world so large that one scene may hold dozens (the
+        // solver kernels for them cost 2 to 4 us a step where they idle)
+        const uint32_t scenes = std::max(d_.n_scenes, 1u);
+        d_.crowds = d_.pairs_expected >= 1000000u || (scenes > 27u && d_.pairs_expected / scenes >= 512u);
         d_.desc_cap = cap + d_.n_joints + kJointReserve;
         for (int k = 0; k < 2; ++k) {
             dalloc(sets_[k].key, cap, pair_owned_);
