@@ -2426,6 +2426,7 @@ void init_solver_kernels() {
     cudaFuncSetAttribute(k_pgs_group, cudaFuncAttributeMaxDynamicSharedMemorySize, int(GroupUnit::kBytes));
 }
 
+constexpr uint32_t kWidePrepPairs = 300000;   // live pairs; see enqueue_solver's row preparation
 void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, const Branches* br) {
     uint32_t* lvl_bound = s.lvl_bound;
     const uint32_t T = s.elem_block;   // elementwise kernels (at most 56 registers, no launch bounds)
@@ -2455,13 +2456,16 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     // and leave most of the device idle.  Contacts and joints one after the
     // other beside the partitions only: 300 mechanisms 846 us for four steps
     // against 778, 131,072-body pile 4,085 against 3,925, 4,096 scenes 8,870
-    // against 8,595.  Two CTAs an SM instead of eight, to leave the sort's CTAs
-    // room, are no faster (pile of 20,011 1,754 us against 1,756, 32,768 hulls
-    // 1,776 against 1,798 with runs 1 % apart) and slower in large worlds
-    // (131,072-body pile 4,005 against 3,925).
+    // against 8,595.  Below the pair count where preparation outlasts that chain
+    // it gets two CTAs an SM: at eight it is over sooner (32,768 hulls 28 us a
+    // step, with two 43), but its registers keep the sort's CTAs waiting, and
+    // four steps are longer: hulls 1,776 us against 1,745, 40,000 resting bodies
+    // 2,706 against 2,671, pile of 20,011 1,772 against 1,757 (runs of one side
+    // 0.2 % apart).  Above, two are too few (131,072-body pile 4,005 against 3,925).
+    const uint32_t prep_blocks = s.pairs_expected >= kWidePrepPairs ? cap_blocks : 148u * 2u;
     fork_branches(br, st, 2);
     hook(kStPrep, side(0));
-    k_prep_contacts<<<grid_for(s.desc_cap, 128, cap_blocks), 128, 0, side(0)>>>(s);
+    k_prep_contacts<<<grid_for(s.desc_cap, 128, prep_blocks), 128, 0, side(0)>>>(s);
     hook(kStPrepEnd, side(0));
     if (s.n_joints) {
         k_prep_joints<<<grid_for(s.n_joints, 128, 1u << 30), 128, 0, side(1)>>>(s);   // ~150 registers
