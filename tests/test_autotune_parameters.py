@@ -46,3 +46,14 @@ def test_each_parameter_follows_its_own_timing(monkeypatch, tmp_path):
                 lambda p: 0.9 if p["island_cta"] == 256 else 1.0)
     want = dict(DEFAULTS, elem_block=512, island_cta=256)
     assert got == {"large_scene": want, "many_scenes": want}
+
+
+def test_a_lead_that_does_not_repeat_is_noise(monkeypatch, tmp_path):
+    seen = []
+
+    def once_fast(p):
+        first = p["radix_bits"] == 9 and seen.count(9) < 2
+        seen.append(p["radix_bits"])
+        return 0.9 if first else 1.0
+    got = table(monkeypatch, tmp_path, once_fast, lambda p: 1.0)
+    assert got == {"large_scene": DEFAULTS, "many_scenes": DEFAULTS}
