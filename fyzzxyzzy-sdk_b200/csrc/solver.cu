@@ -1400,14 +1400,16 @@ constexpr uint32_t kNoBody = 0x1fffu;
 __device__ __forceinline__ uint32_t slot_word(uint32_t la, uint32_t lb, uint32_t count, uint32_t anchors, bool joint) {
     return (la & kNoBody) | ((lb & kNoBody) << 13) | (count << 26) | (anchors << 29) | (joint ? 1u << 31 : 0u);
 }
-__device__ __forceinline__ int32_t word_body(uint32_t bits) { return (bits & kNoBody) == kNoBody ? -1 : int32_t(bits & kNoBody); }
+__device__ __forceinline__ int32_t word_body(uint32_t bits) {
+    return (bits & kNoBody) == kNoBody ? -1 : int32_t(bits & kNoBody);
+}
 // 32 bytes per thread in one load (sm_100's 256-bit global loads): a solver
 // row is two loads instead of four 128-bit ones.  Scattered rows (one
 // manager per thread) cost one L1 wavefront per thread and load instruction,
 // so halving the instructions halves the L1 work of reading them: once a step
-// where the rows go to shared memory, in every pass of an island beyond
-// kBigIsland descriptors.  There the same kernel writes the rows' impulses in
-// an earlier pass, so the load is ordered against memory.
+// where the rows go to shared memory, in every pass of a crowd's islands and
+// of those beyond kBigIsland descriptors.  There the same kernel writes the
+// rows' impulses in an earlier pass, so the load is ordered against memory.
 __device__ __forceinline__ void ldg256(const void* p, float4& a, float4& b) {
     asm volatile("ld.global.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
@@ -1953,9 +1955,9 @@ template <uint32_t CAP, uint32_t NBOD, uint32_t NT, uint32_t CL> struct Unit {
 // with its rows in global memory and an island a CTA, is the faster form; if
 // one class is that crowded all three take it, since clusters beside it starve.
 // Scenes of one heap each, a step with clusters / crowded: 48 x 1,000 boxes
-// (islands up to 2,048) 731 / 779 us, 64 906 / 861, 256 2,640 / 1,915; 24 x 1,500
-// (up to 4,096) 769 / 860, 32 957 / 958, 256 5,502 / 3,190; 64 x 500 (up to 1,024)
-// 490 / 527, 96 611 / 595, 256 1,218 / 926.
+// (islands up to 2,048) 731 / 779 us, 64 906 / 893, 256 2,640 / 1,756; 24 x 1,500
+// (up to 4,096) 769 / 860, 32 957 / 891, 64 1,598 / 1,205; 64 x 500 (up to 1,024)
+// 490 / 527, 96 611 / 595, 256 1,218 / 846.
 template <uint32_t CAP, uint32_t NT> constexpr uint32_t kCrowdLimit =
     148u * uint32_t(232448u / Unit<CAP, CAP + 1, NT, 8>::kBytes) / 8u * 3u / 2u;
 static_assert(pgs_list(1024) == 8 && pgs_list(2048) == 9 && pgs_list(4096) == 10, "lists of the cluster classes");
@@ -2491,8 +2493,10 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
     fork_branches(br, st, 4);
     launch(k_partition_smem<kBigIsland>, grid_for(s.desc_cap, kMidIsland + 1, 148u * 2u), PartSmem<kBigIsland>::kThreads,
                 PartSmem<kBigIsland>::kBytes, 1u, g_high_priority, side(2), s, lvl_bound, 2);
-    launch(k_partition_large, grid_for(s.pairs_expected + s.n_joints, kBigIsland + 1, 148u), 256u, size_t(0), 1u, g_high_priority, side(2), s,
-                lvl_bound);
+    // (a CTA that finds no such island still switches an SM's L1 over: no more
+    // of them than the expected descriptors can need)
+    const uint32_t biggest = grid_for(s.pairs_expected + s.n_joints, kBigIsland + 1, 148u);
+    launch(k_partition_large, biggest, 256u, size_t(0), 1u, g_high_priority, side(2), s, lvl_bound);
     k_partition<<<grid_for(s.desc_cap, kPartWarps, 148u * 16u), kPartWarps * 32, 0, st>>>(s, lvl_bound);
     k_partition_smem<kMidIsland><<<grid_for(s.desc_cap, kSerialIsland + 1, 148u * 8u), 256,
                                    PartSmem<kMidIsland>::kBytes, side(3)>>>(s, lvl_bound, 0);
@@ -2516,8 +2520,7 @@ void enqueue_solver(const DevState& s, cudaStream_t st, const StageHook& hook, c
         const uint32_t islands = grid_for(s.desc_cap, kListMinDesc[list] + 1, 148u * uint32_t(232448u / smem) / cl);
         launch(kernel, islands * cl, nt, smem, cl, cl > 1 ? g_high_priority : 0, side(branch++), s, list);
     });
-    launch(k_pgs_block, grid_for(s.pairs_expected + s.n_joints, kBigIsland + 1, 148u), 256u, size_t(0), 1u, g_high_priority, side(0), s,
-           lvl_bound);
+    launch(k_pgs_block, biggest, 256u, size_t(0), 1u, g_high_priority, side(0), s, lvl_bound);
     k_pgs_group<<<grid_for(s.desc_cap, kGroupCap / kSmallUnit, 148u * 4u), kGroupThreads, GroupUnit::kBytes, st>>>(s);
     join_branches(br, st, Branches::kN);
     hook(kStIntegrate, st);
